@@ -27,8 +27,7 @@ static inline float u2f_host(uint32_t u) {
 __device__ __forceinline__ uint64_t linear_id() { return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// ROPE (ggml_rope_ext forward), modes NORMAL and NEOX, optional frequency factors, YaRN mixing. One thread per element
-// pair. The angle is built as ggml's CPU backend builds it: theta = pos * theta_scale^j by repeated f32 multiplication
+// ROPE (ggml_rope_ext forward), modes NORMAL and NEOX, optional frequency factors, YaRN mixing. The angle is built as ggml's CPU backend builds it: theta = pos * theta_scale^j by repeated f32 multiplication
 // (bit-identical angle), divided by the frequency factor, mixed, then sinf / cosf. F16: source and destination are f16
 // and may be the same range (llama.cpp rotates stored keys in place): a thread reads its two elements before it writes
 // them and no other thread touches them; 16-bit stores need no atomics here.
@@ -51,48 +50,94 @@ __device__ __forceinline__ float ld_elem<__half>(const __half* p, uint64_t i) { 
 __device__ __forceinline__ void st_elem(float* p, uint64_t i, float v) { p[i] = v; }
 __device__ __forceinline__ void st_elem(__half* p, uint64_t i, float v) { p[i] = __float2half_rn(v); }
 
+// The angle and its sine and cosine depend on the position and the pair only, so a thread forms them once and rotates that
+// pair in up to kRopeHeads heads, all of whose loads are in flight together (one thread per element pair of one head, with
+// its own sinf / cosf and 64-bit divisions, took 15 us for 512 positions x 32 heads of 128).
+constexpr uint32_t kRopeHeads = 8;
+
+template <typename T>
+__device__ __forceinline__ void ld_pair(const T* a, uint64_t e0, uint64_t e1, bool vec, float& x0, float& x1) {
+    if constexpr (sizeof(T) == 4) {
+        if (vec) {
+            const float2 x = *reinterpret_cast<const float2*>(a + e0);
+            x0 = x.x;
+            x1 = x.y;
+            return;
+        }
+    }
+    x0 = ld_elem(a, e0);
+    x1 = ld_elem(a, e1);
+}
+template <typename T>
+__device__ __forceinline__ void st_pair(T* d, uint64_t e0, uint64_t e1, bool vec, float x0, float x1) {
+    if constexpr (sizeof(T) == 4) {
+        if (vec) {
+            *reinterpret_cast<float2*>(d + e0) = make_float2(x0, x1);
+            return;
+        }
+    }
+    st_elem(d, e0, x0);
+    st_elem(d, e1, x1);
+}
+
+// CTA: one position (blockIdx.x / chunks) and `heads_per_cta` heads; threads: jt consecutive pairs x 256 / jt head lanes.
+// vec: f32 pairs (e0, e0 + 1) start on 8 bytes in source and destination.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_kernel(const T* a, const int32_t* __restrict__ pos,
-                                                   const float* __restrict__ ff, T* d, const RopeArgs pc) {
+                                                   const float* __restrict__ ff, T* d, const RopeArgs pc, uint32_t jt,
+                                                   uint32_t chunks, uint32_t heads_per_cta, uint32_t vec) {
     pdl_trigger();
     pdl_wait();
-    const uint32_t half_ne0 = pc.ne0 >> 1;
-    const uint64_t i = linear_id();
-    if (i >= (uint64_t)half_ne0 * pc.ne1 * pc.ne2 * pc.ne3) return;
-    uint64_t t = i;
-    const uint32_t j = (uint32_t)(t % half_ne0);
-    t /= half_ne0;
-    const uint32_t i1 = (uint32_t)(t % pc.ne1);
-    t /= pc.ne1;
-    const uint32_t i2 = (uint32_t)(t % pc.ne2), i3 = (uint32_t)(t / pc.ne2);
-    const uint64_t ab = pc.a_off + (uint64_t)i1 * pc.a_s1 + (uint64_t)i2 * pc.a_s2 + (uint64_t)i3 * pc.a_s3;
-    const uint64_t db = pc.d_off + (uint64_t)i1 * pc.d_s1 + (uint64_t)i2 * pc.d_s2 + (uint64_t)i3 * pc.d_s3;
-    if (2u * j >= pc.n_dims) {   // past the rotated part: copied
-        const float c0 = ld_elem(a, ab + 2u * j), c1 = ld_elem(a, ab + 2u * j + 1u);
-        st_elem(d, db + 2u * j, c0);
-        st_elem(d, db + 2u * j + 1u, c1);
-        return;
-    }
-    float theta = (float)pos[pc.pos_off + i2];
-    const float ts = u2f(pc.theta_scale);
-    for (uint32_t k = 0; k < j; ++k) theta = __fmul_rn(theta, ts);
-    const float theta_extrap = pc.has_ff ? __fdiv_rn(theta, ff[pc.ff_off + j]) : theta;
+    const uint32_t half_ne0 = pc.ne0 >> 1, hg = 256u / jt, j0 = threadIdx.x & (jt - 1u), hl = threadIdx.x / jt;
+    const uint32_t row = blockIdx.x / chunks, chunk = blockIdx.x - row * chunks;
+    const uint32_t i3 = row / pc.ne2, i2 = row - i3 * pc.ne2;
+    const uint64_t a23 = pc.a_off + (uint64_t)i2 * pc.a_s2 + (uint64_t)i3 * pc.a_s3;
+    const uint64_t d23 = pc.d_off + (uint64_t)i2 * pc.d_s2 + (uint64_t)i3 * pc.d_s3;
+    const uint32_t h_end = min(pc.ne1, (chunk + 1u) * heads_per_cta);
+    const float theta0 = (float)pos[pc.pos_off + i2], ts = u2f(pc.theta_scale);
     const float freq_scale = u2f(pc.freq_scale), ext_factor = u2f(pc.ext_factor);
-    float mscale = u2f(pc.attn_factor);
-    const float theta_interp = __fmul_rn(freq_scale, theta_extrap);
-    float th = theta_interp;
-    if (ext_factor != 0.0f) {
-        const float low = u2f(pc.corr0), high = u2f(pc.corr1);
-        const float y = __fdiv_rn((float)j - low, fmaxf(0.001f, high - low));
-        const float ramp_mix = __fmul_rn(1.0f - fminf(1.0f, fmaxf(0.0f, y)), ext_factor);
-        th = __fadd_rn(__fmul_rn(theta_interp, 1.0f - ramp_mix), __fmul_rn(theta_extrap, ramp_mix));
-        mscale = __fmul_rn(mscale, 1.0f + __fmul_rn(0.1f, logf(__fdiv_rn(1.0f, freq_scale))));
+    for (uint32_t j = j0; j < half_ne0; j += jt) {
+        const bool rotated = 2u * j < pc.n_dims;   // past the rotated part: copied
+        const bool neox = rotated && pc.mode_neox;
+        const uint32_t e0 = neox ? j : 2u * j, e1 = neox ? j + (pc.n_dims >> 1) : 2u * j + 1u;
+        const bool pair = vec && !neox;
+        float sin_t = 0.0f, cos_t = 1.0f;
+        if (rotated) {
+            float theta = theta0;
+            for (uint32_t k = 0; k < j; ++k) theta = __fmul_rn(theta, ts);
+            const float theta_extrap = pc.has_ff ? __fdiv_rn(theta, ff[pc.ff_off + j]) : theta;
+            float mscale = u2f(pc.attn_factor);
+            const float theta_interp = __fmul_rn(freq_scale, theta_extrap);
+            float th = theta_interp;
+            if (ext_factor != 0.0f) {
+                const float low = u2f(pc.corr0), high = u2f(pc.corr1);
+                const float y = __fdiv_rn((float)j - low, fmaxf(0.001f, high - low));
+                const float ramp_mix = __fmul_rn(1.0f - fminf(1.0f, fmaxf(0.0f, y)), ext_factor);
+                th = __fadd_rn(__fmul_rn(theta_interp, 1.0f - ramp_mix), __fmul_rn(theta_extrap, ramp_mix));
+                mscale = __fmul_rn(mscale, 1.0f + __fmul_rn(0.1f, logf(__fdiv_rn(1.0f, freq_scale))));
+            }
+            sin_t = __fmul_rn(sinf(th), mscale);
+            cos_t = __fmul_rn(cosf(th), mscale);
+        }
+        for (uint32_t h0 = chunk * heads_per_cta + hl; h0 < h_end; h0 += kRopeHeads * hg) {
+            float x0[kRopeHeads], x1[kRopeHeads];
+#pragma unroll
+            for (uint32_t k = 0; k < kRopeHeads; ++k) {
+                const uint32_t h = h0 + k * hg;
+                const uint64_t ab = a23 + (uint64_t)h * pc.a_s1;
+                if (h < h_end) ld_pair(a, ab + e0, ab + e1, pair, x0[k], x1[k]);
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kRopeHeads; ++k) {
+                const uint32_t h = h0 + k * hg;
+                if (h >= h_end) continue;
+                const uint64_t db = d23 + (uint64_t)h * pc.d_s1;
+                const float y0 = rotated ? __fsub_rn(__fmul_rn(x0[k], cos_t), __fmul_rn(x1[k], sin_t)) : x0[k];
+                const float y1 = rotated ? __fadd_rn(__fmul_rn(x0[k], sin_t), __fmul_rn(x1[k], cos_t)) : x1[k];
+                st_pair(d, db + e0, db + e1, pair, y0, y1);
+            }
+        }
     }
-    const float sin_t = __fmul_rn(sinf(th), mscale), cos_t = __fmul_rn(cosf(th), mscale);
-    const uint32_t e0 = pc.mode_neox ? j : 2u * j, e1 = pc.mode_neox ? j + (pc.n_dims >> 1) : 2u * j + 1u;
-    const float x0 = ld_elem(a, ab + e0), x1 = ld_elem(a, ab + e1);
-    st_elem(d, db + e0, __fsub_rn(__fmul_rn(x0, cos_t), __fmul_rn(x1, sin_t)));
-    st_elem(d, db + e1, __fadd_rn(__fmul_rn(x0, sin_t), __fmul_rn(x1, cos_t)));
 }
 
 // the largest element index a strided 4-D walk reaches, + 1
@@ -115,9 +160,21 @@ static AcResult launch_rope_t(const LaunchArgs& a) {
         a.range[1] < ((uint64_t)pc.pos_off + pc.ne2) * 4u ||
         (pc.has_ff && a.range[2] < ((uint64_t)pc.ff_off + pc.n_dims / 2u) * 4u))
         return AC_ERR_INVALID_BUFFER_SIZE;
-    const uint64_t pairs = (uint64_t)(pc.ne0 / 2u) * pc.ne1 * pc.ne2 * pc.ne3;
-    launch_pdl(rope_kernel<T>, dim3((unsigned)((pairs + 255u) / 256u)), dim3(256), 0, a.stream, (const T*)a.ptr[0],
-               (const int32_t*)a.ptr[1], (const float*)a.ptr[2], (T*)a.ptr[3], pc);
+    const uint64_t rows = (uint64_t)pc.ne2 * pc.ne3;
+    uint32_t jt = 8u;
+    while (jt < pc.ne0 / 2u && jt < 256u) jt *= 2u;
+    const uint32_t hg = 256u / jt;
+    // few positions (token generation): one head per thread, so that the heads spread over the SMs; many: all the heads a
+    // thread can carry, so that sine and cosine are formed once
+    const uint64_t sms = a.sm_count > 0 ? (uint64_t)a.sm_count : 148u;
+    const uint32_t heads_per_cta = rows >= sms ? kRopeHeads * hg : hg;
+    const uint32_t chunks = (uint32_t)(((uint64_t)pc.ne1 + heads_per_cta - 1u) / heads_per_cta);
+    if (rows * chunks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
+    const bool vec = sizeof(T) == 4 && !((pc.a_off | pc.a_s1 | pc.a_s2 | pc.a_s3 | pc.d_off | pc.d_s1 | pc.d_s2 | pc.d_s3) & 1u) &&
+                     !(((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[3]) & 7u);
+    launch_pdl(rope_kernel<T>, dim3((unsigned)(rows * chunks)), dim3(256), 0, a.stream, (const T*)a.ptr[0],
+               (const int32_t*)a.ptr[1], (const float*)a.ptr[2], (T*)a.ptr[3], pc, jt, chunks, heads_per_cta,
+               (uint32_t)vec);
     return check_launch();
 }
 AcResult launch_rope(const LaunchArgs& a) { return launch_rope_t<float>(a); }
@@ -218,6 +275,44 @@ __global__ void __launch_bounds__(256) set_rows_kernel(const float* __restrict__
     else ((float*)d)[di] = v;
 }
 
+// The same with one CTA per span of kSetRowsSpan columns of one row: the index is read and checked once, four columns (16
+// bytes in, 16 or 8 out) per thread. One thread per element with five 64-bit divisions took 7 us for 512 rows of 1024.
+constexpr uint32_t kSetRowsThreads = 256, kSetRowsSpan = 4u * kSetRowsThreads;
+__global__ void __launch_bounds__(kSetRowsThreads) set_rows_vec_kernel(const float* __restrict__ a, const uint32_t* __restrict__ idx,
+                                                                       uint32_t* status, void* d, const SetRowsArgs pc,
+                                                                       uint32_t spans) {
+    pdl_trigger();
+    pdl_wait();
+    uint32_t t = blockIdx.x;
+    const uint32_t span = t % spans;
+    t /= spans;
+    const uint32_t r = t % pc.nr;
+    t /= pc.nr;
+    const uint32_t i02 = t % pc.ne02, i03 = t / pc.ne02;
+    const uint32_t c = span * kSetRowsSpan + 4u * threadIdx.x;
+    const uint64_t iw = pc.i_off + (uint64_t)r * pc.i_s0 + (uint64_t)(i02 % pc.i_ne1) * pc.i_s1 +
+                        (uint64_t)(i03 % pc.i_ne2) * pc.i_s2;
+    const uint32_t row = idx[iw], high = pc.idx64 ? idx[iw + 1u] : 0u;
+    if (row >= pc.dst_rows || high != 0u) {
+        if (c == 0u) {
+            atomicAdd(status, 1u);
+            atomicMin(status + 1, pc.node);
+        }
+        return;
+    }
+    if (c >= pc.nc) return;
+    const float4 v = *reinterpret_cast<const float4*>(a + pc.a_off + c + (uint64_t)r * pc.a_s1 + (uint64_t)i02 * pc.a_s2 +
+                                                      (uint64_t)i03 * pc.a_s3);
+    const uint64_t di = pc.d_off + c + (uint64_t)row * pc.d_s1 + (uint64_t)i02 * pc.d_s2 + (uint64_t)i03 * pc.d_s3;
+    if (pc.dst_f16) {
+        const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>((__half*)d + di) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    } else {
+        *reinterpret_cast<float4*>((float*)d + di) = v;
+    }
+}
+
 // ameva_set_rows: bindings 0 src0 f32, 1 indices (words), 2 status (>= 8 bytes), 3 dst; push = SetRowsArgs (22 words)
 AcResult launch_set_rows(const LaunchArgs& a) {
     SetRowsArgs pc;
@@ -231,6 +326,15 @@ AcResult launch_set_rows(const LaunchArgs& a) {
         a.range[1] < idx_words * 4u || a.range[2] < 8u ||
         a.range[3] < span_elems(pc.d_off, pc.nc, pc.dst_rows, pc.ne02, pc.ne03, pc.d_s1, pc.d_s2, pc.d_s3) * (pc.dst_f16 ? 2u : 4u))
         return AC_ERR_INVALID_BUFFER_SIZE;
+    // rows of whole, aligned pieces of four columns
+    const uint64_t spans = ((uint64_t)pc.nc + kSetRowsSpan - 1u) / kSetRowsSpan, ctas = spans * pc.nr * pc.ne02 * pc.ne03;
+    if (!((pc.nc | pc.a_off | pc.a_s1 | pc.a_s2 | pc.a_s3 | pc.d_off | pc.d_s1 | pc.d_s2 | pc.d_s3) & 3u) &&
+        !((uintptr_t)a.ptr[0] & 15u) && !((uintptr_t)a.ptr[3] & (pc.dst_f16 ? 7u : 15u)) && ctas <= 0x7FFFFFFFull &&
+        pc.nc <= 0x7FFFFFFFu) {
+        launch_pdl(set_rows_vec_kernel, dim3((unsigned)ctas), dim3(kSetRowsThreads), 0, a.stream, (const float*)a.ptr[0],
+                   (const uint32_t*)a.ptr[1], (uint32_t*)a.ptr[2], (void*)a.ptr[3], pc, (uint32_t)spans);
+        return check_launch();
+    }
     const uint64_t total = (uint64_t)pc.nc * pc.nr * pc.ne02 * pc.ne03;
     launch_pdl(set_rows_kernel, dim3((unsigned)((total + 255u) / 256u)), dim3(256), 0, a.stream, (const float*)a.ptr[0],
                (const uint32_t*)a.ptr[1], (uint32_t*)a.ptr[2], (void*)a.ptr[3], pc);

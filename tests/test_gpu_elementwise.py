@@ -90,3 +90,36 @@ def test_argument_checks(ctx):
             batch.submit().wait()
         batch.destroy()
     a.destroy()
+
+
+@pytest.mark.parametrize("n", [1, 2049, 65535, 65536, 65537, 67583, 67584, 67587, 200003])
+def test_swiglu_and_add_at_the_edges_of_the_vector_forms(ctx, n):
+    """From 65536 elements: pieces of four, two per thread, 2048 elements per CTA; below, one element per thread."""
+    rng = np.random.default_rng(n)
+    g, u = rng.standard_normal(n).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    g64 = g.astype(np.float64)
+    want = g64 / (1.0 + np.exp(-g64)) * u
+    gb, ub, db = ctx.buffer(data=g), ctx.buffer(data=u), ctx.buffer(4 * n)
+    _run(ctx, "ameva_swiglu_f32", [gb, ub, db], [n])
+    # expf (2 ulp), one division and two multiplications: well below 1e-6 of the value
+    assert np.all(np.abs(db.read(np.float32) - want) <= 1e-6 * np.abs(want) + 1e-30)
+    _run(ctx, "ameva_add_f32", [gb, ub, db], [n, 1, n])
+    assert np.array_equal(db.read(np.float32), g + u)
+    for b in (gb, ub, db):
+        b.destroy()
+
+
+@pytest.mark.parametrize("cols", [4, 1020, 1024, 1028, 4100, 8192, 8196])
+def test_rms_norm_at_the_edges_of_the_register_form(ctx, cols):
+    rng = np.random.default_rng(cols)
+    x = rng.standard_normal((3, cols)).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(cols)).astype(np.float32)
+    eps = np.float32(1e-5)
+    xb, wb = ctx.buffer(data=x), ctx.buffer(data=w)
+    _run(ctx, "ameva_rms_norm_f32", [xb, wb, xb], [3, cols, int(eps.view(np.uint32)), 1])      # in place
+    x64 = x.astype(np.float64)
+    want = x64 / np.sqrt(np.mean(x64 * x64, axis=1, keepdims=True) + float(eps)) * w
+    # the fp32 sum of squares (8192 terms by a tree: well below 1e-6) and four roundings
+    assert np.all(np.abs(xb.read(np.float32).reshape(3, cols) - want) <= 1.5e-6 * np.abs(want) + 1e-30)
+    xb.destroy()
+    wb.destroy()

@@ -393,3 +393,46 @@ def test_unary_ops_follow_the_cpu_formulas(ctx):
         _run(ctx, "ameva_unary", [ab, db], [cols, rows, 1, 1, 0, pitch, 0, 0, 0, cols, 0, 0, 19, 0, 0])
     ab.destroy()
     db.destroy()
+
+
+# ---- the forms that share the angle between heads, and the vector form of the cache write --------------------------------
+@pytest.mark.parametrize("neox", [False, True])
+@pytest.mark.parametrize("shape,n_dims,a_off", [((1, 200, 1, 6), 6, 0), ((1, 149, 37, 64), 48, 0), ((2, 100, 33, 128), 128, 2),
+                                                ((1, 150, 3, 128), 128, 1), ((1, 3, 2, 1030), 1026, 0)])
+def test_rope_over_many_positions_and_odd_heads(ctx, shape, n_dims, a_off, neox):
+    rng = np.random.default_rng(shape[1] + a_off)
+    x = rng.standard_normal(shape).astype(np.float32)
+    pos = rng.integers(0, 8192, shape[1]).astype(np.int32)
+    ts = ops.rope_theta_scale(10000.0, n_dims)
+    src = np.zeros(x.size + a_off, np.float32)
+    src[a_off:] = x.ravel()
+    xb, pb, db = ctx.buffer(data=src), ctx.buffer(data=pos), ctx.buffer(x.nbytes)
+    _run(ctx, "ameva_rope", [xb, pb, pb, db], _rope_push(shape, n_dims, neox, 0, ts, 1.0, 0.0, 1.0, (0.0, 0.0), a_off=a_off))
+    got = db.read(np.float32).reshape(shape)
+    want = ops.rope(x, pos, n_dims, neox, 10000.0)
+    assert np.max(np.abs(got - want)) <= 4e-6 * np.max(np.abs(x))     # (as test_rope_f32_both_modes)
+    assert np.array_equal(got[..., n_dims:], x[..., n_dims:])
+    for b in (xb, pb, db):
+        b.destroy()
+
+
+@pytest.mark.parametrize("dst_dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("nc", [4, 1020, 1024, 1028, 1030])
+def test_set_rows_at_the_edges_of_the_vector_form(ctx, nc, dst_dtype):
+    dst_rows, nr, ne02 = 40, 5, 2
+    rng = np.random.default_rng(nc)
+    cache = rng.standard_normal((1, ne02, dst_rows, nc)).astype(dst_dtype)
+    src = (rng.standard_normal((1, ne02, nr, nc)) * 3).astype(np.float32)
+    idx = rng.permutation(dst_rows)[:nr].astype(np.int64).reshape(1, 1, nr)
+    bad = idx.copy()
+    bad[0, 0, 1], bad[0, 0, 4] = -1, 1 << 33
+    cb, sb, ib = ctx.buffer(data=cache), ctx.buffer(data=src), ctx.buffer(data=bad)
+    stb = ctx.buffer(data=np.array([0, 0xFFFFFFFF], np.uint32))
+    push = [nc, nr, ne02, 1, 0, nc, nc * nr, nc * nr * ne02, 0, 2, 2 * nr, 2 * nr, 1, 1, 1, dst_rows, 0, nc, nc * dst_rows,
+            nc * dst_rows * ne02, int(dst_dtype == np.float16), 11]
+    _run(ctx, "ameva_set_rows", [sb, ib, stb, cb], push)
+    keep = [0, 2, 3]
+    assert np.array_equal(cb.read(dst_dtype).reshape(cache.shape), ops.set_rows(cache, src[:, :, keep], idx[:, :, keep]))
+    assert list(stb.read(np.uint32)) == [2 * ne02, 11]
+    for b in (cb, sb, ib, stb):
+        b.destroy()
