@@ -10,6 +10,7 @@
 
 #include "act_quant.cuh"
 #include "common.cuh"
+#include "fuse.h"
 
 namespace amv {
 
@@ -414,6 +415,118 @@ __global__ void __launch_bounds__(256) bitnet_norm_q8_kernel(const float* __rest
     }
 }
 
+// The plain quantize of such a row (mode 0, no norm: what every I2_S product of a graph runs) with the dispatch that formed
+// the row in the same launch, and for every product that reads the row: y, q, act (and qeo) of up to four destinations.
+// One CTA per row, the row in registers (J pieces of four per thread), so that it is read once and nothing is read back;
+// with one row the work is a chain of latencies, and a launch of its own for each step and destination costs 2-4 us more.
+// The arithmetic and its order are those of the separate kernels (rms_norm_f32_vec_kernel, swiglu_f32_vec_kernel, the kernel
+// above): the bytes are equal.
+struct BitnetDst {
+    float* y;
+    uint32_t* q;
+    uint32_t* act;
+    uint2* qeo;
+};
+struct BitnetRows {
+    const float *a, *b;   // PLAIN: a; NORM: a = x, b = weight row or nullptr; SWIGLU: a = gate, b = up
+    float* h;             // NORM, SWIGLU: the f32 rows they write
+    float eps;
+    uint32_t n;
+    BitnetDst dst[kFuseMax];
+};
+
+template <int SOURCE, int J>
+__global__ void __launch_bounds__(256) bitnet_rows_kernel(const BitnetRows g, uint32_t dim) {
+    __shared__ float red[8], red_max[8];
+    __shared__ int redi[8];
+    const uint32_t row = blockIdx.x, t = threadIdx.x, words = dim >> 2;
+    const float4* a = reinterpret_cast<const float4*>(g.a + (size_t)row * dim);
+    pdl_trigger();
+    pdl_wait();
+    float4 v[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const uint32_t i = t + 256u * j;
+        v[j] = i < words ? a[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if constexpr (SOURCE == BITNET_NORM) {
+        float4 w[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (g.b && t + 256u * j < words) w[j] = reinterpret_cast<const float4*>(g.b)[t + 256u * j];
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < J; ++j) ss = fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, fmaf(v[j].z, v[j].z, fmaf(v[j].w, v[j].w, ss))));
+        ss = warp_sum(ss);
+        if ((t & 31u) == 0) red[t >> 5] = ss;
+        __syncthreads();
+        float tot = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tot += red[i];
+        const float scale = __fdiv_rn(1.0f, sqrtf(__fdiv_rn(tot, (float)dim) + g.eps));
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            v[j] = make_float4(__fmul_rn(v[j].x, scale), __fmul_rn(v[j].y, scale), __fmul_rn(v[j].z, scale), __fmul_rn(v[j].w, scale));
+            if (g.b && t + 256u * j < words)
+                v[j] = make_float4(__fmul_rn(v[j].x, w[j].x), __fmul_rn(v[j].y, w[j].y), __fmul_rn(v[j].z, w[j].z), __fmul_rn(v[j].w, w[j].w));
+        }
+    } else if constexpr (SOURCE == BITNET_SWIGLU) {
+        const float4* up = reinterpret_cast<const float4*>(g.b + (size_t)row * dim);
+        float4 u[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) u[j] = t + 256u * j < words ? up[t + 256u * j] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            v[j] = make_float4(swiglu_f32(v[j].x, u[j].x), swiglu_f32(v[j].y, u[j].y), swiglu_f32(v[j].z, u[j].z), swiglu_f32(v[j].w, u[j].w));
+    }
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const uint32_t i = t + 256u * j;
+        if (i >= words) continue;
+        if (SOURCE != BITNET_PLAIN) reinterpret_cast<float4*>(g.h + (size_t)row * dim)[i] = v[j];
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+    }
+    amax = warp_max(amax);
+    if ((t & 31u) == 0) red_max[t >> 5] = amax;
+    __syncthreads();
+    amax = red_max[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, red_max[i]);
+    const float qs = __fdiv_rn(127.0f, fmaxf(amax, 1e-7f));
+    int qsum = 0;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const uint32_t i = t + 256u * j;
+        if (i >= words) continue;
+        const float x[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+        uint32_t packed = 0, u[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int iv = max(-127, min(127, (int)roundf(__fmul_rn(x[k], qs))));
+            packed |= (uint32_t)(iv & 0xFF) << (8 * k);
+            qsum += iv;
+            u[k] = (uint32_t)(iv + 128);
+        }
+        for (uint32_t d = 0; d < g.n; ++d) {
+            const size_t o = (size_t)row * words + i;
+            reinterpret_cast<float4*>(g.dst[d].y)[o] = v[j];
+            g.dst[d].q[o] = packed;
+            if (g.dst[d].qeo) g.dst[d].qeo[o] = make_uint2((u[0] << 16) | u[2], (u[1] << 16) | u[3]);
+        }
+    }
+    qsum = warp_sum_i(qsum);
+    if ((t & 31u) == 0) redi[t >> 5] = qsum;
+    __syncthreads();
+    if (t < g.n) {
+        int sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += redi[i];
+        g.dst[t].act[2u * row] = __float_as_uint(__fdiv_rn(1.0f, qs));
+        g.dst[t].act[2u * row + 1u] = (uint32_t)sum;
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------------------------------------
@@ -527,13 +640,69 @@ AcResult launch_rms_norm_quant_a8b(const LaunchArgs& a) { return launch_rms_norm
 
 // bitnet_norm_q8: bindings 0 a, 1 b, 2 w, 3 y, 4 q, 5 act, 6 qeo; push {dim, eps_bits, mode, do_norm}; grid.x = rows
 // (argument contract of src/shaders/bitnet_norm_q8.comp:20-44, extended from one row to grid.x rows).
-AcResult launch_bitnet_norm_q8(const LaunchArgs& a) {
+AcResult check_bitnet_norm_q8(const LaunchArgs& a) {
     const uint32_t dim = a.push[0], mode = a.push[2], do_norm = a.push[3], rows = a.grid.x;
     if (dim == 0 || (dim & 3u) || mode > 2u || a.grid.y != 1 || a.grid.z != 1) return AC_ERR_KERNEL_ARG_INVALID;
     const uint64_t need = (uint64_t)rows * dim * 4u;
     if (a.range[0] < need || (mode != 0u && a.range[1] < need) || (do_norm && a.range[2] < (uint64_t)dim * 4u) ||
         a.range[3] < need || a.range[4] < (uint64_t)rows * dim || a.range[5] < (uint64_t)rows * 8u)
         return AC_ERR_INVALID_BUFFER_SIZE;
+    return AC_SUCCESS;
+}
+
+// rows that stay in registers: at most eight pieces of four per thread; the kernel above serves longer rows and the other modes
+bool bitnet_rows_fits(const LaunchArgs& a) {
+    return a.push[2] == 0u && a.push[3] == 0u && a.push[0] <= 8192u && !(((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[3]) & 15u) &&
+           !((uintptr_t)a.ptr[4] & 3u) && !((uintptr_t)a.ptr[5] & 3u) && !((uintptr_t)a.ptr[6] & 7u);
+}
+
+template <int SOURCE>
+static void launch_bitnet_rows_j(cudaStream_t stream, const BitnetRows& g, uint32_t dim, uint32_t rows) {
+    const uint32_t J = ((dim >> 2) + 255u) / 256u;
+    const dim3 grid(rows), block(256);
+    if (J <= 1) launch_pdl(bitnet_rows_kernel<SOURCE, 1>, grid, block, 0, stream, g, dim);
+    else if (J <= 2) launch_pdl(bitnet_rows_kernel<SOURCE, 2>, grid, block, 0, stream, g, dim);
+    else if (J <= 4) launch_pdl(bitnet_rows_kernel<SOURCE, 4>, grid, block, 0, stream, g, dim);
+    else launch_pdl(bitnet_rows_kernel<SOURCE, 8>, grid, block, 0, stream, g, dim);
+}
+
+AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const LaunchArgs* const* norm_q8, uint32_t n) {
+    const LaunchArgs& first = *norm_q8[0];
+    const uint32_t dim = first.push[0], rows = first.grid.x;
+    BitnetRows g;
+    memset(&g, 0, sizeof(g));
+    g.n = n;
+    for (uint32_t d = 0; d < n; ++d) {
+        const LaunchArgs& a = *norm_q8[d];
+        g.dst[d] = {(float*)a.ptr[3], (uint32_t*)a.ptr[4], (uint32_t*)a.ptr[5],
+                    a.range[6] >= (uint64_t)rows * dim * 2u ? (uint2*)a.ptr[6] : nullptr};
+    }
+    if (source == BITNET_PLAIN) {
+        g.a = (const float*)first.ptr[0];
+        launch_bitnet_rows_j<BITNET_PLAIN>(first.stream, g, dim, rows);
+    } else if (source == BITNET_NORM) {
+        g.a = (const float*)head->ptr[0];
+        g.b = head->push[3] ? (const float*)head->ptr[1] : nullptr;
+        g.h = (float*)head->ptr[2];
+        memcpy(&g.eps, &head->push[2], 4);
+        launch_bitnet_rows_j<BITNET_NORM>(first.stream, g, dim, rows);
+    } else {
+        g.a = (const float*)head->ptr[0];
+        g.b = (const float*)head->ptr[1];
+        g.h = (float*)head->ptr[2];
+        launch_bitnet_rows_j<BITNET_SWIGLU>(first.stream, g, dim, rows);
+    }
+    return check_launch();
+}
+
+AcResult launch_bitnet_norm_q8(const LaunchArgs& a) {
+    const AcResult rc = check_bitnet_norm_q8(a);
+    if (rc != AC_SUCCESS) return rc;
+    if (bitnet_rows_fits(a)) {
+        const LaunchArgs* one = &a;
+        return launch_bitnet_rows(BITNET_PLAIN, nullptr, &one, 1u);
+    }
+    const uint32_t dim = a.push[0], mode = a.push[2], do_norm = a.push[3], rows = a.grid.x;
     uint2* qeo = a.range[6] >= (uint64_t)rows * dim * 2u ? (uint2*)a.ptr[6] : nullptr;
     float eps;
     memcpy(&eps, &a.push[1], 4);

@@ -196,6 +196,9 @@ __device__ __forceinline__ uint4 ld_cached_u4(const void* p) { return __ldg(rein
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 __device__ __forceinline__ uint16_t f2h(float f) { return __half_as_ushort(__float2half_rn(f)); }
 
+// the split SWIGLU gate: silu(g) * u
+__device__ __forceinline__ float swiglu_f32(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
+
 __device__ __forceinline__ int dp4a_ss(uint32_t a, uint32_t b, int c) { return __dp4a((int)a, (int)b, c); }
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -64,8 +64,6 @@ __global__ void __launch_bounds__(256) binary_f32_kernel(const float* __restrict
     dst[i] = binary_op<OP>(a[i], b[(r % b_rows) * cols + c]);
 }
 
-__device__ __forceinline__ float swiglu(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
-
 // dst = silu(gate) * up
 __global__ void __launch_bounds__(kVecThreads) swiglu_f32_vec_kernel(const float* gate, const float* up, float* dst,
                                                                      uint64_t total) {
@@ -86,11 +84,11 @@ __global__ void __launch_bounds__(kVecThreads) swiglu_f32_vec_kernel(const float
         const uint64_t i = i0 + k * kVecThreads;
         if (i < n4)
             reinterpret_cast<float4*>(dst)[i] =
-                make_float4(swiglu(g[k].x, u[k].x), swiglu(g[k].y, u[k].y), swiglu(g[k].z, u[k].z), swiglu(g[k].w, u[k].w));
+                make_float4(swiglu_f32(g[k].x, u[k].x), swiglu_f32(g[k].y, u[k].y), swiglu_f32(g[k].z, u[k].z), swiglu_f32(g[k].w, u[k].w));
     }
     if (blockIdx.x == gridDim.x - 1u && threadIdx.x < (total & 3u)) {
         const uint64_t i = 4u * n4 + threadIdx.x;
-        dst[i] = swiglu(gate[i], up[i]);
+        dst[i] = swiglu_f32(gate[i], up[i]);
     }
 }
 __global__ void __launch_bounds__(256) swiglu_f32_kernel(const float* __restrict__ gate, const float* __restrict__ up,
@@ -98,7 +96,7 @@ __global__ void __launch_bounds__(256) swiglu_f32_kernel(const float* __restrict
     pdl_trigger();
     pdl_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < total) dst[i] = swiglu(gate[i], up[i]);
+    if (i < total) dst[i] = swiglu_f32(gate[i], up[i]);
 }
 
 // one CTA per row: y = x * rsqrt(mean(x^2) + eps) [* w]

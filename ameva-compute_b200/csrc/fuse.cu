@@ -1,0 +1,195 @@
+// Matching of recorded dispatches with fused launches (fuse.h). A dispatch may join one recorded before it when nothing
+// recorded in between touches any range it binds (reads of the same range count as touching: the check knows no directions),
+// so running it early changes neither what it reads nor what the others read. Only kernels whose effects are confined to
+// their bindings are looked past (the output exchange between ranks and kernels a host has registered are not). A form is
+// taken only when every member passes the checks of its own launcher; anything else is launched by itself, errors included.
+#include "fuse.h"
+
+namespace amv {
+
+AcResult launch_add_f32(const LaunchArgs&);
+AcResult launch_bitnet_gemm_i2_s(const LaunchArgs&);
+AcResult launch_bitnet_gemv_i2_s(const LaunchArgs&);
+AcResult launch_bitnet_norm_q8(const LaunchArgs&);
+AcResult launch_rms_norm_f32(const LaunchArgs&);
+AcResult launch_swiglu_f32(const LaunchArgs&);
+
+namespace {
+
+constexpr uint32_t kLookahead = 12;   // operations looked at past the first
+
+bool is(const FuseOp& op, LaunchFn fn) { return op.entry->launch == fn; }
+
+bool overlap(const void* p, uint64_t n, const void* q, uint64_t m) {
+    const uintptr_t a = (uintptr_t)p, b = (uintptr_t)q;
+    return a < b + m && b < a + n;
+}
+bool touches(const LaunchArgs& a, const void* p, uint64_t n) {
+    for (uint32_t i = 0; i < a.binding_count; ++i)
+        if (overlap(a.ptr[i], a.range[i], p, n)) return true;
+    return false;
+}
+bool disjoint(const LaunchArgs& a, const LaunchArgs& b) {
+    for (uint32_t i = 0; i < b.binding_count; ++i)
+        if (touches(a, b.ptr[i], b.range[i])) return false;
+    return true;
+}
+
+// kernels that read and write their bindings and nothing else
+bool confined(const FuseOp& op) {
+    return is(op, launch_bitnet_gemv_i2_s) || is(op, launch_bitnet_gemm_i2_s) || is(op, launch_bitnet_norm_q8);
+}
+
+// May ops[j] run together with ops[i], i < j? Members of the group being formed (marked in `member`) are checked by the caller.
+bool can_hoist(const FuseOp* ops, uint32_t i, uint32_t j, uint64_t member) {
+    for (uint32_t k = i + 1; k < j; ++k) {
+        if (ops[k].done || (member >> (k - i) & 1u)) continue;
+        if (!confined(ops[k]) || !disjoint(ops[k].args, ops[j].args)) return false;
+    }
+    return true;
+}
+
+// ---- RMS norm, SWIGLU or nothing, then the quantize of every I2_S product that reads the rows ----
+AcResult fuse_bitnet_rows(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
+    const LaunchArgs& head = ops[i].args;
+    BitnetSource source = BITNET_PLAIN;
+    const void* rows_ptr = head.ptr[0];
+    uint32_t dim = 0, rows = 0;
+    const LaunchArgs* member[kFuseMax];
+    uint32_t count = 0;
+    uint64_t mask = 0;
+    if (is(ops[i], launch_bitnet_norm_q8)) {
+        if (check_bitnet_norm_q8(head) != AC_SUCCESS || !bitnet_rows_fits(head)) return AC_SUCCESS;
+        dim = head.push[0];
+        rows = head.grid.x;
+        member[count++] = &head;
+    } else if (is(ops[i], launch_rms_norm_f32)) {
+        source = BITNET_NORM;
+        rows = head.push[0];
+        dim = head.push[1];
+        rows_ptr = head.ptr[2];
+        float eps;
+        memcpy(&eps, &head.push[2], 4);
+        const uint64_t bytes = (uint64_t)rows * dim * 4u;
+        if (!rows || !dim || head.push[3] > 1u || !(eps >= 0.0f) || head.range[0] < bytes || head.range[2] < bytes ||
+            (head.push[3] && (head.range[1] < (uint64_t)dim * 4u || ((uintptr_t)head.ptr[1] & 15u) ||
+                              overlap(head.ptr[1], (uint64_t)dim * 4u, head.ptr[2], bytes))))
+            return AC_SUCCESS;
+        if (head.ptr[0] != head.ptr[2] && overlap(head.ptr[0], bytes, head.ptr[2], bytes)) return AC_SUCCESS;
+    } else {
+        source = BITNET_SWIGLU;
+        rows_ptr = head.ptr[2];
+    }
+    const uint64_t swiglu_n = source == BITNET_SWIGLU ? head.push[0] : 0u;
+    for (uint32_t j = i + 1; j < n && j <= i + kLookahead && count < kFuseMax; ++j) {
+        if (ops[j].done) continue;
+        const LaunchArgs& q = ops[j].args;
+        if (is(ops[j], launch_bitnet_norm_q8) && q.ptr[0] == rows_ptr && check_bitnet_norm_q8(q) == AC_SUCCESS && bitnet_rows_fits(q)) {
+            bool ok = true;
+            if (source == BITNET_SWIGLU && count == 0) {   // the first quantize says how the elements form rows
+                dim = q.push[0];
+                rows = q.grid.x;
+                const uint64_t bytes = swiglu_n * 4u;
+                ok = swiglu_n && (uint64_t)dim * rows == swiglu_n && head.range[0] >= bytes && head.range[1] >= bytes &&
+                     head.range[2] >= bytes && (head.ptr[0] == head.ptr[2] || !overlap(head.ptr[0], bytes, head.ptr[2], bytes)) &&
+                     (head.ptr[1] == head.ptr[2] || !overlap(head.ptr[1], bytes, head.ptr[2], bytes)) && !((uintptr_t)head.ptr[1] & 15u);
+            }
+            ok = ok && q.push[0] == dim && q.grid.x == rows && !((uintptr_t)head.ptr[0] & 15u) && can_hoist(ops, i, j, mask);
+            // what this member writes (y, q, act, qeo) meets nothing that the head or another member reads or writes
+            for (uint32_t b = 3; b < 7u && ok; ++b) {
+                for (uint32_t h = 0; h < head.binding_count && ok; ++h) {
+                    if (source == BITNET_NORM && h == 1u && !head.push[3]) continue;   // (the unused weight binding)
+                    if (source == BITNET_PLAIN && (h == 1u || h == 2u)) continue;      // (b and w, unused in this mode)
+                    ok = !overlap(head.ptr[h], head.range[h], q.ptr[b], q.range[b]);
+                }
+                for (uint32_t m = 0; m < count && ok; ++m)
+                    for (uint32_t h = 3; h < 7u && ok; ++h) ok = !overlap(member[m]->ptr[h], member[m]->range[h], q.ptr[b], q.range[b]);
+                for (uint32_t h = 3; h < b && ok; ++h) ok = !overlap(q.ptr[h], q.range[h], q.ptr[b], q.range[b]);
+                ok = ok && !overlap(rows_ptr, (uint64_t)rows * dim * 4u, q.ptr[b], q.range[b]);
+            }
+            if (ok) {
+                member[count++] = &q;
+                mask |= 1ull << (j - i);
+                continue;
+            }
+        }
+        if (!confined(ops[j])) break;
+    }
+    if (count == 0 || (count == 1 && source == BITNET_PLAIN)) return AC_SUCCESS;
+    if (rows > 0x7fffffffu) return AC_SUCCESS;
+    *taken = true;
+    ops[i].done = true;
+    for (uint32_t k = 0; k <= kLookahead; ++k)
+        if (mask >> k & 1u) ops[i + k].done = true;
+    return launch_bitnet_rows(source, &head, member, count);
+}
+
+// ---- I2_S products: several in one launch, or one with the ADD that consumes it ----
+AcResult fuse_bitnet_gemv(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
+    const LaunchArgs& head = ops[i].args;
+    if (check_bitnet_gemv_i2_s(head) != AC_SUCCESS) return AC_SUCCESS;
+    const uint32_t K = head.push[0], M = head.push[4] ? head.push[4] : 1u;
+    const LaunchArgs* member[kFuseMax] = {&head};
+    uint32_t count = 1;
+    uint64_t mask = 0;
+    for (uint32_t j = i + 1; j < n && j <= i + kLookahead && count < kFuseMax; ++j) {
+        if (ops[j].done) continue;
+        const LaunchArgs& p = ops[j].args;
+        if (is(ops[j], launch_bitnet_gemv_i2_s) && p.push[0] == K && (p.push[4] ? p.push[4] : 1u) == M &&
+            check_bitnet_gemv_i2_s(p) == AC_SUCCESS && can_hoist(ops, i, j, mask)) {
+            bool ok = true;   // no product writes what another one reads or writes
+            for (uint32_t m = 0; m < count && ok; ++m)
+                ok = !touches(*member[m], p.ptr[2], p.range[2]) && !touches(p, member[m]->ptr[2], member[m]->range[2]);
+            if (ok) {
+                member[count++] = &p;
+                mask |= 1ull << (j - i);
+                continue;
+            }
+        }
+        if (!confined(ops[j])) break;
+    }
+    const LaunchArgs* add = nullptr;
+    bool swapped = false;
+    uint32_t add_at = 0;
+    if (count == 1) {   // the next operation adds rows to the product
+        uint32_t j = i + 1;
+        while (j < n && ops[j].done) ++j;
+        if (j < n && is(ops[j], launch_add_f32)) {
+            const LaunchArgs& s = ops[j].args;
+            const uint32_t N = head.push[1], stride = head.push[5] ? head.push[5] : N;
+            const uint64_t bytes = (uint64_t)M * N * 4u;
+            const char* product = (const char*)head.ptr[2] + 4ull * head.push[3];
+            swapped = s.ptr[1] == product;
+            const void* e = s.ptr[swapped ? 0 : 1];
+            if ((swapped || s.ptr[0] == product) && stride == N && s.push[0] == M && s.push[1] == N && s.push[2] == M &&
+                s.range[0] >= bytes && s.range[1] >= bytes && s.range[2] >= bytes && !overlap(e, bytes, product, bytes) &&
+                (e == s.ptr[2] || !overlap(e, bytes, s.ptr[2], bytes)) && !touches(head, s.ptr[2], s.range[2])) {
+                add = &s;
+                add_at = j;
+            }
+        }
+        if (!add) return AC_SUCCESS;
+        ops[add_at].done = true;
+    }
+    *taken = true;
+    ops[i].done = true;
+    for (uint32_t k = 0; k <= kLookahead; ++k)
+        if (mask >> k & 1u) ops[i + k].done = true;
+    return launch_bitnet_gemv_i2_s_group(member, count, add, swapped);
+}
+
+}  // namespace
+
+AcResult launch_fused(FuseOp* ops, uint32_t n, uint32_t i) {
+    bool taken = false;
+    AcResult rc = AC_SUCCESS;
+    if (is(ops[i], launch_bitnet_norm_q8) || is(ops[i], launch_rms_norm_f32) || is(ops[i], launch_swiglu_f32))
+        rc = fuse_bitnet_rows(ops, n, i, &taken);
+    else if (is(ops[i], launch_bitnet_gemv_i2_s))
+        rc = fuse_bitnet_gemv(ops, n, i, &taken);
+    if (taken) return rc;
+    ops[i].done = true;
+    return ops[i].entry->launch(ops[i].args);
+}
+
+}  // namespace amv

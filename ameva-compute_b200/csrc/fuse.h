@@ -1,0 +1,34 @@
+// Recorded dispatches that leave the host in one launch. A batch is launched in the order it was recorded; where a run of
+// its dispatches has a fused form, fuse.cu launches that form instead, with the same results in the same buffers (every
+// destination a separate dispatch would have written is written). At token generation a layer is a chain of launches of 2-4
+// us whose work takes a fraction of that, so the number of launches is what it costs.
+#pragma once
+#include "common.cuh"
+
+namespace amv {
+
+struct FuseOp {
+    const KernelEntry* entry;
+    LaunchArgs args;
+    bool done;   // launched, alone or as part of a fused form
+};
+
+// Launches ops[i] together with the later operations that can join it, and marks all of them done.
+AcResult launch_fused(FuseOp* ops, uint32_t n, uint32_t i);
+
+// ---- fused forms (each launcher validates what the separate launchers validate; the matching is in fuse.cu) ------------
+constexpr uint32_t kFuseMax = 4;   // members of a group
+
+// bitnet rows (act_quant.cu): the quantize of an I2_S product over rows that are copied (PLAIN), RMS-normalised (NORM, the
+// arguments of ameva_rms_norm_f32) or formed by SWIGLU (ameva_swiglu_f32) by the dispatch before, written to n destinations
+enum BitnetSource { BITNET_PLAIN, BITNET_NORM, BITNET_SWIGLU };
+AcResult check_bitnet_norm_q8(const LaunchArgs& a);
+bool bitnet_rows_fits(const LaunchArgs& norm_q8);   // a plain quantize (mode 0, no norm) the row kernel serves
+AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const LaunchArgs* const* norm_q8, uint32_t n);
+
+// up to four I2_S products (bitnet_gemv_i2_s_*) of the same K and row count in one launch; add: with n == 1, the
+// ameva_add_f32 whose first (swapped: second) operand is the product
+AcResult check_bitnet_gemv_i2_s(const LaunchArgs& a);
+AcResult launch_bitnet_gemv_i2_s_group(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped);
+
+}  // namespace amv

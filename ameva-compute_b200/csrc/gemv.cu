@@ -13,6 +13,7 @@
 
 #include "act_quant.cuh"
 #include "common.cuh"
+#include "fuse.h"
 
 namespace amv {
 
@@ -527,16 +528,39 @@ gemv_group_kernel(const WeightGroup g, const float* __restrict__ X, const int8_t
 // chunk, group g: codes = (word >> (6-2g)) & 0x03030303 meet the activation word of elements b*128 + g*32 + 16hh + 4w.
 //   total = sum code*q - sum q (exact int32);  y = float(total) * (act_dequant * w_scale)  [+ y_old when ACC]
 // ---------------------------------------------------------------------------------------------------------------------
+// Up to four products of the same K and row count share a launch (q / k / v, gate / up: launches of 4-5 us for less than
+// 2 us of reading each); a single one may carry the ADD that consumes it (out = product + e, N floats per activation row).
+struct I2sGroup {
+    const uint4* W[kFuseMax];
+    const int8_t* AQ[kFuseMax];
+    const uint32_t* ACT[kFuseMax];
+    float* dst[kFuseMax];
+    float w_scale[kFuseMax];
+    uint32_t N[kFuseMax], dst_stride[kFuseMax];
+    uint32_t warp_end[kFuseMax];   // warps of products 0..j
+    const float* e;
+    float* out;                    // nullptr: no ADD
+};
+
 template <int M, int R, bool ACC>
 __global__ void __launch_bounds__(kGemvThreads)
-gemv_i2_s_kernel(const uint4* __restrict__ W, const int8_t* __restrict__ AQ, float* __restrict__ dst,
-                 const uint32_t* __restrict__ ACT, uint32_t N, uint32_t K, float w_scale, uint32_t dst_stride,
-                 uint32_t aq_stride) {
+gemv_i2_s_kernel(const I2sGroup gr, uint32_t K) {
+    uint32_t warp = (blockIdx.x * kGemvThreads + threadIdx.x) >> 5, j = 0;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (warp >= gr.warp_end[kFuseMax - 1]) return;
+#pragma unroll
+    for (uint32_t i = 0; i + 1u < kFuseMax; ++i)
+        if (warp >= gr.warp_end[i]) j = i + 1u;
+    if (j) warp -= gr.warp_end[j - 1u];
+    const uint4* __restrict__ W = gr.W[j];
+    const int8_t* __restrict__ AQ = gr.AQ[j];
+    const uint32_t* __restrict__ ACT = gr.ACT[j];
+    float* dst = gr.dst[j];
+    const float w_scale = gr.w_scale[j];
+    const uint32_t N = gr.N[j], dst_stride = gr.dst_stride[j], aq_stride = K;
     constexpr int UN = M <= 2 ? 4 : 2;
     const uint32_t C = K >> 6;  // 16-byte chunks per row
-    const uint32_t warp = (blockIdx.x * kGemvThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     const uint32_t row0 = warp * R;
-    if (row0 >= N) return;
     size_t rbase[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) rbase[r] = (size_t)min(row0 + r, N - 1) * C;
@@ -603,6 +627,7 @@ gemv_i2_s_kernel(const uint4* __restrict__ W, const int8_t* __restrict__ AQ, flo
                 const float v = __fmul_rn((float)sum, total_scale);
                 float* o = dst + (size_t)m * dst_stride + row0 + r;
                 *o = ACC ? __fadd_rn(*o, v) : v;
+                if (!ACC && gr.out) gr.out[(size_t)m * N + row0 + r] = v + gr.e[(size_t)m * N + row0 + r];
             }
         }
 }
@@ -853,8 +878,7 @@ AcResult launch_mmvqb_q4_K_fq(const LaunchArgs& a) { return launch_fq<2>(a); }
 //   push {in_dim (%128), out_dim, weight_scale_bits, output_offset_words, rows (0 or absent = 1), out_stride (0 =
 //   out_dim)}: the last two extend the reference's single-vector contract to M <= 8 token rows (activation rows in_dim
 //   bytes apart, act 2 words apart, outputs out_stride floats apart).
-template <bool ACC>
-static AcResult launch_i2s(const LaunchArgs& a) {
+AcResult check_bitnet_gemv_i2_s(const LaunchArgs& a) {
     const uint32_t K = a.push[0], N = a.push[1], off = a.push[3];
     const uint32_t M = a.push[4] ? a.push[4] : 1u, dst_stride = a.push[5] ? a.push[5] : N;
     if (M > 8) return AC_ERR_INVALID_SHAPE;
@@ -862,14 +886,50 @@ static AcResult launch_i2s(const LaunchArgs& a) {
     if (a.range[0] < (uint64_t)N * (K >> 2) || a.range[1] < (uint64_t)M * K ||
         a.range[2] < ((uint64_t)off + (uint64_t)(M - 1) * dst_stride + N) * 4u || a.range[3] < (uint64_t)M * 8u)
         return AC_ERR_INVALID_BUFFER_SIZE;
-    float w_scale;
-    memcpy(&w_scale, &a.push[2], 4);
-    float* dst = (float*)a.ptr[2] + off;
-    AMV_GEMV_SWITCH(gemv_i2_s_kernel, ACC, (const uint4*)a.ptr[0], (const int8_t*)a.ptr[1], dst,
-                    (const uint32_t*)a.ptr[3], N, K, w_scale, dst_stride, K)
+    return AC_SUCCESS;
+}
+
+// checked products of the same K and row count
+template <bool ACC>
+static AcResult launch_i2s(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped) {
+    const LaunchArgs& a = *gemv[0];
+    const uint32_t K = a.push[0], M = a.push[4] ? a.push[4] : 1u, R = M <= 2u ? 2u : 4u;   // (R as in AMV_GEMV_SWITCH)
+    I2sGroup g;
+    memset(&g, 0, sizeof(g));
+    uint64_t warps = 0;
+    for (uint32_t j = 0; j < kFuseMax; ++j) {
+        if (j < n) {
+            const LaunchArgs& p = *gemv[j];
+            g.W[j] = (const uint4*)p.ptr[0];
+            g.AQ[j] = (const int8_t*)p.ptr[1];
+            g.ACT[j] = (const uint32_t*)p.ptr[3];
+            g.dst[j] = (float*)p.ptr[2] + p.push[3];
+            memcpy(&g.w_scale[j], &p.push[2], 4);
+            g.N[j] = p.push[1];
+            g.dst_stride[j] = p.push[5] ? p.push[5] : p.push[1];
+            warps += (p.push[1] + R - 1u) / R;
+        }
+        if (warps > 0x1fffffffull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
+        g.warp_end[j] = (uint32_t)warps;
+    }
+    if (add) {
+        g.e = (const float*)add->ptr[swapped ? 0 : 1];
+        g.out = (float*)add->ptr[2];
+    }
+    const uint32_t N = (uint32_t)warps * R;   // (the switch's row count: whole warps of every product)
+    AMV_GEMV_SWITCH(gemv_i2_s_kernel, ACC, g, K)
     return check_launch();
 }
-AcResult launch_bitnet_gemv_i2_s(const LaunchArgs& a) { return launch_i2s<false>(a); }
-AcResult launch_bitnet_gemv_i2_s_acc(const LaunchArgs& a) { return launch_i2s<true>(a); }
+AcResult launch_bitnet_gemv_i2_s_group(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped) {
+    return launch_i2s<false>(gemv, n, add, swapped);
+}
+template <bool ACC>
+static AcResult launch_i2s_one(const LaunchArgs& a) {
+    const AcResult rc = check_bitnet_gemv_i2_s(a);
+    const LaunchArgs* one = &a;
+    return rc != AC_SUCCESS ? rc : launch_i2s<ACC>(&one, 1u, nullptr, false);
+}
+AcResult launch_bitnet_gemv_i2_s(const LaunchArgs& a) { return launch_i2s_one<false>(a); }
+AcResult launch_bitnet_gemv_i2_s_acc(const LaunchArgs& a) { return launch_i2s_one<true>(a); }
 
 }  // namespace amv

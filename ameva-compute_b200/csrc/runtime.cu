@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fuse.h"
 
 using namespace amv;
 
@@ -174,20 +175,8 @@ AcResult wait_cuda_event(AcContext* ctx, cudaEvent_t ev, uint64_t timeout_ns) {
     }
 }
 
-AcResult launch_record(AcContext* ctx, const KernelEntry* e, uint32_t nbind, void* const* ptrs, const uint64_t* ranges,
-                       const uint32_t* push, AcDim3 grid) {
-    if (!e->launch) {   // a registered kernel: the public form of the same arguments
-        AcB200Launch l;
-        l.stream = ctx->stream;
-        l.binding_count = nbind;
-        l.ptr = ptrs;
-        l.range = ranges;
-        l.push = push;
-        l.push_bytes = e->push_bytes;
-        l.sm_count = ctx->prop.multiProcessorCount;
-        l.grid = grid;
-        return e->ext(&l);
-    }
+LaunchArgs launch_args(AcContext* ctx, uint32_t nbind, void* const* ptrs, const uint64_t* ranges, const uint32_t* push,
+                       AcDim3 grid) {
     LaunchArgs a;
     memset(&a, 0, sizeof(a));
     a.stream = ctx->stream;
@@ -203,7 +192,24 @@ AcResult launch_record(AcContext* ctx, const KernelEntry* e, uint32_t nbind, voi
     a.workspace = ctx->workspace;
     a.workspace_bytes = kWorkspaceBytes;
     a.side = &ctx->side;
-    return e->launch(a);
+    return a;
+}
+
+AcResult launch_record(AcContext* ctx, const KernelEntry* e, uint32_t nbind, void* const* ptrs, const uint64_t* ranges,
+                       const uint32_t* push, AcDim3 grid) {
+    if (!e->launch) {   // a registered kernel: the public form of the same arguments
+        AcB200Launch l;
+        l.stream = ctx->stream;
+        l.binding_count = nbind;
+        l.ptr = ptrs;
+        l.range = ranges;
+        l.push = push;
+        l.push_bytes = e->push_bytes;
+        l.sm_count = ctx->prop.multiProcessorCount;
+        l.grid = grid;
+        return e->ext(&l);
+    }
+    return e->launch(launch_args(ctx, nbind, ptrs, ranges, push, grid));
 }
 
 bool abi_ok(uint32_t abi_version, uint32_t struct_size, size_t expect) {
@@ -304,11 +310,23 @@ AcResult flush_batch(AcCommandBatch* b) {
             cudaEventRecord(b->t_begin, ctx->stream);
         }
     }
-    for (; b->flushed < b->records.size(); ++b->flushed) {
-        BatchRecord& r = b->records[b->flushed];
+    const size_t first = b->flushed, n = b->records.size() - first;
+    std::vector<FuseOp> ops(n);   // the launches in recorded order; runs of them may leave as one (fuse.h)
+    for (size_t k = 0; k < n; ++k) {
+        const BatchRecord& r = b->records[first + k];
         void* ptrs[16];
         for (uint32_t i = 0; i < r.nbind; ++i) ptrs[i] = (char*)r.buf[i]->dptr + r.offset[i];
-        const AcResult rc = launch_record(ctx, r.kernel->entry, r.nbind, ptrs, r.range, r.push, r.grid);
+        ops[k] = {r.kernel->entry, launch_args(ctx, r.nbind, ptrs, r.range, r.push, r.grid), false};
+    }
+    // dispatch timestamps ask for the time of every dispatch: each is launched by itself
+    const bool fuse = !(b->flags & AC_BATCH_FLAG_DISPATCH_TIMESTAMPS);
+    for (; b->flushed < b->records.size(); ++b->flushed) {
+        const size_t k = b->flushed - first;
+        if (ops[k].done) continue;
+        const KernelEntry* e = ops[k].entry;
+        const LaunchArgs& a = ops[k].args;
+        const AcResult rc = fuse && e->launch ? launch_fused(ops.data(), (uint32_t)n, (uint32_t)k)
+                                              : launch_record(ctx, e, a.binding_count, a.ptr, a.range, a.push, a.grid);
         if (rc != AC_SUCCESS) return fail(ctx, rc, AMEVA_BACKEND_OP_DISPATCH);
         if (b->flags & AC_BATCH_FLAG_DISPATCH_TIMESTAMPS) {
             cudaEvent_t ev;

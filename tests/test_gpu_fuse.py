@@ -1,0 +1,172 @@
+"""Dispatches that leave the host in one launch (csrc/fuse.cu) against the same dispatches submitted one by one: every buffer
+ends with the same bytes, whether the operands allow a fused form or (aliased, overlapping, strided) do not."""
+import struct
+
+import numpy as np
+import pytest
+
+from conftest import load_pkg
+
+pytestmark = pytest.mark.gpu
+pkg = load_pkg()
+rt, qmm = pkg.runtime, pkg.qmm
+
+
+def fbits(v):
+    return struct.unpack("<I", struct.pack("<f", float(v)))[0]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = rt.init()
+    yield c
+    c.destroy()
+
+
+def check(ctx, bufs, ops):
+    """bufs: name -> initial array; ops: (kernel, [name or (name, byte offset[, bytes])], push, grid)."""
+    held = {n: ctx.buffer(data=a) for n, a in bufs.items()}
+
+    def bind(x):
+        return held[x] if isinstance(x, str) else (held[x[0]],) + tuple(x[1:])
+
+    def run(groups, replay=False):
+        for n, a in bufs.items():
+            held[n].write(a)
+        for g in groups:
+            batch = ctx.batch(len(g) + 1)
+            for name, binds, push, grid in g:
+                batch.dispatch(ctx.kernel(name), [bind(b) for b in binds], push, grid)
+            if replay:
+                batch.instantiate()
+                ev = batch.replay()
+            else:
+                ev = batch.submit()
+            ev.wait()
+            ev.destroy()
+            batch.destroy()
+        return {n: held[n].read(np.uint8) for n in bufs}
+
+    alone = run([[op] for op in ops])
+    for got in (run([ops]), run([ops], replay=True)):
+        for n in bufs:
+            assert np.array_equal(alone[n], got[n]), n
+    for b in held.values():
+        b.destroy()
+    return alone
+
+
+ONE = (1, 1, 1)
+
+
+def i2_s(prefix, src, M, N, K, rng, bufs, out, y=None):
+    """The quantize and the product of one I2_S weight."""
+    bufs[prefix + "w"] = rng.integers(0, 256, N * K // 4).astype(np.uint8)
+    for name, size in (("y", M * K * 4), ("q", M * K), ("act", M * 8), ("qeo", 64)):
+        bufs[prefix + name] = np.zeros(size, np.uint8)
+    bufs[out] = np.zeros(M * N, np.float32)
+    return [("bitnet_norm_q8", [src, src, src, y or prefix + "y", prefix + "q", prefix + "act", prefix + "qeo"], [K, 0, 0, 0], (M, 1, 1)),
+            ("bitnet_gemv_i2_s_l32w1", [prefix + "w", prefix + "q", out, prefix + "act"], [K, N, fbits(0.02), 0, M, N], ONE)]
+
+
+@pytest.mark.parametrize("M,K,ns", [(1, 128, (1, 2)), (1, 2560, (2560, 640, 641)), (3, 1152, (33, 7, 64, 9)), (8, 8192, (5, 6)),
+                                    (1, 8320, (40, 41)), (2, 256, (17, 18, 19, 20, 21))])
+def test_bitnet_products_of_one_row(ctx, M, K, ns):
+    rng = np.random.default_rng(K + M)
+    bufs = {"x": rng.standard_normal(M * K).astype(np.float32), "w": rng.standard_normal(K).astype(np.float32),
+            "h": np.zeros(M * K, np.float32)}
+    ops = [("ameva_rms_norm_f32", ["x", "w", "h"], [M, K, fbits(1e-5), 1], ONE)]
+    for j, N in enumerate(ns):
+        ops += i2_s(f"p{j}", "h", M, N, K, rng, bufs, f"o{j}")
+    out = check(ctx, bufs, ops)
+    assert any(out["o0"])
+    # no weight row; the norm in place; a quantize that writes its own source (that one and what follows stay apart)
+    check(ctx, bufs, [("ameva_rms_norm_f32", ["x", "w", "x"], [M, K, fbits(1e-5), 0], ONE)] +
+          [(k, ["x" if b == "h" else b for b in binds], p, g) for k, binds, p, g in ops[1:]])
+    bufs2 = dict(bufs)
+    check(ctx, bufs2, ops[:1] + i2_s("p0", "h", M, ns[0], K, rng, bufs2, "o0", y="h") + ops[3:])
+
+
+@pytest.mark.parametrize("M,N", [(1, 77), (1, 2560), (4, 130)])
+@pytest.mark.parametrize("form", ["ab", "ba", "in place", "onto the activations"])
+def test_bitnet_gate_and_residual(ctx, M, N, form):
+    K = 384
+    rng = np.random.default_rng(N)
+    bufs = {n: rng.standard_normal(M * K).astype(np.float32) for n in ("gate", "up", "act")}
+    bufs["res"], bufs["sum"] = rng.standard_normal(M * N).astype(np.float32), np.zeros(max(M * N, M * K), np.float32)
+    ops = [("ameva_swiglu_f32", ["gate", "up", "act"], [M * K], ONE)] + i2_s("d", "act", M, N, K, rng, bufs, "tmp")
+    a, b, o = {"ab": ("tmp", "res", "sum"), "ba": ("res", "tmp", "sum"), "in place": ("tmp", "res", "res"),
+               "onto the activations": ("tmp", "res", "sum")}[form]
+    if form == "onto the activations":   # the sum overwrites what the product reads: not in one launch
+        ops = [(k, ["sum" if x == "dq" else x for x in binds], p, g) for k, binds, p, g in ops]
+    ops.append(("ameva_add_f32", [a, b, o], [M, N, M], ONE))
+    check(ctx, bufs, ops)
+    check(ctx, bufs, [(ops[0][0], ["gate", "up", "gate"], ops[0][2], ONE)] +     # the gate in place
+          [(k, ["gate" if x == "act" else x for x in binds], p, g) for k, binds, p, g in ops[1:]])
+
+
+def rope(a, d, D, heads, M, pos="pos", neox=1, d_off=0):
+    w = heads * D
+    return ("ameva_rope", [a, pos, pos, d], [D, heads, M, 1, 0, D, w, w * M, d_off, D, w, w * M, 0, 0, D, neox, 0, fbits(0.9), fbits(1.0),
+                                            fbits(0.0), fbits(1.0), 0, 0], ONE)
+
+
+def store(src, cache, width, M, rows, f16=1, a_off=0, node=3):
+    return ("ameva_set_rows", [src, "idx", "status", cache],
+            [width, M, 1, 1, a_off, width, width * M, width * M, 0, 2, 2 * M, 2 * M, 1, 1, 1, rows, 0, width, width * rows, width * rows,
+             f16, node], ONE)
+
+
+@pytest.mark.parametrize("M", [1, 5, 160])
+@pytest.mark.parametrize("D,heads,kv,f16", [(128, 32, 8, 1), (64, 14, 2, 1), (64, 3, 1, 0), (6, 5, 3, 1)])
+def test_ropes_and_cache_writes(ctx, M, D, heads, kv, f16):
+    rng = np.random.default_rng(M + D)
+    rows = 300
+    bufs = {n: rng.standard_normal(M * w * D).astype(np.float32) for n, w in (("q", heads), ("k", kv), ("v", kv), ("qr", heads), ("kr", kv))}
+    bufs["pos"] = rng.integers(0, 4096, M).astype(np.int32)
+    idx = rng.permutation(rows)[:M].astype(np.int64)
+    if M > 1:
+        idx[1] = rows + 7          # reported, not written
+    bufs["idx"], bufs["status"] = idx, np.array([0, 0xFFFFFFFF], np.uint32)
+    bufs["kc"], bufs["vc"] = (rng.standard_normal(rows * kv * D).astype(np.float16 if f16 else np.float32) for _ in range(2))
+    q, k = rope("q", "qr", D, heads, M), rope("k", "kr", D, kv, M)
+    ks, vs = store("kr", "kc", kv * D, M, rows, f16), store("v", "vc", kv * D, M, rows, f16, node=9)
+    out = check(ctx, bufs, [q, k, ks, vs])
+    assert list(out["status"].view(np.uint32)) == ([2, 3] if M > 1 else [0, 0xFFFFFFFF])
+    for ops in ([q, k, vs, ks], [k, ks, q, vs], [q, k], [ks, vs], [k, vs, q, ks, rope("q", "kr2", D, heads, M)],
+                [rope("q", "q", D, heads, M, neox=0), rope("k", "k", D, kv, M, neox=0), store("k", "kc", kv * D, M, rows, f16), vs],
+                [q, rope("qr", "q", D, heads, M), k, ks],          # the second reads what the first writes
+                [k, store("kr", "kc", kv * D, M, rows, f16), store("kr", "vc", kv * D, M, rows, f16)],   # one result stored twice
+                [k, rope("k", "k", D, kv, M), vs]):                # writes what the first reads
+        b = dict(bufs, kr2=np.zeros(M * heads * D, np.float32))
+        check(ctx, b, ops)
+
+
+QUANT = {("a8", 0): "ameva_quant_a8", ("a8", 1): "ameva_quant_a8_f16", ("a8b", 0): "ameva_quant_a8b", ("a8b", 1): "ameva_quant_a8b_f16"}
+
+
+def quant(scheme, f16, src, dst, M, K, bufs, stride=None, mode=0):
+    ab = M * (K // 256) * 48 if scheme == "a8b" else M * (K // 32) * 4
+    for name, size in ((dst + "q", M * K), (dst + "d", ab), (dst + "h", M * K * 2), (dst + "e", M * 4)):
+        bufs[name] = np.zeros(size, np.uint8)
+    return (QUANT[scheme, f16], [src, dst + "q", dst + "d"] + ([dst + "h", dst + "e"] if f16 else []), [M, K, stride or K, mode], ONE)
+
+
+@pytest.mark.parametrize("scheme", ["a8", "a8b"])
+@pytest.mark.parametrize("M,K,f16", [(1, 256, 0), (1, 4864, 0), (8, 1024, 0), (1, 11008, 0), (9, 256, 1), (40, 2304, 1), (12, 14336, 1)])
+def test_quantizes_of_the_same_rows(ctx, scheme, M, K, f16):
+    rng = np.random.default_rng(K + M)
+    bufs = {n: (rng.standard_normal(M * K) * 2).astype(np.float32) for n in ("x", "gate", "up")}
+    bufs.update(y=np.zeros(M * K, np.float32), w=rng.standard_normal(K).astype(np.float32))
+    qs = [quant(scheme, f16, "y", f"m{j}", M, K, bufs) for j in range(5)]
+    other = quant("a8b" if scheme == "a8" and K % 256 == 0 else "a8", f16, "y", "o", M, K, bufs)
+    gate = ("ameva_swiglu_f32", ["gate", "up", "y"], [M * K], ONE)
+    norm = (f"ameva_rms_norm_quant_{scheme}", ["x", "w", "y", "nq", "nd", "nh", "ne"], [M, K, K, 0, fbits(1e-5), 1, f16], (M, 1, 1))
+    for a, b in zip("qdhe", "qdhe"):
+        bufs["n" + a] = np.zeros_like(bufs["m0" + b])
+    out = check(ctx, bufs, [gate] + qs[:1])
+    assert any(out["m0q"])
+    for ops in ([gate] + qs, [gate, other] + qs, [norm] + qs, [norm, other, qs[0]], [gate, quant(scheme, f16, "y", "m0", M, K, bufs, mode=1), qs[1]],
+                [(gate[0], ["gate", "up", "gate"], gate[2], ONE)] + [(q[0], ["gate"] + q[1][1:], q[2], ONE) for q in qs[:2]],
+                [norm, (qs[0][0], ["y"] + norm[1][3:3 + len(qs[0][1]) - 1], qs[0][2], ONE), qs[1]]):     # the same destination twice
+        check(ctx, bufs, ops)
