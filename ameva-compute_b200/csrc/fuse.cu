@@ -12,6 +12,8 @@ AcResult launch_bitnet_gemm_i2_s(const LaunchArgs&);
 AcResult launch_bitnet_gemv_i2_s(const LaunchArgs&);
 AcResult launch_bitnet_norm_q8(const LaunchArgs&);
 AcResult launch_rms_norm_f32(const LaunchArgs&);
+AcResult launch_rope(const LaunchArgs&);
+AcResult launch_set_rows(const LaunchArgs&);
 AcResult launch_swiglu_f32(const LaunchArgs&);
 
 namespace {
@@ -178,6 +180,57 @@ AcResult fuse_bitnet_gemv(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
     return launch_bitnet_gemv_i2_s_group(member, count, add, swapped);
 }
 
+// ---- ROPEs and cache writes in a row ----
+// Ranges an operation reads (ROPE: source, positions, factors; SET_ROWS: source, indices); both write binding 3. A status
+// binding (SET_ROWS 2) takes atomics only, so several operations may share it.
+bool row_op_writes_meet(const LaunchArgs& w, const LaunchArgs& other, bool other_rope, bool except_source) {
+    for (uint32_t b = 0; b < 4u; ++b) {
+        if (b == 0u && except_source) continue;
+        if (b == 2u && other_rope && !other.push[16]) continue;   // (no frequency factors: the binding is not read)
+        if (overlap(w.ptr[3], w.range[3], other.ptr[b], other.range[b])) return true;
+    }
+    return false;
+}
+bool status_meets(const LaunchArgs& set, const LaunchArgs& other, bool other_rope) {
+    for (uint32_t b = 0; b < 4u; ++b)
+        if ((b != 2u || (other_rope && other.push[16])) && overlap(set.ptr[2], set.range[2], other.ptr[b], other.range[b])) return true;
+    return false;
+}
+
+AcResult fuse_row_ops(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
+    const LaunchArgs *rope[2], *store[2] = {nullptr, nullptr}, *set[2];
+    uint32_t n_rope = 0, n_set = 0, count = 0, at[6];
+    for (uint32_t j = i; j < n && count < 6u; ++j) {
+        if (ops[j].done) continue;
+        const bool r = is(ops[j], launch_rope);
+        if (!r && !is(ops[j], launch_set_rows)) break;
+        const LaunchArgs& p = ops[j].args;
+        if (!row_op_serves(p, r)) break;
+        int chain = -1;
+        if (!r)
+            for (uint32_t k = 0; k < n_rope; ++k)
+                if (!store[k] && rope_feeds_set_rows(*rope[k], p)) chain = (int)k;
+        if (r ? n_rope == 2u : (chain < 0 && n_set == 2u)) break;
+        bool ok = true;
+        for (uint32_t k = 0; k < count && ok; ++k) {
+            const LaunchArgs& o = ops[at[k]].args;
+            const bool o_rope = is(ops[at[k]], launch_rope), source = chain >= 0 && &o == rope[chain];
+            // neither writes what the other reads or writes (the rotated rows that p stores excepted)
+            ok = !row_op_writes_meet(p, o, o_rope, false) && !row_op_writes_meet(o, p, r, source) &&
+                 (r || !status_meets(p, o, o_rope)) && (o_rope || !status_meets(o, p, r));
+        }
+        if (!ok) break;
+        if (r) rope[n_rope++] = &p;
+        else if (chain >= 0) store[chain] = &p;
+        else set[n_set++] = &p;
+        at[count++] = j;
+    }
+    if (count < 2u) return AC_SUCCESS;
+    *taken = true;
+    for (uint32_t k = 0; k < count; ++k) ops[at[k]].done = true;
+    return launch_row_ops(rope, store, n_rope, set, n_set);
+}
+
 }  // namespace
 
 AcResult launch_fused(FuseOp* ops, uint32_t n, uint32_t i) {
@@ -187,6 +240,8 @@ AcResult launch_fused(FuseOp* ops, uint32_t n, uint32_t i) {
         rc = fuse_bitnet_rows(ops, n, i, &taken);
     else if (is(ops[i], launch_bitnet_gemv_i2_s))
         rc = fuse_bitnet_gemv(ops, n, i, &taken);
+    else if (is(ops[i], launch_rope) || is(ops[i], launch_set_rows))
+        rc = fuse_row_ops(ops, n, i, &taken);
     if (taken) return rc;
     ops[i].done = true;
     return ops[i].entry->launch(ops[i].args);

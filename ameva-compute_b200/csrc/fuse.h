@@ -31,4 +31,11 @@ AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const L
 AcResult check_bitnet_gemv_i2_s(const LaunchArgs& a);
 AcResult launch_bitnet_gemv_i2_s_group(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped);
 
+// ROPE / SET_ROWS of the same new positions (layer_ops.cu): up to two of each beside one another, and per ROPE a SET_ROWS of
+// its result (store[i], nullptr: none)
+bool row_op_serves(const LaunchArgs& a, bool rope);
+bool rope_feeds_set_rows(const LaunchArgs& rope, const LaunchArgs& set);
+AcResult launch_row_ops(const LaunchArgs* const* rope, const LaunchArgs* const* store, uint32_t n_rope, const LaunchArgs* const* set,
+                        uint32_t n_set);
+
 }  // namespace amv

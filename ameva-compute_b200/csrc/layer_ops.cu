@@ -81,22 +81,56 @@ __device__ __forceinline__ void st_pair(T* d, uint64_t e0, uint64_t e1, bool vec
     st_elem(d, e1, x1);
 }
 
-// CTA: one position (blockIdx.x / chunks) and `heads_per_cta` heads; threads: jt consecutive pairs x 256 / jt head lanes.
-// vec: f32 pairs (e0, e0 + 1) start on 8 bytes in source and destination.
+// How the pairs are dealt to a grid: a CTA takes one position and `heads_per_cta` heads (`chunks` CTAs per position); threads:
+// jt consecutive pairs x 256 / jt head lanes. vec: f32 pairs (e0, e0 + 1) start on 8 bytes in source and destination.
+struct RopePlan {
+    uint32_t jt, chunks, heads_per_cta, vec, ctas;
+};
+
+struct SetRowsArgs {
+    uint32_t nc, nr, ne02, ne03;
+    uint32_t a_off, a_s1, a_s2, a_s3;
+    uint32_t i_off, i_s0, i_s1, i_s2;
+    uint32_t i_ne1, i_ne2, idx64, dst_rows;
+    uint32_t d_off, d_s1, d_s2, d_s3;
+    uint32_t dst_f16, node;
+};
+// A SET_ROWS whose source is the rotated rows (the key cache write), done by the threads that rotate: row i2 of the rotated
+// positions, heads side by side in a row. cache == nullptr: none.
+struct RopeStore {
+    const uint32_t* idx;
+    uint32_t* status;
+    void* cache;
+    SetRowsArgs st;
+};
+
 template <typename T>
-__global__ void __launch_bounds__(256) rope_kernel(const T* a, const int32_t* __restrict__ pos,
-                                                   const float* __restrict__ ff, T* d, const RopeArgs pc, uint32_t jt,
-                                                   uint32_t chunks, uint32_t heads_per_cta, uint32_t vec) {
-    pdl_trigger();
-    pdl_wait();
+__device__ __forceinline__ void rope_body(const T* a, const int32_t* __restrict__ pos, const float* __restrict__ ff, T* d,
+                                          const RopeArgs& pc, const RopePlan& plan, const uint32_t block, const RopeStore* store) {
+    const uint32_t jt = plan.jt, chunks = plan.chunks, heads_per_cta = plan.heads_per_cta, vec = plan.vec;
     const uint32_t half_ne0 = pc.ne0 >> 1, hg = 256u / jt, j0 = threadIdx.x & (jt - 1u), hl = threadIdx.x / jt;
-    const uint32_t row = blockIdx.x / chunks, chunk = blockIdx.x - row * chunks;
+    const uint32_t row = block / chunks, chunk = block - row * chunks;
     const uint32_t i3 = row / pc.ne2, i2 = row - i3 * pc.ne2;
     const uint64_t a23 = pc.a_off + (uint64_t)i2 * pc.a_s2 + (uint64_t)i3 * pc.a_s3;
     const uint64_t d23 = pc.d_off + (uint64_t)i2 * pc.d_s2 + (uint64_t)i3 * pc.d_s3;
     const uint32_t h_end = min(pc.ne1, (chunk + 1u) * heads_per_cta);
     const float theta0 = (float)pos[pc.pos_off + i2], ts = u2f(pc.theta_scale);
     const float freq_scale = u2f(pc.freq_scale), ext_factor = u2f(pc.ext_factor);
+    bool stored = store && store->cache;
+    uint64_t c_row = 0;   // element of the cache row
+    if (stored) {
+        const SetRowsArgs& st = store->st;
+        const uint64_t iw = st.i_off + (uint64_t)i2 * st.i_s0;
+        const uint32_t to = store->idx[iw], high = st.idx64 ? store->idx[iw + 1u] : 0u;
+        if (to >= st.dst_rows || high != 0u) {
+            stored = false;
+            if (chunk == 0u && threadIdx.x == 0u) {
+                atomicAdd(store->status, 1u);
+                atomicMin(store->status + 1, st.node);
+            }
+        }
+        c_row = st.d_off + (uint64_t)to * st.d_s1;
+    }
     for (uint32_t j = j0; j < half_ne0; j += jt) {
         const bool rotated = 2u * j < pc.n_dims;   // past the rotated part: copied
         const bool neox = rotated && pc.mode_neox;
@@ -136,9 +170,29 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* a, const int32_t* __
                 const float y0 = rotated ? __fsub_rn(__fmul_rn(x0[k], cos_t), __fmul_rn(x1[k], sin_t)) : x0[k];
                 const float y1 = rotated ? __fadd_rn(__fmul_rn(x0[k], sin_t), __fmul_rn(x1[k], cos_t)) : x1[k];
                 st_pair(d, db + e0, db + e1, pair, y0, y1);
+                if (stored) {
+                    const uint64_t c = c_row + (uint64_t)h * pc.ne0;
+                    if (store->st.dst_f16) {
+                        __half* cache = (__half*)store->cache;
+                        cache[c + e0] = __float2half_rn(y0);
+                        cache[c + e1] = __float2half_rn(y1);
+                    } else {
+                        float* cache = (float*)store->cache;
+                        cache[c + e0] = y0;
+                        cache[c + e1] = y1;
+                    }
+                }
             }
         }
     }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) rope_kernel(const T* a, const int32_t* __restrict__ pos, const float* __restrict__ ff, T* d,
+                                                   const RopeArgs pc, const RopePlan plan) {
+    pdl_trigger();
+    pdl_wait();
+    rope_body<T>(a, pos, ff, d, pc, plan, blockIdx.x, nullptr);
 }
 
 // the largest element index a strided 4-D walk reaches, + 1
@@ -150,7 +204,7 @@ static uint64_t span_elems(uint32_t off, uint32_t ne0, uint32_t ne1, uint32_t ne
 // ameva_rope / ameva_rope_f16: bindings 0 source, 1 positions i32, 2 frequency factors f32 (any range when has_ff = 0),
 // 3 destination; push = RopeArgs (23 words)
 template <typename T>
-static AcResult launch_rope_t(const LaunchArgs& a) {
+static AcResult check_rope_t(const LaunchArgs& a, RopeArgs* out, RopePlan* plan) {
     RopeArgs pc;
     memcpy(&pc, a.push, sizeof(pc));
     if (!pc.ne0 || (pc.ne0 & 1u) || !pc.ne1 || !pc.ne2 || !pc.ne3 || pc.n_dims > pc.ne0 || (pc.n_dims & 1u) ||
@@ -168,14 +222,24 @@ static AcResult launch_rope_t(const LaunchArgs& a) {
     // few positions (token generation): one head per thread, so that the heads spread over the SMs; many: all the heads a
     // thread can carry, so that sine and cosine are formed once
     const uint64_t sms = a.sm_count > 0 ? (uint64_t)a.sm_count : 148u;
-    const uint32_t heads_per_cta = rows >= sms ? kRopeHeads * hg : hg;
-    const uint32_t chunks = (uint32_t)(((uint64_t)pc.ne1 + heads_per_cta - 1u) / heads_per_cta);
-    if (rows * chunks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
-    const bool vec = sizeof(T) == 4 && !((pc.a_off | pc.a_s1 | pc.a_s2 | pc.a_s3 | pc.d_off | pc.d_s1 | pc.d_s2 | pc.d_s3) & 1u) &&
-                     !(((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[3]) & 7u);
-    launch_pdl(rope_kernel<T>, dim3((unsigned)(rows * chunks)), dim3(256), 0, a.stream, (const T*)a.ptr[0],
-               (const int32_t*)a.ptr[1], (const float*)a.ptr[2], (T*)a.ptr[3], pc, jt, chunks, heads_per_cta,
-               (uint32_t)vec);
+    plan->jt = jt;
+    plan->heads_per_cta = rows >= sms ? kRopeHeads * hg : hg;
+    plan->chunks = (uint32_t)(((uint64_t)pc.ne1 + plan->heads_per_cta - 1u) / plan->heads_per_cta);
+    if (rows * plan->chunks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
+    plan->ctas = (uint32_t)(rows * plan->chunks);
+    plan->vec = sizeof(T) == 4 && !((pc.a_off | pc.a_s1 | pc.a_s2 | pc.a_s3 | pc.d_off | pc.d_s1 | pc.d_s2 | pc.d_s3) & 1u) &&
+                !(((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[3]) & 7u);
+    *out = pc;
+    return AC_SUCCESS;
+}
+template <typename T>
+static AcResult launch_rope_t(const LaunchArgs& a) {
+    RopeArgs pc;
+    RopePlan plan;
+    const AcResult rc = check_rope_t<T>(a, &pc, &plan);
+    if (rc != AC_SUCCESS) return rc;
+    launch_pdl(rope_kernel<T>, dim3(plan.ctas), dim3(256), 0, a.stream, (const T*)a.ptr[0], (const int32_t*)a.ptr[1],
+               (const float*)a.ptr[2], (T*)a.ptr[3], pc, plan);
     return check_launch();
 }
 AcResult launch_rope(const LaunchArgs& a) { return launch_rope_t<float>(a); }
@@ -239,15 +303,6 @@ AcResult launch_get_rows(const LaunchArgs& a) {
 // words (i_s0 = 2 for i64; a non-zero high word counts as out of range). The indices repeat over dimensions 2 and 3.
 // Out-of-range indices are not written and are reported as in GET_ROWS.
 // ---------------------------------------------------------------------------------------------------------------------
-struct SetRowsArgs {
-    uint32_t nc, nr, ne02, ne03;
-    uint32_t a_off, a_s1, a_s2, a_s3;
-    uint32_t i_off, i_s0, i_s1, i_s2;
-    uint32_t i_ne1, i_ne2, idx64, dst_rows;
-    uint32_t d_off, d_s1, d_s2, d_s3;
-    uint32_t dst_f16, node;
-};
-
 __global__ void __launch_bounds__(256) set_rows_kernel(const float* __restrict__ a, const uint32_t* __restrict__ idx,
                                                        uint32_t* status, void* d, const SetRowsArgs pc) {
     pdl_trigger();
@@ -279,12 +334,8 @@ __global__ void __launch_bounds__(256) set_rows_kernel(const float* __restrict__
 // The same with one CTA per span of kSetRowsSpan columns of one row: the index is read and checked once, four columns (16
 // bytes in, 16 or 8 out) per thread. One thread per element with five 64-bit divisions took 7 us for 512 rows of 1024.
 constexpr uint32_t kSetRowsThreads = 256, kSetRowsSpan = 4u * kSetRowsThreads;
-__global__ void __launch_bounds__(kSetRowsThreads) set_rows_vec_kernel(const float* __restrict__ a, const uint32_t* __restrict__ idx,
-                                                                       uint32_t* status, void* d, const SetRowsArgs pc,
-                                                                       uint32_t spans) {
-    pdl_trigger();
-    pdl_wait();
-    uint32_t t = blockIdx.x;
+__device__ __forceinline__ void set_rows_vec_body(const float* __restrict__ a, const uint32_t* __restrict__ idx, uint32_t* status,
+                                                  void* d, const SetRowsArgs& pc, uint32_t spans, uint32_t t) {
     const uint32_t span = t % spans;
     t /= spans;
     const uint32_t r = t % pc.nr;
@@ -314,8 +365,17 @@ __global__ void __launch_bounds__(kSetRowsThreads) set_rows_vec_kernel(const flo
     }
 }
 
+__global__ void __launch_bounds__(kSetRowsThreads) set_rows_vec_kernel(const float* __restrict__ a, const uint32_t* __restrict__ idx,
+                                                                       uint32_t* status, void* d, const SetRowsArgs pc,
+                                                                       uint32_t spans) {
+    pdl_trigger();
+    pdl_wait();
+    set_rows_vec_body(a, idx, status, d, pc, spans, blockIdx.x);
+}
+
 // ameva_set_rows: bindings 0 src0 f32, 1 indices (words), 2 status (>= 8 bytes), 3 dst; push = SetRowsArgs (22 words)
-AcResult launch_set_rows(const LaunchArgs& a) {
+// vec_ctas: the grid of the vector form where it serves the operands, else 0
+static AcResult check_set_rows_args(const LaunchArgs& a, SetRowsArgs* out, uint32_t* spans_out, uint32_t* vec_ctas) {
     SetRowsArgs pc;
     memcpy(&pc, a.push, sizeof(pc));
     if (!pc.nc || !pc.nr || !pc.ne02 || !pc.ne03 || !pc.i_ne1 || !pc.i_ne2 || !pc.dst_rows || pc.idx64 > 1u ||
@@ -329,16 +389,122 @@ AcResult launch_set_rows(const LaunchArgs& a) {
         return AC_ERR_INVALID_BUFFER_SIZE;
     // rows of whole, aligned pieces of four columns
     const uint64_t spans = ((uint64_t)pc.nc + kSetRowsSpan - 1u) / kSetRowsSpan, ctas = spans * pc.nr * pc.ne02 * pc.ne03;
-    if (!((pc.nc | pc.a_off | pc.a_s1 | pc.a_s2 | pc.a_s3 | pc.d_off | pc.d_s1 | pc.d_s2 | pc.d_s3) & 3u) &&
-        !((uintptr_t)a.ptr[0] & 15u) && !((uintptr_t)a.ptr[3] & (pc.dst_f16 ? 7u : 15u)) && ctas <= 0x7FFFFFFFull &&
-        pc.nc <= 0x7FFFFFFFu) {
-        launch_pdl(set_rows_vec_kernel, dim3((unsigned)ctas), dim3(kSetRowsThreads), 0, a.stream, (const float*)a.ptr[0],
-                   (const uint32_t*)a.ptr[1], (uint32_t*)a.ptr[2], (void*)a.ptr[3], pc, (uint32_t)spans);
+    const bool vec = !((pc.nc | pc.a_off | pc.a_s1 | pc.a_s2 | pc.a_s3 | pc.d_off | pc.d_s1 | pc.d_s2 | pc.d_s3) & 3u) &&
+                     !((uintptr_t)a.ptr[0] & 15u) && !((uintptr_t)a.ptr[3] & (pc.dst_f16 ? 7u : 15u)) && ctas <= 0x7FFFFFFFull &&
+                     pc.nc <= 0x7FFFFFFFu;
+    *out = pc;
+    *spans_out = (uint32_t)spans;
+    *vec_ctas = vec ? (uint32_t)ctas : 0u;
+    return AC_SUCCESS;
+}
+AcResult launch_set_rows(const LaunchArgs& a) {
+    SetRowsArgs pc;
+    uint32_t spans, ctas;
+    const AcResult rc = check_set_rows_args(a, &pc, &spans, &ctas);
+    if (rc != AC_SUCCESS) return rc;
+    if (ctas) {
+        launch_pdl(set_rows_vec_kernel, dim3(ctas), dim3(kSetRowsThreads), 0, a.stream, (const float*)a.ptr[0],
+                   (const uint32_t*)a.ptr[1], (uint32_t*)a.ptr[2], (void*)a.ptr[3], pc, spans);
         return check_launch();
     }
     const uint64_t total = (uint64_t)pc.nc * pc.nr * pc.ne02 * pc.ne03;
     launch_pdl(set_rows_kernel, dim3((unsigned)((total + 255u) / 256u)), dim3(256), 0, a.stream, (const float*)a.ptr[0],
                (const uint32_t*)a.ptr[1], (uint32_t*)a.ptr[2], (void*)a.ptr[3], pc);
+    return check_launch();
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// The row operations between a layer's q / k / v products and its attention in one launch: up to two ROPEs, up to two
+// SET_ROWS beside them, and a SET_ROWS of rotated rows done by the threads that rotate them. None of them reads what another
+// one writes (fuse.cu checks the ranges), so the CTAs of all of them form one grid. Each is a launch of 2-4 us for well under
+// a microsecond of work at token generation.
+// ---------------------------------------------------------------------------------------------------------------------
+struct RowOps {
+    uint32_t end[4];   // CTAs of rope 0, rope 1, set 0, set 1, cumulative
+    const float* a[4];
+    const int32_t* pos[2];
+    const float* ff[2];
+    float* d[2];
+    RopeArgs rope[2];
+    RopePlan plan[2];
+    RopeStore store[2];
+    const uint32_t* idx[2];
+    uint32_t* status[2];
+    void* cache[2];
+    SetRowsArgs set[2];
+    uint32_t spans[2];
+};
+
+__global__ void __launch_bounds__(256) row_ops_kernel(const __grid_constant__ RowOps g) {
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t b = blockIdx.x;
+    if (b < g.end[0]) rope_body<float>(g.a[0], g.pos[0], g.ff[0], g.d[0], g.rope[0], g.plan[0], b, &g.store[0]);
+    else if (b < g.end[1]) rope_body<float>(g.a[1], g.pos[1], g.ff[1], g.d[1], g.rope[1], g.plan[1], b - g.end[0], &g.store[1]);
+    else if (b < g.end[2]) set_rows_vec_body(g.a[2], g.idx[0], g.status[0], g.cache[0], g.set[0], g.spans[0], b - g.end[1]);
+    else set_rows_vec_body(g.a[3], g.idx[1], g.status[1], g.cache[1], g.set[1], g.spans[1], b - g.end[2]);
+}
+
+bool row_op_serves(const LaunchArgs& a, bool rope) {
+    if (rope) {
+        RopeArgs pc;
+        RopePlan plan;
+        return check_rope_t<float>(a, &pc, &plan) == AC_SUCCESS;
+    }
+    SetRowsArgs pc;
+    uint32_t spans, ctas;
+    return check_set_rows_args(a, &pc, &spans, &ctas) == AC_SUCCESS && ctas;
+}
+
+// `set` writes the rows that `rope` produces: one row per position, its heads side by side
+bool rope_feeds_set_rows(const LaunchArgs& rope, const LaunchArgs& set) {
+    RopeArgs r;
+    SetRowsArgs st;
+    memcpy(&r, rope.push, sizeof(r));
+    memcpy(&st, set.push, sizeof(st));
+    return (const char*)set.ptr[0] + 4ull * st.a_off == (const char*)rope.ptr[3] + 4ull * r.d_off && r.ne3 == 1u &&
+           (r.ne1 == 1u || r.d_s1 == r.ne0) && (uint64_t)st.nc == (uint64_t)r.ne0 * r.ne1 && st.nr == r.ne2 && st.ne02 == 1u &&
+           st.ne03 == 1u && (st.nr == 1u || st.a_s1 == r.d_s2);
+}
+
+AcResult launch_row_ops(const LaunchArgs* const* rope, const LaunchArgs* const* store, uint32_t n_rope, const LaunchArgs* const* set,
+                        uint32_t n_set) {
+    RowOps g;
+    memset(&g, 0, sizeof(g));
+    uint64_t ctas = 0;
+    for (uint32_t i = 0; i < 2u; ++i) {
+        if (i < n_rope) {
+            const LaunchArgs& a = *rope[i];
+            const AcResult rc = check_rope_t<float>(a, &g.rope[i], &g.plan[i]);
+            if (rc != AC_SUCCESS) return rc;
+            g.a[i] = (const float*)a.ptr[0];
+            g.pos[i] = (const int32_t*)a.ptr[1];
+            g.ff[i] = (const float*)a.ptr[2];
+            g.d[i] = (float*)a.ptr[3];
+            ctas += g.plan[i].ctas;
+            if (store[i]) {
+                g.store[i] = {(const uint32_t*)store[i]->ptr[1], (uint32_t*)store[i]->ptr[2], store[i]->ptr[3], {}};
+                memcpy(&g.store[i].st, store[i]->push, sizeof(SetRowsArgs));
+            }
+        }
+        g.end[i] = (uint32_t)ctas;
+    }
+    for (uint32_t i = 0; i < 2u; ++i) {
+        if (i < n_set) {
+            const LaunchArgs& a = *set[i];
+            uint32_t n;
+            const AcResult rc = check_set_rows_args(a, &g.set[i], &g.spans[i], &n);
+            if (rc != AC_SUCCESS || !n) return rc != AC_SUCCESS ? rc : AC_ERR_KERNEL_ARG_INVALID;
+            g.a[2 + i] = (const float*)a.ptr[0];
+            g.idx[i] = (const uint32_t*)a.ptr[1];
+            g.status[i] = (uint32_t*)a.ptr[2];
+            g.cache[i] = a.ptr[3];
+            ctas += n;
+        }
+        g.end[2 + i] = (uint32_t)ctas;
+    }
+    if (ctas > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
+    launch_pdl(row_ops_kernel, dim3((unsigned)ctas), dim3(256), 0, n_rope ? rope[0]->stream : set[0]->stream, g);
     return check_launch();
 }
 
