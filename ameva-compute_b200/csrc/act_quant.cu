@@ -14,14 +14,34 @@
 
 namespace amv {
 
+// Where a quantize kernel writes: one destination, or up to four equal ones (products of one graph that read the same rows and
+// keep scratch of their own: one pass over the rows instead of one launch for each). ah / ae: the tensor-core operand.
+struct QuantDst {
+    int8_t* aq;
+    uint8_t* ad;
+    __half* ah;
+    float* ae;
+};
+struct QuantDsts {
+    uint32_t n;
+    QuantDst d[kFuseMax];
+};
+// What is quantized: the rows at src; or, SWIGLU, silu(src) * up, written to act as ameva_swiglu_f32 writes it (rows of K
+// floats, no gaps in any of the three).
+struct GateArgs {
+    const float* up;
+    float* act;
+};
+
 // ---------------------------------------------------------------------------------------------------------------------
 // per-32: 8 lanes per unit, one float4 each (128 B coalesced per unit, 4 units per warp).
 //   d = amax / 127 (f32); id = d ? 1/d : 0; q = clamp(round(x*id), +-127); stored d = fp16(d) (what the dot uses).
 //   round_mode 0 = ties-to-even (reference shaders, ggml SIMD quantizers), 1 = ties-away (ggml quantize_row_q8_0_ref).
 // ---------------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) quant_q8_0_kernel(const float* __restrict__ src, int8_t* __restrict__ aq,
-                                                         uint32_t* __restrict__ ad, uint32_t M, uint32_t K,
-                                                         uint32_t src_stride, uint32_t round_mode) {
+template <bool SWIGLU>
+__global__ void __launch_bounds__(256) quant_q8_0_kernel(const float* __restrict__ src, const QuantDsts dst, uint32_t M,
+                                                         uint32_t K, uint32_t src_stride, uint32_t round_mode,
+                                                         const GateArgs ga) {
     pdl_trigger();   // the mul_mat behind this kernel may be scheduled already (it can request its weights meanwhile; it
                      // waits for this grid before reading the quantized activations)
     pdl_wait();      // the activations may come from the kernel before (it let this one be scheduled early)
@@ -32,14 +52,23 @@ __global__ void __launch_bounds__(256) quant_q8_0_kernel(const float* __restrict
     const bool live = gi < total;
     const uint32_t m = live ? (uint32_t)(gi / U) : 0u;
     const uint32_t u = live ? (uint32_t)(gi - (uint64_t)m * U) : 0u;
+    const size_t at = (size_t)m * src_stride + 32u * u + 4u * sub;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) x = *reinterpret_cast<const float4*>(src + (size_t)m * src_stride + 32u * u + 4u * sub);
+    if (live) x = *reinterpret_cast<const float4*>(src + at);
+    if (SWIGLU && live) {
+        const float4 y = *reinterpret_cast<const float4*>(ga.up + at);
+        x = make_float4(swiglu_f32(x.x, y.x), swiglu_f32(x.y, y.y), swiglu_f32(x.z, y.z), swiglu_f32(x.w, y.w));
+        *reinterpret_cast<float4*>(ga.act + at) = x;
+    }
     int q[4], s;
     float d;
     quant_unit_q8_0(x, round_mode, q, d, s);
     if (live) {
-        reinterpret_cast<uint32_t*>(aq + (size_t)m * K + 32u * u)[sub] = pack_q4(q);
-        if (sub == 0) ad[(size_t)m * U + u] = scale_word_q8_0(d, s);
+        const uint32_t word = scale_word_q8_0(d, s);
+        for (uint32_t i = 0; i < dst.n; ++i) {
+            reinterpret_cast<uint32_t*>(dst.d[i].aq + (size_t)m * K + 32u * u)[sub] = pack_q4(q);
+            if (sub == 0) reinterpret_cast<uint32_t*>(dst.d[i].ad)[(size_t)m * U + u] = word;
+        }
     }
 }
 
@@ -50,9 +79,9 @@ __global__ void __launch_bounds__(256) quant_q8_0_kernel(const float* __restrict
 //   mode 1 (ameva_quant_a8b.comp): d = amax/127, q = clamp(roundEven(x * (1/d)), +-127).
 //   bsums[j] = sum of q over elements 16j..16j+15.
 // ---------------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) quant_q8_K_kernel(const float* __restrict__ src, int8_t* __restrict__ aq,
-                                                         uint8_t* __restrict__ ab, uint32_t M, uint32_t K,
-                                                         uint32_t src_stride, uint32_t mode) {
+template <bool SWIGLU>
+__global__ void __launch_bounds__(256) quant_q8_K_kernel(const float* __restrict__ src, const QuantDsts dst, uint32_t M,
+                                                         uint32_t K, uint32_t src_stride, uint32_t mode, const GateArgs ga) {
     pdl_trigger();   // the mul_mat behind this kernel may be scheduled already (it can request its weights meanwhile; it
                      // waits for this grid before reading the quantized activations)
     pdl_wait();      // the activations may come from the kernel before (it let this one be scheduled early)
@@ -63,10 +92,18 @@ __global__ void __launch_bounds__(256) quant_q8_K_kernel(const float* __restrict
     if (gi >= total) return;  // whole warps leave together
     const uint32_t m = (uint32_t)(gi / B);
     const uint32_t b = (uint32_t)(gi - (uint64_t)m * B);
-    const float* p = src + (size_t)m * src_stride + 256u * b + 8u * lane;
-    const float4 x0 = *reinterpret_cast<const float4*>(p);
-    const float4 x1 = *reinterpret_cast<const float4*>(p + 4);
-    const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    const size_t at = (size_t)m * src_stride + 256u * b + 8u * lane;
+    const float4 x0 = *reinterpret_cast<const float4*>(src + at);
+    const float4 x1 = *reinterpret_cast<const float4*>(src + at + 4);
+    float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    if constexpr (SWIGLU) {
+        const float4 y0 = *reinterpret_cast<const float4*>(ga.up + at), y1 = *reinterpret_cast<const float4*>(ga.up + at + 4);
+        const float y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = swiglu_f32(x[i], y[i]);
+        *reinterpret_cast<float4*>(ga.act + at) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4*>(ga.act + at + 4) = make_float4(x[4], x[5], x[6], x[7]);
+    }
     int q[8];
     float d;
     quant_block_q8_K(x, mode, lane, q, d);
@@ -78,14 +115,16 @@ __global__ void __launch_bounds__(256) quant_q8_K_kernel(const float* __restrict
         w0 |= (uint32_t)(q[i] & 0xFF) << (8 * i);
         w1 |= (uint32_t)(q[i + 4] & 0xFF) << (8 * i);
     }
-    *reinterpret_cast<uint2*>(aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
     s += __shfl_xor_sync(0xffffffffu, s, 1);  // lanes 2j, 2j+1 -> 16-element group j
-    uint8_t* blk = ab + ((size_t)m * B + b) * kABBytes;
-    if ((lane & 1u) == 0u) reinterpret_cast<int16_t*>(blk)[lane >> 1] = (int16_t)s;
-    if (lane == 0) {
-        *reinterpret_cast<float*>(blk + 32) = d;
-        *reinterpret_cast<uint32_t*>(blk + 36) = 0u;
-        *reinterpret_cast<uint2*>(blk + 40) = make_uint2(0u, 0u);
+    for (uint32_t i = 0; i < dst.n; ++i) {
+        *reinterpret_cast<uint2*>(dst.d[i].aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
+        uint8_t* blk = dst.d[i].ad + ((size_t)m * B + b) * kABBytes;
+        if ((lane & 1u) == 0u) reinterpret_cast<int16_t*>(blk)[lane >> 1] = (int16_t)s;
+        if (lane == 0) {
+            *reinterpret_cast<float*>(blk + 32) = d;
+            *reinterpret_cast<uint32_t*>(blk + 36) = 0u;
+            *reinterpret_cast<uint2*>(blk + 40) = make_uint2(0u, 0u);
+        }
     }
 }
 
@@ -146,11 +185,14 @@ __device__ __forceinline__ double block_sum_f64(double v, double* red) {
     return r;
 }
 
-template <int SCHEME, int J, bool NORM = false>
-__global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float* __restrict__ src, int8_t* __restrict__ aq,
-                                                                     uint8_t* __restrict__ ad, __half* __restrict__ ah,
-                                                                     float* __restrict__ ae, uint32_t K,
-                                                                     uint32_t src_stride, uint32_t mode, const NormArgs na) {
+// PRE: ROWS_PLAIN, ROWS_NORM (na) or ROWS_SWIGLU (na.w = up, na.y = act, rows of K floats).
+enum RowsPre { ROWS_PLAIN, ROWS_NORM, ROWS_SWIGLU };
+
+template <int SCHEME, int J, int PRE = ROWS_PLAIN>
+__global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float* __restrict__ src, const QuantDsts dst,
+                                                                     uint32_t K, uint32_t src_stride, uint32_t mode,
+                                                                     const NormArgs na) {
+    constexpr bool NORM = PRE == ROWS_NORM;
     pdl_trigger();   // the GEMM behind this kernel may be scheduled already; it waits for this grid before reading
     pdl_wait();      // the activations may come from the kernel before
     __shared__ float red[kRowThreads / 32];
@@ -165,6 +207,22 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
         for (int j = 0; j < J; ++j) {
             const uint32_t i = t + (uint32_t)kRowThreads * j;
             v[j] = i < P ? *reinterpret_cast<const float4*>(row + 4u * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if constexpr (PRE == ROWS_SWIGLU) {
+            float4 up[J];
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const uint32_t i = t + (uint32_t)kRowThreads * j;
+                if (i < P) up[j] = *reinterpret_cast<const float4*>(na.w + (size_t)m * K + 4u * i);
+            }
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const uint32_t i = t + (uint32_t)kRowThreads * j;
+                if (i >= P) continue;
+                v[j] = make_float4(swiglu_f32(v[j].x, up[j].x), swiglu_f32(v[j].y, up[j].y), swiglu_f32(v[j].z, up[j].z),
+                                   swiglu_f32(v[j].w, up[j].w));
+                *reinterpret_cast<float4*>(na.y + (size_t)m * K + 4u * i) = v[j];
+            }
         }
         if constexpr (NORM) {
             double ss = 0.0;
@@ -196,8 +254,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
         amax = block_max<kRowThreads / 32>(amax, red);
         float s, inv;
         row_factor(amax, s, inv);
-        if (t == 0 && ae) ae[m] = inv;
-        uint32_t* adw = reinterpret_cast<uint32_t*>(ad);
+        if (t < dst.n && dst.d[t].ae) dst.d[t].ae[m] = inv;
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const uint32_t i = t + (uint32_t)kRowThreads * j, u = i >> 3;
@@ -206,16 +263,16 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
             float d;
             quant_unit_q8_0(v[j], mode, q, d, sum);
             if (live) {
-                reinterpret_cast<uint32_t*>(aq + (size_t)m * K)[i] = pack_q4(q);
-                if (sub == 0) adw[(size_t)m * U + u] = scale_word_q8_0(d, sum);
-                if (ah) {
-                    const float dh = __fmul_rn(h2f(f2h(d)), s);   // the fp16-rounded scale the dot product uses, times 2^-e
-                    const __half2 h01 = __floats2half2_rn((float)q[0] * dh, (float)q[1] * dh);
-                    const __half2 h23 = __floats2half2_rn((float)q[2] * dh, (float)q[3] * dh);
-                    uint2 o;
-                    o.x = *reinterpret_cast<const uint32_t*>(&h01);
-                    o.y = *reinterpret_cast<const uint32_t*>(&h23);
-                    *reinterpret_cast<uint2*>(ah + (size_t)m * K + 4u * i) = o;
+                const uint32_t word = scale_word_q8_0(d, sum);
+                const float dh = __fmul_rn(h2f(f2h(d)), s);   // the fp16-rounded scale the dot product uses, times 2^-e
+                const __half2 h01 = __floats2half2_rn((float)q[0] * dh, (float)q[1] * dh);
+                const __half2 h23 = __floats2half2_rn((float)q[2] * dh, (float)q[3] * dh);
+                const uint2 o = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+                for (uint32_t k = 0; k < dst.n; ++k) {
+                    const QuantDst& to = dst.d[k];
+                    reinterpret_cast<uint32_t*>(to.aq + (size_t)m * K)[i] = pack_q4(q);
+                    if (sub == 0) reinterpret_cast<uint32_t*>(to.ad)[(size_t)m * U + u] = word;
+                    if (to.ah) *reinterpret_cast<uint2*>(to.ah + (size_t)m * K + 4u * i) = o;
                 }
             }
         }
@@ -233,6 +290,20 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
             }
             x[j][0] = x0.x; x[j][1] = x0.y; x[j][2] = x0.z; x[j][3] = x0.w;
             x[j][4] = x1.x; x[j][5] = x1.y; x[j][6] = x1.z; x[j][7] = x1.w;
+        }
+        if constexpr (PRE == ROWS_SWIGLU) {
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const uint32_t b = (t >> 5) + (uint32_t)(kRowThreads / 32) * j;
+                if (b >= B) continue;
+                const size_t at = (size_t)m * K + 256u * b + 8u * lane;
+                const float4 u0 = *reinterpret_cast<const float4*>(na.w + at), u1 = *reinterpret_cast<const float4*>(na.w + at + 4);
+                const float up[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[j][i] = swiglu_f32(x[j][i], up[i]);
+                *reinterpret_cast<float4*>(na.y + at) = make_float4(x[j][0], x[j][1], x[j][2], x[j][3]);
+                *reinterpret_cast<float4*>(na.y + at + 4) = make_float4(x[j][4], x[j][5], x[j][6], x[j][7]);
+            }
         }
         if constexpr (NORM) {
             double ss = 0.0;
@@ -274,7 +345,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
         amax = block_max<kRowThreads / 32>(amax, red);
         float s, inv;
         row_factor(amax, s, inv);
-        if (t == 0 && ae) ae[m] = inv;
+        if (t < dst.n && dst.d[t].ae) dst.d[t].ae[m] = inv;
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const uint32_t b = (t >> 5) + (uint32_t)(kRowThreads / 32) * j;
@@ -290,24 +361,26 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
                 w0 |= (uint32_t)(q[i] & 0xFF) << (8 * i);
                 w1 |= (uint32_t)(q[i + 4] & 0xFF) << (8 * i);
             }
-            *reinterpret_cast<uint2*>(aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
-            if (ah) {
-                const float ds = __fmul_rn(d, s);
-                uint32_t o[4];
+            const float ds = __fmul_rn(d, s);
+            uint32_t o[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const __half2 hh = __floats2half2_rn((float)q[2 * i] * ds, (float)q[2 * i + 1] * ds);
-                    o[i] = *reinterpret_cast<const uint32_t*>(&hh);
-                }
-                *reinterpret_cast<uint4*>(ah + (size_t)m * K + 256u * b + 8u * lane) = make_uint4(o[0], o[1], o[2], o[3]);
+            for (int i = 0; i < 4; ++i) {
+                const __half2 hh = __floats2half2_rn((float)q[2 * i] * ds, (float)q[2 * i + 1] * ds);
+                o[i] = *reinterpret_cast<const uint32_t*>(&hh);
             }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);  // lanes 2j, 2j+1 -> 16-element group j
-            uint8_t* blk = ad + ((size_t)m * B + b) * kABBytes;
-            if ((lane & 1u) == 0u) reinterpret_cast<int16_t*>(blk)[lane >> 1] = (int16_t)sum;
-            if (lane == 0) {
-                *reinterpret_cast<float*>(blk + 32) = d;
-                *reinterpret_cast<uint32_t*>(blk + 36) = 0u;
-                *reinterpret_cast<uint2*>(blk + 40) = make_uint2(0u, 0u);
+            for (uint32_t k = 0; k < dst.n; ++k) {
+                const QuantDst& to = dst.d[k];
+                *reinterpret_cast<uint2*>(to.aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
+                if (to.ah)
+                    *reinterpret_cast<uint4*>(to.ah + (size_t)m * K + 256u * b + 8u * lane) = make_uint4(o[0], o[1], o[2], o[3]);
+                uint8_t* blk = to.ad + ((size_t)m * B + b) * kABBytes;
+                if ((lane & 1u) == 0u) reinterpret_cast<int16_t*>(blk)[lane >> 1] = (int16_t)sum;
+                if (lane == 0) {
+                    *reinterpret_cast<float*>(blk + 32) = d;
+                    *reinterpret_cast<uint32_t*>(blk + 36) = 0u;
+                    *reinterpret_cast<uint2*>(blk + 40) = make_uint2(0u, 0u);
+                }
             }
         }
     }
@@ -530,113 +603,116 @@ __global__ void __launch_bounds__(256) bitnet_rows_kernel(const BitnetRows g, ui
 // ---------------------------------------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------------------------------------
-// ameva_quant_a8: bindings 0 src f32, 1 AQ, 2 AD; push {M, K, src_stride (floats), round_mode}
-AcResult launch_quant_a8(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], K = a.push[1], stride = a.push[2], round_mode = a.push[3];
-    if (M == 0 || K == 0 || (K & 31u) || stride < K || (stride & 3u) || round_mode > 1u) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t U = K >> 5;
-    if (a.range[0] < ((uint64_t)(M - 1) * stride + K) * 4u || a.range[1] < (uint64_t)M * K ||
-        a.range[2] < (uint64_t)M * U * 4u)
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if ((uintptr_t)a.ptr[0] & 15u) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    const uint64_t threads = (uint64_t)M * U * 8u;
-    const uint64_t blocks = (threads + 255u) / 256u;
-    if (blocks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
-    launch_pdl(quant_q8_0_kernel, dim3((unsigned)blocks), dim3(256), 0, a.stream, (const float*)a.ptr[0],
-               (int8_t*)a.ptr[1], (uint32_t*)a.ptr[2], M, K, stride, round_mode);
-    return check_launch();
-}
-
-// ameva_quant_a8b: bindings 0 src f32, 1 AQ, 2 AB; push {M, K, src_stride (floats), mode}
-AcResult launch_quant_a8b(const LaunchArgs& a) {
+// What the quantize entries share: rows of K floats src_stride apart -> AQ, AD / AB (, AH, AE).
+//   ameva_quant_a8 / ameva_quant_a8b: bindings 0 src f32, 1 AQ, 2 AD (per-32 scale words) or AB (per-256 records);
+//     push {M, K, src_stride (floats), round_mode / mode}
+//   ameva_quant_a8_f16 / ameva_quant_a8b_f16 (in front of ameva_mmtc_*, more than 8 token rows): also 3 AH fp16 [M][K] =
+//     fp16(q * d * s_m), 4 AE f32 [M] = 1 / s_m (s_m the power of two that brings row m's largest magnitude into [1, 2));
+//     K <= 32768
+//   ameva_rms_norm_quant_a8 / ameva_rms_norm_quant_a8b: RMS norm (+ MUL by a weight row) and the activation quantize of the
+//     MUL_MAT that consumes it, one kernel (the reference fuses RMS_NORM + MUL, ggml-ameva.cpp:4347-4357, and norm +
+//     quantize for BitNet, src/shaders/bitnet_norm_q8.comp; here for the per-32 / per-256 schemes): bindings 0 x f32
+//     [M][src_stride], 1 w f32 [K] (any buffer when has_weight = 0), 2 y f32 [M][K] (the normalised rows: what RMS_NORM
+//     (+ MUL) writes), 3 AQ, 4 AD or AB, 5 AH, 6 AE (any buffers when write_h = 0); push {M, K (<= 32768), src_stride,
+//     round_mode / mode, eps (float bits), has_weight, write_h}; AQ / AD / AB are the bytes ameva_quant_a8 / a8b make of y
+AcResult check_quant(const LaunchArgs& a, QuantForm form, uint32_t scheme) {
     const uint32_t M = a.push[0], K = a.push[1], stride = a.push[2], mode = a.push[3];
-    if (M == 0 || K == 0 || (K & 255u) || stride < K || (stride & 3u) || mode > 1u) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t B = K >> 8;
-    if (a.range[0] < ((uint64_t)(M - 1) * stride + K) * 4u || a.range[1] < (uint64_t)M * K ||
-        a.range[2] < (uint64_t)M * B * kABBytes)
+    const bool norm = form == QUANT_NORM, has_w = norm && a.push[5], write_h = form == QUANT_F16 || (norm && a.push[6]);
+    if (M == 0 || K == 0 || (K & (scheme ? 255u : 31u)) || stride < K || (stride & 3u) || mode > 1u ||
+        (norm && (a.push[5] > 1u || a.push[6] > 1u)))
+        return AC_ERR_KERNEL_ARG_INVALID;
+    if (norm) {
+        float eps;
+        memcpy(&eps, &a.push[4], 4);
+        if (!(eps >= 0.0f)) return AC_ERR_KERNEL_ARG_INVALID;
+    }
+    const uint32_t d = norm ? 3u : 1u;   // the binding of AQ
+    const uint64_t scale_bytes = scheme ? (uint64_t)M * (K >> 8) * kABBytes : (uint64_t)M * (K >> 5) * 4u;
+    if (a.range[0] < ((uint64_t)(M - 1) * stride + K) * 4u || (has_w && a.range[1] < (uint64_t)K * 4u) ||
+        (norm && a.range[2] < (uint64_t)M * K * 4u) || a.range[d] < (uint64_t)M * K || a.range[d + 1] < scale_bytes ||
+        (write_h && (a.range[d + 2] < (uint64_t)M * K * 2u || a.range[d + 3] < (uint64_t)M * 4u)))
         return AC_ERR_INVALID_BUFFER_SIZE;
-    if ((uintptr_t)a.ptr[0] & 15u) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    const uint64_t blocks = ((uint64_t)M * B * 32u + 255u) / 256u;
-    if (blocks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
-    launch_pdl(quant_q8_K_kernel, dim3((unsigned)blocks), dim3(256), 0, a.stream, (const float*)a.ptr[0],
-               (int8_t*)a.ptr[1], (uint8_t*)a.ptr[2], M, K, stride, mode);
-    return check_launch();
+    if (((uintptr_t)a.ptr[0] & 15u) || (norm && (((uintptr_t)a.ptr[1] | (uintptr_t)a.ptr[2]) & 15u)) ||
+        (write_h && ((uintptr_t)a.ptr[d + 2] & 15u)))
+        return AC_ERR_BUFFER_ALIGNMENT_INVALID;
+    return AC_SUCCESS;
 }
 
-// ameva_quant_a8_f16 / ameva_quant_a8b_f16: the quantizers in front of ameva_mmtc_* (more than 8 token rows).
-//   bindings 0 src f32, 1 AQ, 2 AD (per-32 scale words) or AB (per-256 records), 3 AH fp16 [M][K] = fp16(q * d * s_m),
-//            4 AE f32 [M] = 1 / s_m (s_m the power of two that brings row m's largest magnitude into [1, 2))
-//   push {M, K, src_stride (floats), round_mode / mode};  K <= 32768
-template <int SCHEME, int J, bool NORM>
-static void launch_rows_j(const LaunchArgs& a, const float* src, int8_t* aq, uint8_t* ad, __half* ah, float* ae, uint32_t M,
-                          uint32_t K, uint32_t stride, uint32_t mode, const NormArgs& na) {
-    launch_pdl(quant_rows_f16_kernel<SCHEME, J, NORM>, dim3(M), dim3(kRowThreads), 0, a.stream, src, aq, ad, ah, ae, K, stride,
-               mode, na);
+static QuantDst quant_dst(const LaunchArgs& a, QuantForm form) {
+    const uint32_t d = form == QUANT_NORM ? 3u : 1u;
+    const bool h = form == QUANT_F16 || (form == QUANT_NORM && a.push[6]);
+    return {(int8_t*)a.ptr[d], (uint8_t*)a.ptr[d + 1], h ? (__half*)a.ptr[d + 2] : nullptr, h ? (float*)a.ptr[d + 3] : nullptr};
 }
 
 // pieces per thread: a row of K floats over 512 threads, 4 (per-32) or 8 (per-256) floats to a piece
-template <int SCHEME, bool NORM>
-static AcResult launch_rows(const LaunchArgs& a, const float* src, int8_t* aq, uint8_t* ad, __half* ah, float* ae, uint32_t M,
-                            uint32_t K, uint32_t stride, uint32_t mode, const NormArgs& na) {
+template <int SCHEME, int PRE>
+static AcResult launch_rows(cudaStream_t stream, const float* src, const QuantDsts& dst, uint32_t M, uint32_t K, uint32_t stride,
+                            uint32_t mode, const NormArgs& na) {
     const uint32_t per_thread = (K + (SCHEME ? 4095u : 2047u)) / (SCHEME ? 4096u : 2048u);
-    if (per_thread <= 1) launch_rows_j<SCHEME, 1, NORM>(a, src, aq, ad, ah, ae, M, K, stride, mode, na);
-    else if (per_thread <= 2) launch_rows_j<SCHEME, 2, NORM>(a, src, aq, ad, ah, ae, M, K, stride, mode, na);
-    else if (per_thread <= 4) launch_rows_j<SCHEME, 4, NORM>(a, src, aq, ad, ah, ae, M, K, stride, mode, na);
-    else if (per_thread <= 8) launch_rows_j<SCHEME, 8, NORM>(a, src, aq, ad, ah, ae, M, K, stride, mode, na);
-    else if (per_thread <= 16 && SCHEME == 0)
-        launch_rows_j<SCHEME, (SCHEME == 0 ? 16 : 8), NORM>(a, src, aq, ad, ah, ae, M, K, stride, mode, na);
+    auto go = [&](auto kernel) { launch_pdl(kernel, dim3(M), dim3(kRowThreads), 0, stream, src, dst, K, stride, mode, na); };
+    if (per_thread <= 1) go(quant_rows_f16_kernel<SCHEME, 1, PRE>);
+    else if (per_thread <= 2) go(quant_rows_f16_kernel<SCHEME, 2, PRE>);
+    else if (per_thread <= 4) go(quant_rows_f16_kernel<SCHEME, 4, PRE>);
+    else if (per_thread <= 8) go(quant_rows_f16_kernel<SCHEME, 8, PRE>);
+    else if (per_thread <= 16 && SCHEME == 0) go(quant_rows_f16_kernel<SCHEME, (SCHEME == 0 ? 16 : 8), PRE>);
     else return AC_ERR_INVALID_SHAPE;   // K above 32768: beyond the rows this kernel keeps in registers
     return check_launch();
 }
 
 template <int SCHEME>
-static AcResult launch_quant_rows(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], K = a.push[1], stride = a.push[2], mode = a.push[3];
-    const uint32_t kmask = SCHEME ? 255u : 31u;
-    if (M == 0 || K == 0 || (K & kmask) || stride < K || (stride & 3u) || mode > 1u) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t scale_bytes = SCHEME ? (uint64_t)M * (K >> 8) * kABBytes : (uint64_t)M * (K >> 5) * 4u;
-    if (a.range[0] < ((uint64_t)(M - 1) * stride + K) * 4u || a.range[1] < (uint64_t)M * K || a.range[2] < scale_bytes ||
-        a.range[3] < (uint64_t)M * K * 2u || a.range[4] < (uint64_t)M * 4u)
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if (((uintptr_t)a.ptr[0] & 15u) || ((uintptr_t)a.ptr[3] & 15u)) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    const NormArgs na = {nullptr, nullptr, 0.0f};
-    return launch_rows<SCHEME, false>(a, (const float*)a.ptr[0], (int8_t*)a.ptr[1], (uint8_t*)a.ptr[2], (__half*)a.ptr[3],
-                                      (float*)a.ptr[4], M, K, stride, mode, na);
+static AcResult launch_quant_scheme(QuantForm form, const LaunchArgs& first, const QuantDsts& dst, const LaunchArgs* swiglu) {
+    const uint32_t M = first.push[0], K = first.push[1], stride = first.push[2], mode = first.push[3];
+    if (form == QUANT_NORM) {
+        float eps;
+        memcpy(&eps, &first.push[4], 4);
+        const NormArgs na = {first.push[5] ? (const float*)first.ptr[1] : nullptr, (float*)first.ptr[2], eps};
+        return launch_rows<SCHEME, ROWS_NORM>(first.stream, (const float*)first.ptr[0], dst, M, K, stride, mode, na);
+    }
+    const float* src = (const float*)(swiglu ? swiglu->ptr[0] : first.ptr[0]);
+    if (form == QUANT_F16) {
+        if (swiglu) {
+            const NormArgs na = {(const float*)swiglu->ptr[1], (float*)swiglu->ptr[2], 0.0f};
+            return launch_rows<SCHEME, ROWS_SWIGLU>(first.stream, src, dst, M, K, K, mode, na);
+        }
+        const NormArgs na = {nullptr, nullptr, 0.0f};
+        return launch_rows<SCHEME, ROWS_PLAIN>(first.stream, src, dst, M, K, stride, mode, na);
+    }
+    const uint64_t blocks = ((uint64_t)M * (SCHEME ? (K >> 8) * 32ull : (K >> 5) * 8ull) + 255u) / 256u;
+    if (blocks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
+    const GateArgs ga = {swiglu ? (const float*)swiglu->ptr[1] : nullptr, swiglu ? (float*)swiglu->ptr[2] : nullptr};
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, first.stream, src, dst, M, K, swiglu ? K : stride, mode, ga);
+    };
+    if (SCHEME == 0) {
+        if (swiglu) go(quant_q8_0_kernel<true>);
+        else go(quant_q8_0_kernel<false>);
+    } else {
+        if (swiglu) go(quant_q8_K_kernel<true>);
+        else go(quant_q8_K_kernel<false>);
+    }
+    return check_launch();
 }
-AcResult launch_quant_a8_f16(const LaunchArgs& a) { return launch_quant_rows<0>(a); }
-AcResult launch_quant_a8b_f16(const LaunchArgs& a) { return launch_quant_rows<1>(a); }
 
-// ameva_rms_norm_quant_a8 / ameva_rms_norm_quant_a8b: RMS norm (+ MUL by a weight row) and the activation quantize of
-// the MUL_MAT that consumes it, one kernel (the reference fuses RMS_NORM + MUL, ggml-ameva.cpp:4347-4357, and norm +
-// quantize for BitNet, src/shaders/bitnet_norm_q8.comp; here for the per-32 / per-256 schemes).
-//   bindings 0 x f32 [M][src_stride], 1 w f32 [K] (any buffer when has_weight = 0), 2 y f32 [M][K] (the normalised rows:
-//            what RMS_NORM (+ MUL) writes), 3 AQ, 4 AD or AB, 5 AH, 6 AE (any buffers when write_h = 0)
-//   push {M, K (<= 32768), src_stride, round_mode / mode, eps (float bits), has_weight, write_h}
-// AQ / AD / AB are the bytes ameva_quant_a8 / a8b produce from y.
-template <int SCHEME>
-static AcResult launch_rms_norm_quant(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], K = a.push[1], stride = a.push[2], mode = a.push[3], has_w = a.push[5], write_h = a.push[6];
-    const uint32_t kmask = SCHEME ? 255u : 31u;
-    if (M == 0 || K == 0 || (K & kmask) || stride < K || (stride & 3u) || mode > 1u || has_w > 1u || write_h > 1u)
-        return AC_ERR_KERNEL_ARG_INVALID;
-    float eps;
-    memcpy(&eps, &a.push[4], 4);
-    if (!(eps >= 0.0f)) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t scale_bytes = SCHEME ? (uint64_t)M * (K >> 8) * kABBytes : (uint64_t)M * (K >> 5) * 4u;
-    if (a.range[0] < ((uint64_t)(M - 1) * stride + K) * 4u || (has_w && a.range[1] < (uint64_t)K * 4u) ||
-        a.range[2] < (uint64_t)M * K * 4u || a.range[3] < (uint64_t)M * K || a.range[4] < scale_bytes ||
-        (write_h && (a.range[5] < (uint64_t)M * K * 2u || a.range[6] < (uint64_t)M * 4u)))
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if (((uintptr_t)a.ptr[0] & 15u) || ((uintptr_t)a.ptr[1] & 15u) || ((uintptr_t)a.ptr[2] & 15u) ||
-        (write_h && ((uintptr_t)a.ptr[5] & 15u)))
-        return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    const NormArgs na = {has_w ? (const float*)a.ptr[1] : nullptr, (float*)a.ptr[2], eps};
-    return launch_rows<SCHEME, true>(a, (const float*)a.ptr[0], (int8_t*)a.ptr[3], (uint8_t*)a.ptr[4],
-                                     write_h ? (__half*)a.ptr[5] : nullptr, write_h ? (float*)a.ptr[6] : nullptr, M, K, stride,
-                                     mode, na);
+AcResult launch_quant_group(QuantForm form, uint32_t scheme, const LaunchArgs& first, const LaunchArgs* const* more, uint32_t n_more,
+                            const LaunchArgs* swiglu) {
+    QuantDsts dst;
+    memset(&dst, 0, sizeof(dst));
+    dst.d[dst.n++] = quant_dst(first, form);
+    for (uint32_t i = 0; i < n_more; ++i)
+        dst.d[dst.n++] = quant_dst(*more[i], form == QUANT_NORM && first.push[6] ? QUANT_F16 : form == QUANT_NORM ? QUANT_PLAIN : form);
+    return scheme ? launch_quant_scheme<1>(form, first, dst, swiglu) : launch_quant_scheme<0>(form, first, dst, swiglu);
 }
-AcResult launch_rms_norm_quant_a8(const LaunchArgs& a) { return launch_rms_norm_quant<0>(a); }
-AcResult launch_rms_norm_quant_a8b(const LaunchArgs& a) { return launch_rms_norm_quant<1>(a); }
+
+static AcResult launch_quant(const LaunchArgs& a, QuantForm form, uint32_t scheme) {
+    const AcResult rc = check_quant(a, form, scheme);
+    return rc != AC_SUCCESS ? rc : launch_quant_group(form, scheme, a, nullptr, 0u, nullptr);
+}
+AcResult launch_quant_a8(const LaunchArgs& a) { return launch_quant(a, QUANT_PLAIN, 0u); }
+AcResult launch_quant_a8b(const LaunchArgs& a) { return launch_quant(a, QUANT_PLAIN, 1u); }
+AcResult launch_quant_a8_f16(const LaunchArgs& a) { return launch_quant(a, QUANT_F16, 0u); }
+AcResult launch_quant_a8b_f16(const LaunchArgs& a) { return launch_quant(a, QUANT_F16, 1u); }
+AcResult launch_rms_norm_quant_a8(const LaunchArgs& a) { return launch_quant(a, QUANT_NORM, 0u); }
+AcResult launch_rms_norm_quant_a8b(const LaunchArgs& a) { return launch_quant(a, QUANT_NORM, 1u); }
 
 // bitnet_norm_q8: bindings 0 a, 1 b, 2 w, 3 y, 4 q, 5 act, 6 qeo; push {dim, eps_bits, mode, do_norm}; grid.x = rows
 // (argument contract of src/shaders/bitnet_norm_q8.comp:20-44, extended from one row to grid.x rows).

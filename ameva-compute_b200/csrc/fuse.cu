@@ -11,7 +11,13 @@ AcResult launch_add_f32(const LaunchArgs&);
 AcResult launch_bitnet_gemm_i2_s(const LaunchArgs&);
 AcResult launch_bitnet_gemv_i2_s(const LaunchArgs&);
 AcResult launch_bitnet_norm_q8(const LaunchArgs&);
+AcResult launch_quant_a8(const LaunchArgs&);
+AcResult launch_quant_a8_f16(const LaunchArgs&);
+AcResult launch_quant_a8b(const LaunchArgs&);
+AcResult launch_quant_a8b_f16(const LaunchArgs&);
 AcResult launch_rms_norm_f32(const LaunchArgs&);
+AcResult launch_rms_norm_quant_a8(const LaunchArgs&);
+AcResult launch_rms_norm_quant_a8b(const LaunchArgs&);
 AcResult launch_rope(const LaunchArgs&);
 AcResult launch_set_rows(const LaunchArgs&);
 AcResult launch_swiglu_f32(const LaunchArgs&);
@@ -37,9 +43,13 @@ bool disjoint(const LaunchArgs& a, const LaunchArgs& b) {
     return true;
 }
 
-// kernels that read and write their bindings and nothing else
+// kernels that read and write their bindings and nothing else (products without the exchange between ranks, quantizes)
+bool starts(const FuseOp& op, const char* prefix) { return strncmp(op.entry->name, prefix, strlen(prefix)) == 0; }
 bool confined(const FuseOp& op) {
-    return is(op, launch_bitnet_gemv_i2_s) || is(op, launch_bitnet_gemm_i2_s) || is(op, launch_bitnet_norm_q8);
+    if (!op.entry->launch) return false;
+    if (starts(op, "ameva_mmvs_")) return op.args.push[4] == 0u;   // (peers)
+    return is(op, launch_bitnet_gemv_i2_s) || is(op, launch_bitnet_gemm_i2_s) || is(op, launch_bitnet_norm_q8) ||
+           starts(op, "ameva_quant_a8") || ((starts(op, "ameva_mmv") || starts(op, "ameva_mmtc_")) && !strstr(op.entry->name, "_mp"));
 }
 
 // May ops[j] run together with ops[i], i < j? Members of the group being formed (marked in `member`) are checked by the caller.
@@ -231,11 +241,100 @@ AcResult fuse_row_ops(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
     return launch_row_ops(rope, store, n_rope, set, n_set);
 }
 
+// ---- per-32 / per-256 quantizes of the same rows ----
+bool quant_of(const FuseOp& op, QuantForm* form, uint32_t* scheme) {
+    if (is(op, launch_quant_a8) || is(op, launch_quant_a8b)) *form = QUANT_PLAIN;
+    else if (is(op, launch_quant_a8_f16) || is(op, launch_quant_a8b_f16)) *form = QUANT_F16;
+    else if (is(op, launch_rms_norm_quant_a8) || is(op, launch_rms_norm_quant_a8b)) *form = QUANT_NORM;
+    else return false;
+    *scheme = is(op, launch_quant_a8b) || is(op, launch_quant_a8b_f16) || is(op, launch_rms_norm_quant_a8b);
+    return true;
+}
+
+AcResult fuse_quant(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
+    const LaunchArgs& head = ops[i].args;
+    const bool swiglu = is(ops[i], launch_swiglu_f32);
+    QuantForm form = QUANT_PLAIN, want = QUANT_PLAIN;   // of the first quantize, and of those that may join it
+    uint32_t scheme = 0, K = 0, M = 0;
+    const LaunchArgs* first = nullptr;
+    const void* rows_ptr = nullptr;
+    uint64_t rows_bytes = 0;
+    if (swiglu) {
+        rows_ptr = head.ptr[2];
+        rows_bytes = 4ull * head.push[0];
+        if (!rows_bytes || head.range[0] < rows_bytes || head.range[1] < rows_bytes || head.range[2] < rows_bytes) return AC_SUCCESS;
+        for (uint32_t b = 0; b < 2u; ++b)
+            if (((uintptr_t)head.ptr[b] & 15u) || (head.ptr[b] != rows_ptr && overlap(head.ptr[b], rows_bytes, rows_ptr, rows_bytes)))
+                return AC_SUCCESS;
+    } else {
+        quant_of(ops[i], &form, &scheme);
+        if (check_quant(head, form, scheme) != AC_SUCCESS) return AC_SUCCESS;
+        first = &head;
+        M = head.push[0];
+        K = head.push[1];
+        rows_ptr = form == QUANT_NORM ? head.ptr[2] : head.ptr[0];
+        rows_bytes = form == QUANT_NORM ? 4ull * M * K : head.range[0];
+        want = form == QUANT_NORM ? (head.push[6] ? QUANT_F16 : QUANT_PLAIN) : form;
+    }
+    const LaunchArgs* more[kFuseMax];
+    uint32_t n_more = 0;
+    uint64_t mask = 0;
+    for (uint32_t j = i + 1; j < n && j <= i + kLookahead && n_more + 1u < kFuseMax; ++j) {
+        if (ops[j].done) continue;
+        const LaunchArgs& q = ops[j].args;
+        QuantForm f;
+        uint32_t sch;
+        if (quant_of(ops[j], &f, &sch) && f != QUANT_NORM && q.ptr[0] == rows_ptr && check_quant(q, f, sch) == AC_SUCCESS) {
+            bool ok;
+            if (!first) {   // the quantize that says how the gated elements form rows
+                ok = (uint64_t)q.push[0] * q.push[1] * 4u == rows_bytes && q.push[2] == q.push[1] && q.push[1] <= 32768u;
+            } else {
+                const uint32_t stride = form == QUANT_NORM || swiglu ? K : first->push[2];
+                ok = f == want && sch == scheme && q.push[0] == M && q.push[1] == K && q.push[2] == stride && q.push[3] == first->push[3];
+            }
+            ok = ok && can_hoist(ops, i, j, mask);
+            // what it writes meets nothing that the head or another member reads or writes
+            const uint32_t outs = f == QUANT_F16 ? 5u : 3u;
+            for (uint32_t b = 1; b < outs && ok; ++b) {
+                ok = !touches(head, q.ptr[b], q.range[b]) && !(first && first != &head && touches(*first, q.ptr[b], q.range[b]));
+                for (uint32_t m = 0; m < n_more && ok; ++m) ok = !touches(*more[m], q.ptr[b], q.range[b]);
+                for (uint32_t h = 1; h < b && ok; ++h) ok = !overlap(q.ptr[h], q.range[h], q.ptr[b], q.range[b]);
+            }
+            if (ok) {
+                if (first) {
+                    more[n_more++] = &q;
+                } else {
+                    first = &q;
+                    form = want = f;
+                    scheme = sch;
+                    M = q.push[0];
+                    K = q.push[1];
+                }
+                mask |= 1ull << (j - i);
+                continue;
+            }
+        }
+        if (!confined(ops[j])) break;
+    }
+    if (!mask) return AC_SUCCESS;
+    *taken = true;
+    ops[i].done = true;
+    for (uint32_t k = 0; k <= kLookahead; ++k)
+        if (mask >> k & 1u) ops[i + k].done = true;
+    return launch_quant_group(form, scheme, *first, more, n_more, swiglu ? &head : nullptr);
+}
+
 }  // namespace
 
 AcResult launch_fused(FuseOp* ops, uint32_t n, uint32_t i) {
     bool taken = false;
     AcResult rc = AC_SUCCESS;
+    QuantForm form;
+    uint32_t scheme;
+    if (is(ops[i], launch_swiglu_f32) || quant_of(ops[i], &form, &scheme)) {
+        rc = fuse_quant(ops, n, i, &taken);
+        if (taken) return rc;
+    }
     if (is(ops[i], launch_bitnet_norm_q8) || is(ops[i], launch_rms_norm_f32) || is(ops[i], launch_swiglu_f32))
         rc = fuse_bitnet_rows(ops, n, i, &taken);
     else if (is(ops[i], launch_bitnet_gemv_i2_s))

@@ -31,6 +31,13 @@ AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const L
 AcResult check_bitnet_gemv_i2_s(const LaunchArgs& a);
 AcResult launch_bitnet_gemv_i2_s_group(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped);
 
+// the quantize kernels (act_quant.cu), per-32 (scheme 0) and per-256 (scheme 1): several that read the same rows (the first
+// may be the fused RMS norm + quantize that writes them) in one pass, or the SWIGLU that forms the rows with them
+enum QuantForm { QUANT_PLAIN, QUANT_F16, QUANT_NORM };
+AcResult check_quant(const LaunchArgs& a, QuantForm form, uint32_t scheme);
+AcResult launch_quant_group(QuantForm form, uint32_t scheme, const LaunchArgs& first, const LaunchArgs* const* more, uint32_t n_more,
+                            const LaunchArgs* swiglu);
+
 // ROPE / SET_ROWS of the same new positions (layer_ops.cu): up to two of each beside one another, and per ROPE a SET_ROWS of
 // its result (store[i], nullptr: none)
 bool row_op_serves(const LaunchArgs& a, bool rope);
