@@ -822,19 +822,18 @@ AcResult launch_gemv_f16(const LaunchArgs& a) {
 // (ggml's layout). Scores, probabilities and accumulation in fp32, as the reference's shader keeps them.
 //
 // The keys are split over the grid (flash decoding): CTA (z, kv head, query position) walks keys [z * split, (z + 1) *
-// split) for all G = n_head / n_head_kv heads of its group, so every K and V byte is read once per query position. A
-// warp takes 32 keys at a time: lane l reads the whole K row of key l (16-byte loads; a row is one or more whole
-// sectors) and forms the G scores against the queries in shared memory; an online softmax keeps the running maximum
-// and sum per head; for the P V product the lanes own DV / 32 output columns each and the 32 probabilities are passed
-// round by shuffles, so the V rows are read coalesced. The warps of a CTA, then the splits (ameva_fa_combine's job in
-// the reference: a second kernel here too) are merged with the usual maximum / sum rescaling. The work is bound by
-// reading the KV cache from HBM: n_kv * n_head_kv * (D + DV) * 2 bytes per query position.
+// split) for all G = n_head / n_head_kv heads of its group, so every K and V byte is read once per query position. Each
+// warp takes 16 keys at a time through tiles of its own in shared memory, an online softmax per head; the warps of a CTA are
+// merged in shared memory with the usual maximum / sum rescaling, the CTAs of a row by the one that finishes last
+// (ameva_fa_combine's job in the reference). The work is bound by reading the KV cache from HBM: n_kv * n_head_kv * (D + DV)
+// * 2 bytes per query position.
 // n_q > 1, D <= 128: up to sixteen rows of positions x heads 16 / G positions per CTA (flash_tile_kernel below), more the
 // tensor-core kernel of flash_tc.cu; D = 256: one position per CTA.
 // Not taken: ALiBi (max_bias != 0), f32 or quantized K / V, G > 8, D != DV: refused with AC_ERR_FEATURE_NOT_SUPPORTED
 // (the host keeps such nodes on its other path).
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int kFaWarps = 4;
+constexpr uint32_t kFaMaxSplits = 1024;
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src)
@@ -852,21 +851,27 @@ constexpr size_t flash_tile_smem_bytes() {   // the kernel for prompts merges si
     constexpr size_t tiles = 2 * sizeof(__half) * kFaWarps * 32 * D, merge = sizeof(float) * kFaWarps * 16 * (D + 2);
     return tiles > merge ? tiles : merge;
 }
+// The one-position kernel: a CTA per SM (D = 128: 12 warps with four tiles of 16 keys each, two of K and two of V: 192 KB on
+// their way to an SM that consumes 45 KB per microsecond at the full HBM rate).
+constexpr uint32_t kFdKeys = 16, kFdStages = 2;
+template <int D>
+constexpr int fd_warps() { return D == 64 ? 16 : D == 128 ? 12 : 6; }
 template <int D>
 constexpr size_t flash_smem_bytes() {
-    constexpr size_t tiles = 2 * sizeof(__half) * kFaWarps * 32 * D, merge = sizeof(float) * kFaWarps * kFaHeads * (D + 2);
+    constexpr size_t tiles = 2 * kFdStages * sizeof(__half) * fd_warps<D>() * kFdKeys * D,
+                     merge = sizeof(float) * fd_warps<D>() * kFaHeads * (D + 2);
     return tiles > merge ? tiles : merge;
 }
 
-// 32 rows of D halves from global memory (row r at base + r * stride) into a warp's shared-memory tile, two (D = 128)
+// ROWS rows of D halves from global memory (row r at base + r * stride) into a warp's shared-memory tile, two (D = 128)
 // whole rows per warp instruction; rows from `rows` on are zero-filled. The 16-byte pieces of row r are stored at
 // piece ^ (r mod pieces per row): the eight row addresses of an ldmatrix then fall into eight different bank groups.
-template <int D>
+template <int D, uint32_t ROWS = 32u>
 __device__ __forceinline__ void stage_rows(__half (*tile)[D], const __half* base, uint64_t stride, uint32_t rows,
                                            uint32_t lane) {
     constexpr uint32_t P = D / 8;
 #pragma unroll 8
-    for (uint32_t i = lane; i < 32u * P; i += 32u) {
+    for (uint32_t i = lane; i < ROWS * P; i += 32u) {
         const uint32_t row = i / P, piece = i - row * P;
         __half* dst = &tile[row][8u * (piece ^ (row & (P - 1u)))];
         if (row < rows) cp_async16(dst, base + row * stride + 8u * piece);
@@ -902,34 +907,52 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 // the whole kernel), B = the staged K rows (ldmatrix). The score accumulators already have the A-fragment layout of
 // the second product, P V, whose B fragments are the staged V rows through ldmatrix.trans. Q and the probabilities
 // are rounded to f16 (ggml's CPU kernel rounds Q to f16 as well and accumulates V in f16; here accumulation is fp32).
+//
+// Blocks of 16 keys: a short context then still gives every warp of the chip a block (32 heads x 2048 keys: 4096 blocks on 1776
+// warps; blocks of 32 left a third of the warps with half the work of the others). K(b) .. V(b + 1) are on their way when block
+// b starts; a tile is requested again as soon as it has been read.
+// counters: one zero word per (KV head, position), left zero; nullptr: the partial results are merged by the kernel below.
 template <int D>
-__global__ void __launch_bounds__(kFaWarps * 32) flash_decode_kernel(const float* __restrict__ q, const __half* __restrict__ k,
-                                                                     const __half* __restrict__ v,
-                                                                     const __half* __restrict__ mask, float* __restrict__ o,
-                                                                     float* __restrict__ part, const FlashArgs pc,
-                                                                     uint32_t n_splits) {
+__global__ void __launch_bounds__(fd_warps<D>() * 32, 1) flash_decode_kernel(const float* __restrict__ q, const __half* __restrict__ k,
+                                                                          const __half* __restrict__ v,
+                                                                          const __half* __restrict__ mask, float* __restrict__ o,
+                                                                          float* part, const FlashArgs pc,
+                                                                          uint32_t n_splits, uint32_t* counters) {
     constexpr int KS = D / 16;                // k-steps of the score product
     constexpr int NT = D / 8;                 // n-tiles of the output
     constexpr uint32_t P = D / 8;             // 16-byte pieces per K or V row
+    constexpr uint32_t W = fd_warps<D>(), TILE = kFdKeys * D;   // (halves)
     extern __shared__ __align__(16) uint8_t fa_smem[];
     float (*s_acc)[kFaHeads][D + 2] = reinterpret_cast<float (*)[kFaHeads][D + 2]>(fa_smem);   // per warp: D sums, max, sum
-    uint8_t* tiles = fa_smem;                                                                  // (used before s_acc)
+    __shared__ uint32_t s_last;
     pdl_trigger();
     pdl_wait();
     const uint32_t z = blockIdx.x, hkv = blockIdx.y, iq1 = blockIdx.z;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    __half (*s_k)[D] = reinterpret_cast<__half (*)[D]>(tiles + sizeof(__half) * 32 * D * (2 * warp));       // this warp's
-    __half (*s_v)[D] = reinterpret_cast<__half (*)[D]>(tiles + sizeof(__half) * 32 * D * (2 * warp + 1));   // K and V tile
+    typedef __half (*Tile)[D];
+    __half* mine = reinterpret_cast<__half*>(fa_smem) + warp * (2u * kFdStages * TILE);   // K tiles, then V tiles of this warp
+    auto tile_k = [&](uint32_t st) { return reinterpret_cast<Tile>(mine + st * TILE); };
+    auto tile_v = [&](uint32_t st) { return reinterpret_cast<Tile>(mine + (kFdStages + st) * TILE); };
     const uint32_t G = pc.n_head / pc.n_head_kv, h0 = hkv * G;
     const float ninf = __uint_as_float(0xFF800000u);
     const uint32_t key_begin = z * pc.split_keys, key_end = min(pc.n_kv, key_begin + pc.split_keys);
     const __half* kbase = k + pc.k_off + (uint64_t)hkv * pc.k_s2;
     const __half* vbase = v + pc.v_off + (uint64_t)hkv * pc.v_s2;
-    uint32_t k0 = key_begin + warp * 32u;
-    // the first block's K and V are requested before anything else
-    if (k0 < key_end) {
-        stage_rows<D>(s_k, kbase + (uint64_t)k0 * pc.k_s1, pc.k_s1, min(32u, key_end - k0), lane);
-        stage_rows<D>(s_v, vbase + (uint64_t)k0 * pc.v_s1, pc.v_s1, min(32u, key_end - k0), lane);
+    constexpr uint32_t STEP = W * kFdKeys;
+    // (an empty group keeps the count of the waits where there is nothing to request)
+    auto request_k = [&](uint32_t st, uint32_t key) {
+        if (key < key_end) stage_rows<D, kFdKeys>(tile_k(st), kbase + (uint64_t)key * pc.k_s1, pc.k_s1, min(kFdKeys, key_end - key), lane);
+        else cp_async_commit();
+    };
+    auto request_v = [&](uint32_t st, uint32_t key) {
+        if (key < key_end) stage_rows<D, kFdKeys>(tile_v(st), vbase + (uint64_t)key * pc.v_s1, pc.v_s1, min(kFdKeys, key_end - key), lane);
+        else cp_async_commit();
+    };
+    uint32_t k0 = key_begin + warp * kFdKeys;
+#pragma unroll
+    for (uint32_t st = 0; st < kFdStages; ++st) {   // requested before anything else
+        request_k(st, k0 + st * STEP);
+        request_v(st, k0 + st * STEP);
     }
     // this thread's share of the A fragments of Q: head g = lane / 4, columns 16 ks + 2 (lane % 4) + {0, 1} and + 8
     const uint32_t g = lane >> 2, t4 = lane & 3u;
@@ -952,64 +975,70 @@ __global__ void __launch_bounds__(kFaWarps * 32) flash_decode_kernel(const float
         for (int j = 0; j < 4; ++j) oc[nt][j] = 0.0f;
     float m_run = ninf, l_run = 0.0f;
     const __half* mrow = mask + pc.m_off + (uint64_t)iq1 * pc.m_s1 + (uint64_t)((h0 + (head ? g : 0u)) % (pc.has_mask ? pc.m_ne2 : 1u)) * pc.m_s2;
+    // this thread's four keys of a block: 8 nt + 2 t4 + {0, 1}; their mask values are fetched one block ahead
+    auto load_mask = [&](uint32_t key0, float (&to)[2][2]) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const uint32_t key = key0 + 8u * nt + 2u * t4 + j;
+                to[nt][j] = !head || key >= key_end ? ninf : pc.has_mask ? __half2float(mrow[key]) : 0.0f;
+            }
+    };
+    float mk[2][2];
+    load_mask(k0, mk);
     // ldmatrix row addresses of this lane: matrix lane / 8, row lane % 8
     const uint32_t lm_row = (lane & 7u) + ((lane >> 4) << 3), lm_hi = (lane >> 3) & 1u;   // K: key within 16, upper d half
     const uint32_t lv_row = (lane & 7u) + (((lane >> 3) & 1u) << 3), lv_nt = lane >> 4;    // V: key within 16, second n-tile
-    // Per block of 32 keys: K(b) and V(b) are in flight when the block starts; K(b + 1) is requested as soon as the
-    // scores are formed, V(b + 1) after the P V product: a tile is always on its way while the warp computes.
-    for (; k0 < key_end; k0 += kFaWarps * 32u) {
-        const uint32_t next = k0 + kFaWarps * 32u;
-        const bool more = next < key_end;
-        cp_async_wait_group<1>();   // K(b) has landed (V(b) may still be on its way)
+    uint32_t st = 0;
+    for (; k0 < key_end; k0 += STEP, st = st + 1u == kFdStages ? 0u : st + 1u) {
+        const uint32_t ahead = k0 + kFdStages * STEP;
+        cp_async_wait_group<2 * kFdStages - 1>();   // K(b) has landed
         __syncwarp();
-        float sc[4][4];
+        Tile s_k = tile_k(st), s_v = tile_v(st);
+        float sc[2][4];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int j = 0; j < 4; ++j) sc[nt][j] = 0.0f;
 #pragma unroll
-        for (int np = 0; np < 2; ++np) {          // pairs of n-tiles: keys 16 np .. 16 np + 15
-            const uint32_t key = 16u * np + lm_row;
-#pragma unroll
-            for (int ks = 0; ks < KS; ++ks) {
-                uint32_t b[4];
-                ldmatrix_x4(b, &s_k[key][8u * ((2u * ks + lm_hi) ^ (key & (P - 1u)))]);
-                mma_16816_top(sc[2 * np], qa[ks][0], qa[ks][1], b[0], b[1]);
-                mma_16816_top(sc[2 * np + 1], qa[ks][0], qa[ks][1], b[2], b[3]);
-            }
+        for (int ks = 0; ks < KS; ++ks) {
+            uint32_t b[4];
+            ldmatrix_x4(b, &s_k[lm_row][8u * ((2u * ks + lm_hi) ^ (lm_row & (P - 1u)))]);
+            mma_16816_top(sc[0], qa[ks][0], qa[ks][1], b[0], b[1]);
+            mma_16816_top(sc[1], qa[ks][0], qa[ks][1], b[2], b[3]);
         }
         __syncwarp();   // every lane has read the K tile: it may be refilled
-        if (more) stage_rows<D>(s_k, kbase + (uint64_t)next * pc.k_s1, pc.k_s1, min(32u, key_end - next), lane);
-        else cp_async_commit();   // (an empty group keeps the count of the waits below)
-        // this thread's eight scores: head g, keys k0 + 8 nt + 2 t4 + {0, 1}
-        float x[4][2], bm = ninf;
+        request_k(st, ahead);
+        // this thread's four scores of head g
+        float x[2][2], bm = ninf;
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const uint32_t key = k0 + 8u * nt + 2u * t4 + j;
                 float xv = ninf;
-                if (head && key < key_end) {
+                if (mk[nt][j] != ninf) {
                     xv = sc[nt][j] * scale;
                     if (softcap != 0.0f) xv = softcap * tanhf(xv / softcap);
-                    if (pc.has_mask) xv += __half2float(mrow[key]);
+                    xv += mk[nt][j];
                 }
                 x[nt][j] = xv;
                 bm = fmaxf(bm, xv);
             }
+        load_mask(k0 + STEP, mk);
         bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
         bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
         const float m_new = fmaxf(m_run, bm);
         // nothing but masked keys so far: the maximum stays -inf and nothing is added
         const float factor = m_new == ninf ? 1.0f : expf(m_run - m_new);
         float ps = 0.0f;
-        uint32_t pa[2][2];
+        uint32_t pa[2];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
+        for (int nt = 0; nt < 2; ++nt) {
             const float p0 = x[nt][0] == ninf ? 0.0f : expf(x[nt][0] - m_new);
             const float p1 = x[nt][1] == ninf ? 0.0f : expf(x[nt][1] - m_new);
             ps += p0 + p1;
-            pa[nt >> 1][nt & 1] = pack_h2(p0, p1);
+            pa[nt] = pack_h2(p0, p1);
         }
         ps += __shfl_xor_sync(0xffffffffu, ps, 1);
         ps += __shfl_xor_sync(0xffffffffu, ps, 2);
@@ -1020,23 +1049,18 @@ __global__ void __launch_bounds__(kFaWarps * 32) flash_decode_kernel(const float
             oc[nt][0] *= factor;
             oc[nt][1] *= factor;
         }
-        cp_async_wait_group<1>();   // V(b) has landed (K(b + 1) may still be on its way)
+        cp_async_wait_group<2 * kFdStages - 1>();   // V(b) has landed
         __syncwarp();
         // rows past the last key are zeros and their probabilities are 0
 #pragma unroll
         for (int np = 0; np < NT / 2; ++np) {     // pairs of output n-tiles: columns 16 np .. 16 np + 15
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {      // keys 16 kk .. 16 kk + 15
-                const uint32_t key = 16u * kk + lv_row;
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, &s_v[key][8u * ((2u * np + lv_nt) ^ (key & (P - 1u)))]);
-                mma_16816_top(oc[2 * np], pa[kk][0], pa[kk][1], b[0], b[1]);
-                mma_16816_top(oc[2 * np + 1], pa[kk][0], pa[kk][1], b[2], b[3]);
-            }
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, &s_v[lv_row][8u * ((2u * np + lv_nt) ^ (lv_row & (P - 1u)))]);
+            mma_16816_top(oc[2 * np], pa[0], pa[1], b[0], b[1]);
+            mma_16816_top(oc[2 * np + 1], pa[0], pa[1], b[2], b[3]);
         }
         __syncwarp();   // every lane has read the V tile
-        if (more) stage_rows<D>(s_v, vbase + (uint64_t)next * pc.v_s1, pc.v_s1, min(32u, key_end - next), lane);
-        else cp_async_commit();
+        request_v(st, ahead);
     }
     cp_async_wait_group<0>();
     __syncthreads();   // every warp is done with its tiles: the memory is reused for the merge
@@ -1053,14 +1077,14 @@ __global__ void __launch_bounds__(kFaWarps * 32) flash_decode_kernel(const float
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < G * D; i += kFaWarps * 32) {
+    for (uint32_t i = threadIdx.x; i < G * D; i += W * 32u) {
         const uint32_t gg = i / D, d = i - gg * D;
         float mx = ninf;
 #pragma unroll
-        for (int w = 0; w < kFaWarps; ++w) mx = fmaxf(mx, s_acc[w][gg][D]);
+        for (uint32_t w = 0; w < W; ++w) mx = fmaxf(mx, s_acc[w][gg][D]);
         float num = 0.0f, den = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kFaWarps; ++w) {
+        for (uint32_t w = 0; w < W; ++w) {
             const float mw = s_acc[w][gg][D];
             const float f = mw == ninf ? 0.0f : expf(mw - mx);
             num = fmaf(s_acc[w][gg][d], f, num);
@@ -1077,6 +1101,69 @@ __global__ void __launch_bounds__(kFaWarps * 32) flash_decode_kernel(const float
                 pr[1] = den;
             }
         }
+    }
+    if (n_splits == 1u || counters == nullptr) return;
+    // the CTA that finishes last merges the splits of its rows
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t* c = counters + iq1 * pc.n_head_kv + hkv;
+        const bool last = atomicAdd(c, 1u) == n_splits - 1u;
+        if (last) *c = 0u;   // as the next launch expects it
+        s_last = last;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    float* s_f = reinterpret_cast<float*>(fa_smem);              // [G][n_splits]: exp(m_z - max)
+    float* s_den = s_f + kFaHeads * kFaMaxSplits;                // [G]
+    float4* s_part = reinterpret_cast<float4*>(s_den + kFaHeads);   // [groups of splits][G * D / 4]
+    const float* first = part + pc.part_off + ((uint64_t)iq1 * pc.n_head + h0) * (D + 4);
+    const uint64_t zs = (uint64_t)pc.n_q * pc.n_head * (D + 4);   // floats between two splits of a row
+    for (uint32_t gg = warp; gg < G; gg += W) {
+        float mx = ninf, den = 0.0f;
+        for (uint32_t zz = lane; zz < n_splits; zz += 32u) mx = fmaxf(mx, __ldcg(first + zz * zs + gg * (D + 4)));
+        mx = warp_max(mx);
+        for (uint32_t zz = lane; zz < n_splits; zz += 32u) {
+            const float2 ml = __ldcg(reinterpret_cast<const float2*>(first + zz * zs + gg * (D + 4)));
+            const float f = ml.x == ninf ? 0.0f : expf(ml.x - mx);
+            s_f[gg * n_splits + zz] = f;
+            den = fmaf(ml.y, f, den);
+        }
+        den = warp_sum(den);
+        if (lane == 0) s_den[gg] = den;
+    }
+    __syncthreads();
+    const uint32_t cols = G * (D / 4), groups = W * 32u / cols ? W * 32u / cols : 1u;
+    for (uint32_t i = threadIdx.x; i < groups * cols; i += W * 32u) {
+        const uint32_t grp = i / cols, col = i - grp * cols, gg = col / (D / 4), c4 = col - gg * (D / 4);
+        const float* src = first + gg * (D + 4) + 4 + 4u * c4;
+        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (uint32_t zz = grp; zz < n_splits; zz += groups) {
+            const float4 xx = __ldcg(reinterpret_cast<const float4*>(src + zz * zs));
+            const float f = s_f[gg * n_splits + zz];
+            num.x = fmaf(xx.x, f, num.x);
+            num.y = fmaf(xx.y, f, num.y);
+            num.z = fmaf(xx.z, f, num.z);
+            num.w = fmaf(xx.w, f, num.w);
+        }
+        s_part[i] = num;
+    }
+    __syncthreads();
+    for (uint32_t col = threadIdx.x; col < cols; col += W * 32u) {
+        const uint32_t gg = col / (D / 4), c4 = col - gg * (D / 4);
+        float4 num = s_part[col];
+        for (uint32_t grp = 1; grp < groups; ++grp) {
+            const float4 xx = s_part[grp * cols + col];
+            num.x += xx.x;
+            num.y += xx.y;
+            num.z += xx.z;
+            num.w += xx.w;
+        }
+        const float den = s_den[gg];
+        *reinterpret_cast<float4*>(o + pc.o_off + ((uint64_t)iq1 * pc.n_head + h0 + gg) * D + 4u * c4) =
+            make_float4(num.x / den, num.y / den, num.z / den, num.w / den);
     }
 }
 
@@ -1285,7 +1372,6 @@ __global__ void __launch_bounds__(kFaWarps * 32) flash_tile_kernel(const float* 
 
 // merges the partial results of the key splits: one CTA per output row; the splits' maxima and sums are read in parallel,
 // then every thread sums its columns over the splits (independent, coalesced loads)
-constexpr uint32_t kFaMaxSplits = 1024;
 __global__ void __launch_bounds__(128) flash_combine_kernel(const float* __restrict__ part, float* __restrict__ o,
                                                             uint32_t D, uint32_t rows, uint32_t n_splits, uint32_t part_off,
                                                             uint32_t o_off) {
@@ -1359,12 +1445,13 @@ static bool launch_flash_tile_d(const LaunchArgs& a, const FlashArgs& pc, uint32
 }
 
 template <int D>
-static bool launch_flash_d(const LaunchArgs& a, const FlashArgs& pc, uint32_t n_splits) {
+static bool launch_flash_d(const LaunchArgs& a, const FlashArgs& pc, uint32_t n_splits, uint32_t* counters) {
     constexpr size_t smem = flash_smem_bytes<D>();
+    static_assert(smem >= sizeof(float) * (kFaHeads * kFaMaxSplits + kFaHeads + 4 * fd_warps<D>() * 32 + kFaHeads * D), "the merge of the splits");
     if (!ensure_dynamic_smem<flash_decode_kernel<D>>((int)smem)) return false;
-    const dim3 grid(n_splits, pc.n_head_kv, pc.n_q), block(kFaWarps * 32);
+    const dim3 grid(n_splits, pc.n_head_kv, pc.n_q), block(fd_warps<D>() * 32);
     launch_pdl(flash_decode_kernel<D>, grid, block, smem, a.stream, (const float*)a.ptr[0], (const __half*)a.ptr[1],
-               (const __half*)a.ptr[2], (const __half*)a.ptr[3], (float*)a.ptr[4], (float*)a.ptr[5], pc, n_splits);
+               (const __half*)a.ptr[2], (const __half*)a.ptr[3], (float*)a.ptr[4], (float*)a.ptr[5], pc, n_splits, counters);
     return true;
 }
 
@@ -1405,15 +1492,18 @@ AcResult launch_flash_attn(const LaunchArgs& a) {
     const uint32_t q_tiles = (tile || prompt) ? (pc.n_q + QT - 1u) / QT : pc.n_q;
     const uint64_t ctas = (uint64_t)pc.n_head_kv * q_tiles;
     if (q_tiles > 65535u) return AC_ERR_INVALID_WORK_ITEM_DIMS;
-    const size_t smem = tile ? (pc.D == 64u ? flash_tile_smem_bytes<64>() : flash_tile_smem_bytes<128>())
-                             : pc.D == 64u ? flash_smem_bytes<64>() : pc.D == 128u ? flash_smem_bytes<128>() : flash_smem_bytes<256>();
-    uint32_t per_sm = prompt ? kFlashTcPerSm : (uint32_t)((227u * 1024u) / (smem + 1024u));
+    const size_t smem = pc.D == 64u ? flash_tile_smem_bytes<64>() : flash_tile_smem_bytes<128>();
+    uint32_t per_sm = prompt ? kFlashTcPerSm : tile ? (uint32_t)((227u * 1024u) / (smem + 1024u)) : 1u;
     if (per_sm > 4u) per_sm = 4u;
-    if (per_sm < 1u) per_sm = 1u;
+    // one position: a block of keys for every warp of a CTA before the keys are split further, and no split at all (no merge)
+    // up to two blocks (14 heads on 2 KV heads of 64, 333 keys: a layer takes 35.1 us in one part, 36.9 us in two; 20 heads on
+    // 5 of 128, 777 keys: 48.1 us in five parts, 51.3 us in three)
+    const uint32_t fd_keys = kFdKeys * (pc.D == 64u ? fd_warps<64>() : pc.D == 128u ? fd_warps<128>() : fd_warps<256>());
     uint32_t n_splits = (uint32_t)(((uint64_t)per_sm * sms) / ctas);
-    const uint32_t block = prompt ? kFlashTcKeys : 32u, min_keys = prompt ? 4u * kFlashTcKeys : 128u;
+    const uint32_t block = prompt ? kFlashTcKeys : tile ? 32u : kFdKeys, min_keys = prompt ? 4u * kFlashTcKeys : tile ? 128u : fd_keys;
     const uint32_t max_by_keys = (pc.n_kv + min_keys - 1u) / min_keys;
     if (n_splits > max_by_keys) n_splits = max_by_keys;
+    if (!prompt && !tile && pc.n_kv <= 2u * fd_keys) n_splits = 1u;
     const uint64_t per_split = rows * (pc.D + 4u) * 4u;
     const uint64_t room = a.range[5] > (uint64_t)pc.part_off * 4u ? a.range[5] - (uint64_t)pc.part_off * 4u : 0u;
     if ((uint64_t)n_splits * per_split > room) n_splits = (uint32_t)(room / per_split);
@@ -1423,14 +1513,15 @@ AcResult launch_flash_attn(const LaunchArgs& a) {
     if (n_splits > kFaMaxSplits) n_splits = kFaMaxSplits;
     pc.split_keys = ((pc.n_kv + n_splits - 1u) / n_splits + block - 1u) & ~(block - 1u);
     n_splits = (pc.n_kv + pc.split_keys - 1u) / pc.split_keys;
+    uint32_t* counters = !prompt && !tile && a.workspace && (uint64_t)pc.n_head_kv * pc.n_q * 4u <= a.workspace_bytes ? a.workspace : nullptr;
     const bool fits = prompt ? launch_flash_tc(a, maps, pc, n_splits, q_tiles)
                       : tile ? (pc.D == 64u ? launch_flash_tile_d<64>(a, pc, n_splits, q_tiles)
                                           : launch_flash_tile_d<128>(a, pc, n_splits, q_tiles))
-                      : pc.D == 64u ? launch_flash_d<64>(a, pc, n_splits)
-                      : pc.D == 128u ? launch_flash_d<128>(a, pc, n_splits) : launch_flash_d<256>(a, pc, n_splits);
+                      : pc.D == 64u ? launch_flash_d<64>(a, pc, n_splits, counters)
+                      : pc.D == 128u ? launch_flash_d<128>(a, pc, n_splits, counters) : launch_flash_d<256>(a, pc, n_splits, counters);
     if (!fits) return AC_ERR_INVALID_WORK_GROUP_SIZE;
     AcResult rc = check_launch();
-    if (rc != AC_SUCCESS || n_splits == 1u) return rc;
+    if (rc != AC_SUCCESS || n_splits == 1u || counters) return rc;
     launch_pdl(flash_combine_kernel, dim3((unsigned)rows), dim3(128), 0, a.stream, (const float*)a.ptr[5], (float*)a.ptr[4],
                pc.D, (uint32_t)rows, n_splits, pc.part_off, pc.o_off);
     return check_launch();

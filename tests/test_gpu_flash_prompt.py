@@ -152,3 +152,17 @@ def test_more_keys_than_one_window(ctx):
     mask[:, 1000:20000] = -np.inf
     got = run(ctx, q, k, v, mask, D ** -0.5, scratch=64)
     assert np.max(np.abs(got - attention(q, k, v, mask, D ** -0.5))) < TOL
+
+
+@pytest.mark.parametrize("D,H,Hkv", [(64, 14, 2), (64, 8, 1), (128, 32, 32), (128, 20, 5), (128, 8, 1), (256, 8, 1), (256, 6, 2)])
+@pytest.mark.parametrize("n_kv", [1, 15, 16, 17, 95, 96, 97, 193, 256, 257, 400, 5000])
+def test_one_position_over_few_and_many_blocks(ctx, D, H, Hkv, n_kv):
+    """Blocks of 16 keys per warp, one to many per CTA, one to many CTAs per KV head (merged by the last one)."""
+    q, k, v = inputs(1, n_kv, H, Hkv, D, 11)
+    rng = np.random.default_rng(n_kv)
+    mask = np.where(rng.random((1, (n_kv + 63) // 64 * 64)) < 0.3, -np.inf, rng.standard_normal((1, (n_kv + 63) // 64 * 64))).astype(np.float16)
+    mask[0, n_kv // 2] = 0
+    want = attention(q, k, v, mask[:, :n_kv], D ** -0.5)
+    for _ in range(2):      # (the second launch finds the arrival counters as the first left them)
+        assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5) - want)) < TOL
+    assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5, scratch=64) - want)) < TOL
