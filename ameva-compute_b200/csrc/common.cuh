@@ -40,6 +40,8 @@ struct LaunchArgs {
     uint32_t* workspace;      // device words owned by the context, zero between launches (cross-CTA sequence flags)
     uint64_t workspace_bytes;
     SideQueues* side;         // the context's side queues (copy launchers)
+    const float* add_e;       // set by fuse.cu for the products that carry it: the ADD behind the product, out = product + e
+    float* add_out;
 };
 
 typedef AcResult (*LaunchFn)(const LaunchArgs&);

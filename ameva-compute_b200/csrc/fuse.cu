@@ -11,6 +11,12 @@ AcResult launch_add_f32(const LaunchArgs&);
 AcResult launch_bitnet_gemm_i2_s(const LaunchArgs&);
 AcResult launch_bitnet_gemv_i2_s(const LaunchArgs&);
 AcResult launch_bitnet_norm_q8(const LaunchArgs&);
+AcResult launch_mmvq_q4_1(const LaunchArgs&);
+AcResult launch_mmvqb_iq4_xs(const LaunchArgs&);
+AcResult launch_mmvqb_q2_K(const LaunchArgs&);
+AcResult launch_mmvqb_q3_K(const LaunchArgs&);
+AcResult launch_mmvqb_q5_K(const LaunchArgs&);
+AcResult launch_mmvqb_q6_K(const LaunchArgs&);
 AcResult launch_quant_a8(const LaunchArgs&);
 AcResult launch_quant_a8_f16(const LaunchArgs&);
 AcResult launch_quant_a8b(const LaunchArgs&);
@@ -190,6 +196,28 @@ AcResult fuse_bitnet_gemv(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
     return launch_bitnet_gemv_i2_s_group(member, count, add, swapped);
 }
 
+// ---- a product of a byte-decoded type with the ADD that consumes it ----
+AcResult fuse_product_add(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
+    LaunchArgs p = ops[i].args;
+    const uint32_t M = p.push[0], N = p.push[1];
+    uint32_t j = i + 1;
+    while (j < n && ops[j].done) ++j;
+    if (j >= n || !is(ops[j], launch_add_f32) || !M || !N || p.push[3] != N) return AC_SUCCESS;
+    const LaunchArgs& s = ops[j].args;
+    const uint64_t bytes = (uint64_t)M * N * 4u;
+    const bool swapped = s.ptr[1] == p.ptr[4];
+    void* e = s.ptr[swapped ? 0 : 1];
+    if (!(swapped || s.ptr[0] == p.ptr[4]) || s.push[0] != M || s.push[1] != N || s.push[2] != M || s.range[0] < bytes ||
+        s.range[1] < bytes || s.range[2] < bytes || overlap(e, bytes, p.ptr[4], bytes) ||
+        (e != s.ptr[2] && overlap(e, bytes, s.ptr[2], bytes)) || touches(p, s.ptr[2], s.range[2]))
+        return AC_SUCCESS;
+    p.add_e = (const float*)e;
+    p.add_out = (float*)s.ptr[2];
+    *taken = true;
+    ops[i].done = ops[j].done = true;
+    return ops[i].entry->launch(p);
+}
+
 // ---- ROPEs and cache writes in a row ----
 // Ranges an operation reads (ROPE: source, positions, factors; SET_ROWS: source, indices); both write binding 3. A status
 // binding (SET_ROWS 2) takes atomics only, so several operations may share it.
@@ -339,6 +367,9 @@ AcResult launch_fused(FuseOp* ops, uint32_t n, uint32_t i) {
         rc = fuse_bitnet_rows(ops, n, i, &taken);
     else if (is(ops[i], launch_bitnet_gemv_i2_s))
         rc = fuse_bitnet_gemv(ops, n, i, &taken);
+    else if (is(ops[i], launch_mmvqb_q6_K) || is(ops[i], launch_mmvqb_q5_K) || is(ops[i], launch_mmvqb_iq4_xs) ||
+             is(ops[i], launch_mmvq_q4_1) || is(ops[i], launch_mmvqb_q3_K) || is(ops[i], launch_mmvqb_q2_K))
+        rc = fuse_product_add(ops, n, i, &taken);
     else if (is(ops[i], launch_rope) || is(ops[i], launch_set_rows))
         rc = fuse_row_ops(ops, n, i, &taken);
     if (taken) return rc;

@@ -12,8 +12,12 @@
 // decoded in the shader (adapters/llama/ggml-ameva/shaders/ameva_qdecode.glsl, decode of type 14;
 // ggml-ameva-repack.cpp:21-28 lists q6_K in the repacked family).
 //
-// One warp per weight row, eight rows per CTA; a lane walks the row's 16-weight groups with stride 32, so a warp's loads
-// are 512 contiguous bytes; weights bypass L1, which keeps the activation rows. Bound by HBM: 274 bytes per 256 weights.
+// All seven byte-decoded types run in one kernel body (byte_gemv_kernel) with a policy for the scale records: one warp per
+// weight row, eight rows per CTA; a lane walks the row's 16-weight groups with stride 32, so a warp's loads are 512
+// contiguous bytes; weights bypass L1, which keeps the activation rows. Bound by HBM (Q6_K: 274 bytes per 256 weights) and, at
+// token-generation sizes, by the latency of a launch's dependent loads: the scale records and the first two steps of weights
+// (eight 16-byte loads per lane) are requested before the wait for the preceding kernel, and the step after next is in
+// flight during the arithmetic. 4096 x 11008 in a decoder layer: 16.6 us as one launch of its own before, the layer 85.0 -> 81.1 us.
 #include "common.cuh"
 
 namespace amv {
@@ -39,87 +43,6 @@ __device__ __forceinline__ void group_dot(const uint4 w, uint32_t gi, const uint
         const float da = *reinterpret_cast<const float*>(AB + ((size_t)m * B + blk) * kABBytes + 32);
         acc[m] = fmaf(dw * da, (float)(sc * t), acc[m]);
     }
-}
-
-template <int M>
-__global__ void __launch_bounds__(kQ6Warps * 32) gemv_q6k_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S,
-                                                                 const int8_t* __restrict__ AQ, const uint8_t* __restrict__ AB,
-                                                                 float* __restrict__ dst, uint32_t N, uint32_t K,
-                                                                 uint32_t dst_stride) {
-    pdl_wait();
-    pdl_trigger();
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t row = blockIdx.x * kQ6Warps + warp;
-    if (row >= N) return;
-    const uint32_t B = K >> 8, groups = K >> 4;
-    const uint4* q = reinterpret_cast<const uint4*>(Q + (size_t)row * K);
-    // the row's scale records go to shared memory first (2-byte loads, all in flight at once): inside the loop only the
-    // weight loads wait for HBM
-    extern __shared__ __align__(16) uint8_t q6_smem[];
-    uint8_t* s = q6_smem + (size_t)warp * B * kQ6ScaleBytes;
-    {
-        const uint16_t* src = reinterpret_cast<const uint16_t*>(S + (size_t)row * B * kQ6ScaleBytes);
-        uint16_t* dstp = reinterpret_cast<uint16_t*>(s);
-        for (uint32_t i = lane; i < B * (kQ6ScaleBytes / 2u); i += 32u) dstp[i] = __ldg(src + i);
-        __syncwarp();
-    }
-    float acc[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-    // eight, then four groups per lane and step: that many independent 16-byte loads in flight before the first is used
-    uint32_t gi = lane;
-    for (; gi + 32u * 7u < groups; gi += 32u * 8u) {
-        uint4 w[8];
-#pragma unroll
-        for (uint32_t u = 0; u < 8u; ++u) w[u] = ld_stream_u4(q + gi + 32u * u);
-#pragma unroll
-        for (uint32_t u = 0; u < 8u; ++u) group_dot<M>(w[u], gi + 32u * u, s, AQ, AB, K, B, acc);
-    }
-    for (; gi + 32u * 3u < groups; gi += 32u * 4u) {
-        uint4 w[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) w[u] = ld_stream_u4(q + gi + 32u * u);
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) group_dot<M>(w[u], gi + 32u * u, s, AQ, AB, K, B, acc);
-    }
-    for (; gi < groups; gi += 32u) group_dot<M>(ld_stream_u4(q + gi), gi, s, AQ, AB, K, B, acc);
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-        const float v = warp_sum(acc[m]);
-        if (lane == 0) dst[(size_t)m * dst_stride + row] = v;
-    }
-}
-
-template <int M>
-static void launch_q6k_m(const LaunchArgs& a, uint32_t N, uint32_t K, uint32_t dst_stride) {
-    const size_t smem = (size_t)kQ6Warps * (K >> 8) * kQ6ScaleBytes;   // (K <= 65536: at most 36 KB)
-    launch_pdl(gemv_q6k_kernel<M>, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream,
-               (const uint8_t*)a.ptr[0], (const uint8_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint8_t*)a.ptr[3],
-               (float*)a.ptr[4], N, K, dst_stride);
-}
-
-// ameva_mmvqb_q6_K: bindings 0 Q (int8 [N][K], the decoded weights), 1 S (18-byte records [N][K/256]), 2 AQ int8 [M][K],
-// 3 AB (48-byte Q8_K records [M][K/256]), 4 dst f32 [M][dst_stride]; push {M (1..8), N, K (% 256, <= 65536), dst_stride}
-AcResult launch_mmvqb_q6_K(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], N = a.push[1], K = a.push[2], dst_stride = a.push[3];
-    if (M == 0 || M > 8) return AC_ERR_INVALID_SHAPE;
-    if (N == 0 || K == 0 || (K & 255u) || K > 65536u || dst_stride < N) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t B = K >> 8;
-    if (a.range[0] < (uint64_t)N * K || a.range[1] < (uint64_t)N * B * kQ6ScaleBytes || a.range[2] < (uint64_t)M * K ||
-        a.range[3] < (uint64_t)M * B * kABBytes || a.range[4] < ((uint64_t)(M - 1) * dst_stride + N) * 4u)
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if (((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[2]) & 15u) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    switch (M) {
-        case 1: launch_q6k_m<1>(a, N, K, dst_stride); break;
-        case 2: launch_q6k_m<2>(a, N, K, dst_stride); break;
-        case 3: launch_q6k_m<3>(a, N, K, dst_stride); break;
-        case 4: launch_q6k_m<4>(a, N, K, dst_stride); break;
-        case 5: launch_q6k_m<5>(a, N, K, dst_stride); break;
-        case 6: launch_q6k_m<6>(a, N, K, dst_stride); break;
-        case 7: launch_q6k_m<7>(a, N, K, dst_stride); break;
-        default: launch_q6k_m<8>(a, N, K, dst_stride); break;
-    }
-    return check_launch();
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -161,76 +84,6 @@ __device__ __forceinline__ void group_dot_q5(const uint4 w, uint32_t gi, const u
     }
 }
 
-template <int M>
-__global__ void __launch_bounds__(kQ6Warps * 32) gemv_q5k_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S,
-                                                                 const int8_t* __restrict__ AQ, const uint8_t* __restrict__ AB,
-                                                                 float* __restrict__ dst, uint32_t N, uint32_t K,
-                                                                 uint32_t dst_stride) {
-    pdl_wait();
-    pdl_trigger();
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t row = blockIdx.x * kQ6Warps + warp;
-    if (row >= N) return;
-    const uint32_t B = K >> 8, groups = K >> 4;
-    const uint4* q = reinterpret_cast<const uint4*>(Q + (size_t)row * K);
-    extern __shared__ __align__(16) uint8_t q5_smem[];
-    uint8_t* s = q5_smem + (size_t)warp * B * 16u;
-    {   // the row's scale records (16 bytes per block), all loads in flight at once
-        const uint4* src = reinterpret_cast<const uint4*>(S + (size_t)row * B * 16u);
-        for (uint32_t i = lane; i < B; i += 32u) reinterpret_cast<uint4*>(s)[i] = __ldg(src + i);
-        __syncwarp();
-    }
-    float acc[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-    uint32_t gi = lane;
-    for (; gi + 32u * 3u < groups; gi += 32u * 4u) {
-        uint4 w[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) w[u] = ld_stream_u4(q + gi + 32u * u);
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) group_dot_q5<M>(w[u], gi + 32u * u, s, AQ, AB, K, B, acc);
-    }
-    for (; gi < groups; gi += 32u) group_dot_q5<M>(ld_stream_u4(q + gi), gi, s, AQ, AB, K, B, acc);
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-        const float v = warp_sum(acc[m]);
-        if (lane == 0) dst[(size_t)m * dst_stride + row] = v;
-    }
-}
-
-template <int M>
-static void launch_q5k_m(const LaunchArgs& a, uint32_t N, uint32_t K, uint32_t dst_stride) {
-    const size_t smem = (size_t)kQ6Warps * (K >> 8) * 16u;
-    launch_pdl(gemv_q5k_kernel<M>, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream,
-               (const uint8_t*)a.ptr[0], (const uint8_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint8_t*)a.ptr[3],
-               (float*)a.ptr[4], N, K, dst_stride);
-}
-
-// ameva_mmvqb_q5_K: bindings 0 Q (bytes [N][K], q5 decoded at upload), 1 S (16-byte records [N][K/256]: d, dmin, packed
-// scales), 2 AQ int8 [M][K], 3 AB (48-byte Q8_K records), 4 dst f32; push {M (1..8), N, K (% 256, <= 65536), dst_stride}
-AcResult launch_mmvqb_q5_K(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], N = a.push[1], K = a.push[2], dst_stride = a.push[3];
-    if (M == 0 || M > 8) return AC_ERR_INVALID_SHAPE;
-    if (N == 0 || K == 0 || (K & 255u) || K > 65536u || dst_stride < N) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t B = K >> 8;
-    if (a.range[0] < (uint64_t)N * K || a.range[1] < (uint64_t)N * B * 16u || a.range[2] < (uint64_t)M * K ||
-        a.range[3] < (uint64_t)M * B * kABBytes || a.range[4] < ((uint64_t)(M - 1) * dst_stride + N) * 4u)
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if (((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[1] | (uintptr_t)a.ptr[2]) & 15u) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    switch (M) {
-        case 1: launch_q5k_m<1>(a, N, K, dst_stride); break;
-        case 2: launch_q5k_m<2>(a, N, K, dst_stride); break;
-        case 3: launch_q5k_m<3>(a, N, K, dst_stride); break;
-        case 4: launch_q5k_m<4>(a, N, K, dst_stride); break;
-        case 5: launch_q5k_m<5>(a, N, K, dst_stride); break;
-        case 6: launch_q5k_m<6>(a, N, K, dst_stride); break;
-        case 7: launch_q5k_m<7>(a, N, K, dst_stride); break;
-        default: launch_q5k_m<8>(a, N, K, dst_stride); break;
-    }
-    return check_launch();
-}
-
 // ---------------------------------------------------------------------------------------------------------------------
 // IQ4_XS x Q8_K: a weight is d * (ls[e / 32] - 32) * kvalues_iq4nl[q4] (ggml-common.h block_iq4_xs: d, scales_h,
 // scales_l[4], qs[128]: 136 bytes per 256 weights; ls is 6 bits: four from scales_l, two from scales_h). The upload
@@ -258,76 +111,6 @@ __device__ __forceinline__ void group_dot_iq4xs(const uint4 w, uint32_t gi, cons
     }
 }
 
-template <int M>
-__global__ void __launch_bounds__(kQ6Warps * 32) gemv_iq4xs_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S,
-                                                                   const int8_t* __restrict__ AQ, const uint8_t* __restrict__ AB,
-                                                                   float* __restrict__ dst, uint32_t N, uint32_t K,
-                                                                   uint32_t dst_stride) {
-    pdl_wait();
-    pdl_trigger();
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t row = blockIdx.x * kQ6Warps + warp;
-    if (row >= N) return;
-    const uint32_t B = K >> 8, groups = K >> 4;
-    const uint4* q = reinterpret_cast<const uint4*>(Q + (size_t)row * K);
-    extern __shared__ __align__(16) uint8_t iq_smem[];
-    uint8_t* s = iq_smem + (size_t)warp * B * 8u;
-    {   // the row's scale records (8 bytes per block)
-        const uint2* src = reinterpret_cast<const uint2*>(S + (size_t)row * B * 8u);
-        for (uint32_t i = lane; i < B; i += 32u) reinterpret_cast<uint2*>(s)[i] = __ldg(src + i);
-        __syncwarp();
-    }
-    float acc[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-    uint32_t gi = lane;
-    for (; gi + 32u * 3u < groups; gi += 32u * 4u) {
-        uint4 w[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) w[u] = ld_stream_u4(q + gi + 32u * u);
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) group_dot_iq4xs<M>(w[u], gi + 32u * u, s, AQ, AB, K, B, acc);
-    }
-    for (; gi < groups; gi += 32u) group_dot_iq4xs<M>(ld_stream_u4(q + gi), gi, s, AQ, AB, K, B, acc);
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-        const float v = warp_sum(acc[m]);
-        if (lane == 0) dst[(size_t)m * dst_stride + row] = v;
-    }
-}
-
-template <int M>
-static void launch_iq4xs_m(const LaunchArgs& a, uint32_t N, uint32_t K, uint32_t dst_stride) {
-    const size_t smem = (size_t)kQ6Warps * (K >> 8) * 8u;
-    launch_pdl(gemv_iq4xs_kernel<M>, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream,
-               (const uint8_t*)a.ptr[0], (const uint8_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint8_t*)a.ptr[3],
-               (float*)a.ptr[4], N, K, dst_stride);
-}
-
-// ameva_mmvqb_iq4_xs: bindings 0 Q (int8 [N][K], kvalues decoded at upload), 1 S (8-byte records [N][K/256]: d, scales_h,
-// scales_l), 2 AQ int8 [M][K], 3 AB (48-byte Q8_K records), 4 dst f32; push {M (1..8), N, K (% 256, <= 65536), dst_stride}
-AcResult launch_mmvqb_iq4_xs(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], N = a.push[1], K = a.push[2], dst_stride = a.push[3];
-    if (M == 0 || M > 8) return AC_ERR_INVALID_SHAPE;
-    if (N == 0 || K == 0 || (K & 255u) || K > 65536u || dst_stride < N) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t B = K >> 8;
-    if (a.range[0] < (uint64_t)N * K || a.range[1] < (uint64_t)N * B * 8u || a.range[2] < (uint64_t)M * K ||
-        a.range[3] < (uint64_t)M * B * kABBytes || a.range[4] < ((uint64_t)(M - 1) * dst_stride + N) * 4u)
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if ((((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[2]) & 15u) || ((uintptr_t)a.ptr[1] & 7u)) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    switch (M) {
-        case 1: launch_iq4xs_m<1>(a, N, K, dst_stride); break;
-        case 2: launch_iq4xs_m<2>(a, N, K, dst_stride); break;
-        case 3: launch_iq4xs_m<3>(a, N, K, dst_stride); break;
-        case 4: launch_iq4xs_m<4>(a, N, K, dst_stride); break;
-        case 5: launch_iq4xs_m<5>(a, N, K, dst_stride); break;
-        case 6: launch_iq4xs_m<6>(a, N, K, dst_stride); break;
-        case 7: launch_iq4xs_m<7>(a, N, K, dst_stride); break;
-        default: launch_iq4xs_m<8>(a, N, K, dst_stride); break;
-    }
-    return check_launch();
-}
-
 // ---------------------------------------------------------------------------------------------------------------------
 // Q4_1 / Q5_1 x Q8_0-with-sums (ggml's Q8_1): a weight is d * q + m per 32 (q = 0..15 / 0..31), so
 //   y = sum_blocks (d_w * d_a) * sum_i q * q8 + m_w * (d_a * sum_i q8)
@@ -336,80 +119,22 @@ AcResult launch_mmvqb_iq4_xs(const LaunchArgs& a) {
 // keeps (d, m) as a 4-byte record; one kernel serves both types.
 // ---------------------------------------------------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(kQ6Warps * 32) gemv_q41_kernel(const uint8_t* __restrict__ Q, const uint32_t* __restrict__ S,
-                                                                 const int8_t* __restrict__ AQ, const uint32_t* __restrict__ AD,
-                                                                 float* __restrict__ dst, uint32_t N, uint32_t K,
-                                                                 uint32_t dst_stride) {
-    pdl_wait();
-    pdl_trigger();
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t row = blockIdx.x * kQ6Warps + warp;
-    if (row >= N) return;
-    const uint32_t U = K >> 5, groups = K >> 4;
-    const uint4* q = reinterpret_cast<const uint4*>(Q + (size_t)row * K);
-    extern __shared__ __align__(16) uint8_t q41_smem[];
-    uint32_t* s = reinterpret_cast<uint32_t*>(q41_smem) + (size_t)warp * U;
-    for (uint32_t i = lane; i < U; i += 32u) s[i] = __ldg(S + (size_t)row * U + i);
-    __syncwarp();
-    float acc[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-#pragma unroll 4
-    for (uint32_t gi = lane; gi < groups; gi += 32u) {
-        const uint4 w = ld_stream_u4(q + gi);
-        const uint32_t u = gi >> 1, rec = s[u];
-        const float dw = h2f((uint16_t)(rec & 0xFFFFu)), mw = (gi & 1u) ? 0.0f : h2f((uint16_t)(rec >> 16));
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-            const uint4 a = *reinterpret_cast<const uint4*>(AQ + (size_t)m * K + 16u * gi);
-            int t = dp4a_ss(w.x, a.x, 0);
-            t = dp4a_ss(w.y, a.y, t);
-            t = dp4a_ss(w.z, a.z, t);
-            t = dp4a_ss(w.w, a.w, t);
-            const uint32_t adw = AD[(size_t)m * U + u];
-            const float da = h2f((uint16_t)(adw & 0xFFFFu));
-            acc[m] += (dw * da) * (float)t + mw * (da * (float)(int)(int16_t)(adw >> 16));
-        }
-    }
+__device__ __forceinline__ void group_dot_q41(const uint4 w, uint32_t gi, const uint8_t* s, const int8_t* __restrict__ AQ,
+                                              const uint8_t* __restrict__ ADb, uint32_t K, uint32_t U, float (&acc)[M]) {
+    const uint32_t* AD = reinterpret_cast<const uint32_t*>(ADb);
+    const uint32_t u = gi >> 1, rec = reinterpret_cast<const uint32_t*>(s)[u];
+    const float dw = h2f((uint16_t)(rec & 0xFFFFu)), mw = (gi & 1u) ? 0.0f : h2f((uint16_t)(rec >> 16));
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        const float v = warp_sum(acc[m]);
-        if (lane == 0) dst[(size_t)m * dst_stride + row] = v;
+        const uint4 a = *reinterpret_cast<const uint4*>(AQ + (size_t)m * K + 16u * gi);
+        int t = dp4a_ss(w.x, a.x, 0);
+        t = dp4a_ss(w.y, a.y, t);
+        t = dp4a_ss(w.z, a.z, t);
+        t = dp4a_ss(w.w, a.w, t);
+        const uint32_t adw = AD[(size_t)m * U + u];
+        const float da = h2f((uint16_t)(adw & 0xFFFFu));
+        acc[m] += (dw * da) * (float)t + mw * (da * (float)(int)(int16_t)(adw >> 16));
     }
-}
-
-template <int M>
-static void launch_q41_m(const LaunchArgs& a, uint32_t N, uint32_t K, uint32_t dst_stride) {
-    const size_t smem = (size_t)kQ6Warps * (K >> 5) * 4u;
-    launch_pdl(gemv_q41_kernel<M>, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream,
-               (const uint8_t*)a.ptr[0], (const uint32_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint32_t*)a.ptr[3],
-               (float*)a.ptr[4], N, K, dst_stride);
-}
-
-// ameva_mmvq_q4_1 / ameva_mmvq_q5_1: bindings 0 Q (bytes [N][K], q decoded at upload), 1 S (u32 [N][K/32]: fp16 d | fp16 m
-// << 16), 2 AQ int8 [M][K], 3 AD (u32 [M][K/32]: fp16 d | int16 sum << 16), 4 dst f32;
-// push {M (1..8), N, K (% 32, <= 32768), dst_stride}
-AcResult launch_mmvq_q4_1(const LaunchArgs& a) {
-    const uint32_t M = a.push[0], N = a.push[1], K = a.push[2], dst_stride = a.push[3];
-    if (M == 0 || M > 8) return AC_ERR_INVALID_SHAPE;
-    if (N == 0 || K == 0 || (K & 31u) || K > 32768u || dst_stride < N) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t U = K >> 5;
-    if (a.range[0] < (uint64_t)N * K || a.range[1] < (uint64_t)N * U * 4u || a.range[2] < (uint64_t)M * K ||
-        a.range[3] < (uint64_t)M * U * 4u || a.range[4] < ((uint64_t)(M - 1) * dst_stride + N) * 4u)
-        return AC_ERR_INVALID_BUFFER_SIZE;
-    if ((((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[2]) & 15u) || (((uintptr_t)a.ptr[1] | (uintptr_t)a.ptr[3]) & 3u))
-        return AC_ERR_BUFFER_ALIGNMENT_INVALID;
-    switch (M) {
-        case 1: launch_q41_m<1>(a, N, K, dst_stride); break;
-        case 2: launch_q41_m<2>(a, N, K, dst_stride); break;
-        case 3: launch_q41_m<3>(a, N, K, dst_stride); break;
-        case 4: launch_q41_m<4>(a, N, K, dst_stride); break;
-        case 5: launch_q41_m<5>(a, N, K, dst_stride); break;
-        case 6: launch_q41_m<6>(a, N, K, dst_stride); break;
-        case 7: launch_q41_m<7>(a, N, K, dst_stride); break;
-        default: launch_q41_m<8>(a, N, K, dst_stride); break;
-    }
-    return check_launch();
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -457,83 +182,131 @@ __device__ __forceinline__ void group_dot_q23(const uint4 w, uint32_t gi, const 
     }
 }
 
-template <int M, int KIND>
-__global__ void __launch_bounds__(kQ6Warps * 32) gemv_q23k_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S,
-                                                                  const int8_t* __restrict__ AQ, const uint8_t* __restrict__ AB,
-                                                                  float* __restrict__ dst, uint32_t N, uint32_t K,
-                                                                  uint32_t dst_stride) {
-    constexpr uint32_t kRec = KIND == 3 ? 14u : 20u;
-    pdl_wait();
-    pdl_trigger();
+// ---------------------------------------------------------------------------------------------------------------------
+// The kernel. A policy names the weights per scale record (1 << kUnit), the bytes of a record and the dot product of one
+// 16-weight group. add: the ADD behind the product, when the launch carries it (M rows of N floats without gaps).
+// ---------------------------------------------------------------------------------------------------------------------
+#define AMV_BYTE_POLICY(NAME, UNIT, REC, DOT)                                                                              \
+    struct NAME {                                                                                                          \
+        static constexpr uint32_t kUnit = UNIT, kRec = REC;                                                                \
+        template <int M>                                                                                                   \
+        static __device__ __forceinline__ void dot(const uint4 w, uint32_t gi, const uint8_t* s, const int8_t* __restrict__ AQ, \
+                                                   const uint8_t* __restrict__ AD, uint32_t K, uint32_t units, float (&acc)[M]) { \
+            DOT(w, gi, s, AQ, AD, K, units, acc);                                                                          \
+        }                                                                                                                  \
+    };
+AMV_BYTE_POLICY(ByteQ6K, 8, kQ6ScaleBytes, group_dot<M>)
+AMV_BYTE_POLICY(ByteQ5K, 8, 16, group_dot_q5<M>)
+AMV_BYTE_POLICY(ByteIq4Xs, 8, 8, group_dot_iq4xs<M>)
+AMV_BYTE_POLICY(ByteQ41, 5, 4, group_dot_q41<M>)
+AMV_BYTE_POLICY(ByteQ3K, 8, 14, (group_dot_q23<M, 3>))
+AMV_BYTE_POLICY(ByteQ2K, 8, 20, (group_dot_q23<M, 2>))
+#undef AMV_BYTE_POLICY
+
+struct ByteAdd {
+    const float* e;
+    float* out;
+};
+
+// (one row: 64 registers, so that four CTAs are resident and a 4096-row product is one wave)
+template <class T, int M>
+__global__ void __launch_bounds__(kQ6Warps * 32, M == 1 ? 4 : 1)
+byte_gemv_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S, const int8_t* __restrict__ AQ,
+                 const uint8_t* __restrict__ AD, float* __restrict__ dst, uint32_t N, uint32_t K, uint32_t dst_stride,
+                 const ByteAdd add) {
+    constexpr uint32_t UN = 4, STEP = 32u * UN;   // groups per step of a warp
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t row = blockIdx.x * kQ6Warps + warp;
     if (row >= N) return;
-    const uint32_t B = K >> 8, groups = K >> 4;
+    const uint32_t units = K >> T::kUnit, groups = K >> 4;
     const uint4* q = reinterpret_cast<const uint4*>(Q + (size_t)row * K);
-    extern __shared__ __align__(16) uint8_t q23_smem[];
-    uint8_t* s = q23_smem + (size_t)warp * B * kRec;
-    {   // the row's scale records, by 2-byte loads (a record is 14 or 20 bytes)
-        const uint16_t* src = reinterpret_cast<const uint16_t*>(S + (size_t)row * B * kRec);
-        uint16_t* dstp = reinterpret_cast<uint16_t*>(s);
-        for (uint32_t i = lane; i < B * (kRec / 2u); i += 32u) dstp[i] = __ldg(src + i);
-        __syncwarp();
+    extern __shared__ __align__(16) uint8_t byte_smem[];
+    const uint32_t rec_bytes = units * T::kRec;
+    uint8_t* s = byte_smem + (size_t)warp * ((rec_bytes + 15u) & ~15u);
+    uint4 w[UN], nx[UN];
+    auto load = [&](uint4 (&to)[UN], uint32_t base) {
+#pragma unroll
+        for (uint32_t u = 0; u < UN; ++u) {
+            const uint32_t gi = base + 32u * u + lane;
+            if (gi < groups) to[u] = ld_stream_u4(q + gi);
+        }
+    };
+    // neither the weights nor their scale records depend on the kernel before this one
+    load(w, 0u);
+    load(nx, STEP);
+    const uint8_t* src = S + (size_t)row * rec_bytes;
+    if (((uintptr_t)src & 3u) == 0u && (rec_bytes & 3u) == 0u) {
+        for (uint32_t i = lane; i < rec_bytes / 4u; i += 32u) reinterpret_cast<uint32_t*>(s)[i] = __ldg(reinterpret_cast<const uint32_t*>(src) + i);
+    } else {   // (records of 18 or 14 bytes)
+        for (uint32_t i = lane; i < rec_bytes / 2u; i += 32u) reinterpret_cast<uint16_t*>(s)[i] = __ldg(reinterpret_cast<const uint16_t*>(src) + i);
     }
+    pdl_trigger();   // the kernel behind this one may be scheduled (it waits for this grid before touching what it wrote)
+    pdl_wait();      // the activations come from the preceding kernel
+    __syncwarp();
     float acc[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-    uint32_t gi = lane;
-    for (; gi + 32u * 3u < groups; gi += 32u * 4u) {
-        uint4 w[4];
+    for (uint32_t base = 0; base < groups; base += STEP) {
 #pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) w[u] = ld_stream_u4(q + gi + 32u * u);
+        for (uint32_t u = 0; u < UN; ++u) {
+            const uint32_t gi = base + 32u * u + lane;
+            if (gi < groups) T::template dot<M>(w[u], gi, s, AQ, AD, K, units, acc);
+        }
 #pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) group_dot_q23<M, KIND>(w[u], gi + 32u * u, s, AQ, AB, K, B, acc);
+        for (uint32_t u = 0; u < UN; ++u) w[u] = nx[u];
+        load(nx, base + 2u * STEP);
     }
-    for (; gi < groups; gi += 32u) group_dot_q23<M, KIND>(ld_stream_u4(q + gi), gi, s, AQ, AB, K, B, acc);
 #pragma unroll
     for (int m = 0; m < M; ++m) {
         const float v = warp_sum(acc[m]);
-        if (lane == 0) dst[(size_t)m * dst_stride + row] = v;
+        if (lane == 0) {
+            dst[(size_t)m * dst_stride + row] = v;
+            if (add.out) add.out[(size_t)m * N + row] = v + add.e[(size_t)m * N + row];
+        }
     }
 }
 
-template <int M, int KIND>
-static void launch_q23k_m(const LaunchArgs& a, uint32_t N, uint32_t K, uint32_t dst_stride) {
-    const size_t smem = (size_t)kQ6Warps * (K >> 8) * (KIND == 3 ? 14u : 20u);   // (K <= 65536: at most 40 KB)
-    launch_pdl(gemv_q23k_kernel<M, KIND>, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream,
-               (const uint8_t*)a.ptr[0], (const uint8_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint8_t*)a.ptr[3],
-               (float*)a.ptr[4], N, K, dst_stride);
-}
-
-template <int KIND>
-static AcResult launch_q23k(const LaunchArgs& a) {
-    constexpr uint32_t kRec = KIND == 3 ? 14u : 20u;
+// Bindings 0 Q (one byte per weight, decoded at upload, [N][K]), 1 S (the type's scale records), 2 AQ int8 [M][K], 3 AB
+// (48-byte Q8_K records [M][K/256]) or AD (per-32 scale words), 4 dst f32 [M][dst_stride]; push {M (1..8), N, K, dst_stride}
+template <class T>
+static AcResult launch_byte_gemv(const LaunchArgs& a, uint32_t max_k, uintptr_t s_align) {
     const uint32_t M = a.push[0], N = a.push[1], K = a.push[2], dst_stride = a.push[3];
     if (M == 0 || M > 8) return AC_ERR_INVALID_SHAPE;
-    if (N == 0 || K == 0 || (K & 255u) || K > 65536u || dst_stride < N) return AC_ERR_KERNEL_ARG_INVALID;
-    const uint64_t B = K >> 8;
-    if (a.range[0] < (uint64_t)N * K || a.range[1] < (uint64_t)N * B * kRec || a.range[2] < (uint64_t)M * K ||
-        a.range[3] < (uint64_t)M * B * kABBytes || a.range[4] < ((uint64_t)(M - 1) * dst_stride + N) * 4u)
+    if (N == 0 || K == 0 || (K & ((1u << T::kUnit) - 1u)) || K > max_k || dst_stride < N) return AC_ERR_KERNEL_ARG_INVALID;
+    const uint64_t units = K >> T::kUnit;
+    if (a.range[0] < (uint64_t)N * K || a.range[1] < (uint64_t)N * units * T::kRec || a.range[2] < (uint64_t)M * K ||
+        a.range[3] < (uint64_t)M * units * (T::kUnit == 8u ? kABBytes : 4u) ||
+        a.range[4] < ((uint64_t)(M - 1) * dst_stride + N) * 4u)
         return AC_ERR_INVALID_BUFFER_SIZE;
-    if ((((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[2]) & 15u) || ((uintptr_t)a.ptr[1] & 1u)) return AC_ERR_BUFFER_ALIGNMENT_INVALID;
+    if ((((uintptr_t)a.ptr[0] | (uintptr_t)a.ptr[2]) & 15u) || ((uintptr_t)a.ptr[1] & (s_align - 1u)) ||
+        (T::kUnit == 5u && ((uintptr_t)a.ptr[3] & 3u)))
+        return AC_ERR_BUFFER_ALIGNMENT_INVALID;
+    const size_t smem = (size_t)kQ6Warps * ((units * T::kRec + 15u) & ~15ull);   // (at most 41 KB)
+    const ByteAdd add = {a.add_e, a.add_out};
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream, (const uint8_t*)a.ptr[0],
+                   (const uint8_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint8_t*)a.ptr[3], (float*)a.ptr[4], N, K, dst_stride, add);
+    };
     switch (M) {
-        case 1: launch_q23k_m<1, KIND>(a, N, K, dst_stride); break;
-        case 2: launch_q23k_m<2, KIND>(a, N, K, dst_stride); break;
-        case 3: launch_q23k_m<3, KIND>(a, N, K, dst_stride); break;
-        case 4: launch_q23k_m<4, KIND>(a, N, K, dst_stride); break;
-        case 5: launch_q23k_m<5, KIND>(a, N, K, dst_stride); break;
-        case 6: launch_q23k_m<6, KIND>(a, N, K, dst_stride); break;
-        case 7: launch_q23k_m<7, KIND>(a, N, K, dst_stride); break;
-        default: launch_q23k_m<8, KIND>(a, N, K, dst_stride); break;
+        case 1: go(byte_gemv_kernel<T, 1>); break;
+        case 2: go(byte_gemv_kernel<T, 2>); break;
+        case 3: go(byte_gemv_kernel<T, 3>); break;
+        case 4: go(byte_gemv_kernel<T, 4>); break;
+        case 5: go(byte_gemv_kernel<T, 5>); break;
+        case 6: go(byte_gemv_kernel<T, 6>); break;
+        case 7: go(byte_gemv_kernel<T, 7>); break;
+        default: go(byte_gemv_kernel<T, 8>); break;
     }
     return check_launch();
 }
-
-// ameva_mmvqb_q3_K: bindings 0 Q (int8 [N][K], q3 decoded at upload), 1 S (14-byte records [N][K/256]: scales[12], d),
-// 2 AQ int8 [M][K], 3 AB (48-byte Q8_K records), 4 dst f32; push {M (1..8), N, K (% 256, <= 65536), dst_stride}
-AcResult launch_mmvqb_q3_K(const LaunchArgs& a) { return launch_q23k<3>(a); }
-// ameva_mmvqb_q2_K: the same with Q bytes 0..3 and 20-byte records (scales[16], d, dmin)
-AcResult launch_mmvqb_q2_K(const LaunchArgs& a) { return launch_q23k<2>(a); }
+// S records: Q6_K 18 bytes (scales[16], d), Q5_K 16 (d, dmin, packed scales), IQ4_XS 8 (d, scales_h, scales_l), Q4_1 / Q5_1 4
+// per 32 weights (fp16 d | fp16 m << 16; activations per 32), Q3_K 14 (scales[12], d), Q2_K 20 (scales[16], d, dmin)
+AcResult launch_mmvqb_q6_K(const LaunchArgs& a) { return launch_byte_gemv<ByteQ6K>(a, 65536u, 1u); }
+AcResult launch_mmvqb_q5_K(const LaunchArgs& a) { return launch_byte_gemv<ByteQ5K>(a, 65536u, 16u); }
+AcResult launch_mmvqb_iq4_xs(const LaunchArgs& a) { return launch_byte_gemv<ByteIq4Xs>(a, 65536u, 8u); }
+AcResult launch_mmvq_q4_1(const LaunchArgs& a) { return launch_byte_gemv<ByteQ41>(a, 32768u, 4u); }
+AcResult launch_mmvqb_q3_K(const LaunchArgs& a) { return launch_byte_gemv<ByteQ3K>(a, 65536u, 2u); }
+AcResult launch_mmvqb_q2_K(const LaunchArgs& a) { return launch_byte_gemv<ByteQ2K>(a, 65536u, 2u); }
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Scale table of the tensor-core GEMM for the types above (ameva_mmtc_b8): per 16 weights an fp16 pair (s, o) with

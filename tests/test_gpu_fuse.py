@@ -170,3 +170,19 @@ def test_quantizes_of_the_same_rows(ctx, scheme, M, K, f16):
                 [(gate[0], ["gate", "up", "gate"], gate[2], ONE)] + [(q[0], ["gate"] + q[1][1:], q[2], ONE) for q in qs[:2]],
                 [norm, (qs[0][0], ["y"] + norm[1][3:3 + len(qs[0][1]) - 1], qs[0][2], ONE), qs[1]]):     # the same destination twice
         check(ctx, bufs, ops)
+
+
+@pytest.mark.parametrize("name,unit,rec,act", [("ameva_mmvqb_q6_K", 256, 18, 48), ("ameva_mmvqb_q5_K", 256, 16, 48), ("ameva_mmvqb_iq4_xs", 256, 8, 48),
+                                               ("ameva_mmvq_q4_1", 32, 4, 4), ("ameva_mmvqb_q3_K", 256, 14, 48), ("ameva_mmvqb_q2_K", 256, 20, 48)])
+@pytest.mark.parametrize("M,N,K", [(1, 9, 256), (1, 130, 4352), (3, 17, 2048), (8, 8, 768)])
+def test_byte_decoded_products_with_the_add_behind_them(ctx, name, unit, rec, act, M, N, K):
+    rng = np.random.default_rng(N + K)
+    u = K // unit
+    S = rng.integers(0, 64, (N, u, rec)).astype(np.uint8)
+    A = rng.integers(0, 16, (M, u, act)).astype(np.uint8)
+    bufs = {"q": rng.integers(0, 16, N * K).astype(np.uint8), "s": S, "aq": rng.integers(0, 256, M * K).astype(np.uint8), "ad": A,
+            "o": np.zeros(M * N, np.float32), "e": rng.standard_normal(M * N).astype(np.float32), "r": np.zeros(M * N, np.float32)}
+    gemv = (name, ["q", "s", "aq", "ad", "o"], [M, N, K, N], ONE)
+    for a, b, out in (("o", "e", "r"), ("e", "o", "r"), ("o", "e", "e"), ("o", "e", "o"), ("o", "o", "r")):
+        check(ctx, bufs, [gemv, ("ameva_add_f32", [a, b, out], [M, N, M], ONE)])
+    check(ctx, bufs, [gemv, ("ameva_add_f32", ["o", "e", "r"], [M, N, 1], ONE)])      # one row of e over all
