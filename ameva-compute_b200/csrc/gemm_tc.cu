@@ -231,6 +231,7 @@ struct Params {
     uint32_t n_out;           // destinations (1 = local only; up to 8 with peers)
     uint32_t tiles, row_units;   // output tiles; units of 128 (256 for a CTA pair) weight rows across N
     uint32_t iters, units;    // K blocks per unit in the linear (tile, K block) space; number of units launched
+    uint32_t splits;          // SPLIT kernel: K ranges per tile (2..4), each of `iters` K blocks (the last one the rest)
     uint32_t* flags;          // per (tile, CTA of the pair, epilogue warp) sequence words, zero between launches
     float w_scale;
     uint32_t b8_signed;       // T_B8: the payload bytes are int8 (1) or 0..255 (0)
@@ -266,6 +267,9 @@ __device__ __forceinline__ void trace_cta(const Params& p, uint32_t which) {
 // and a tile cut by a range boundary is produced by several units, whose partial sums are combined in the output
 // itself in a fixed order (descending K): the segment that ends the tile stores, every other one waits for a per-tile
 // sequence flag and then adds with a TMA reduction, so the result does not depend on timing.
+// SPLIT (few tiles): one tile per cluster of 2, 3 or 4 CTA pairs, each taking a K range of it. The partial sums stay in shared
+// memory, and after a cluster barrier every pair adds up its share of the tile's tokens out of the others' shared memory, in
+// order of K: no pair waits for another one's stores (the chain of flags costs about 3 us per K range).
 struct Seg {
     uint32_t tile, kb0, kb1;
 };
@@ -298,7 +302,7 @@ __device__ __forceinline__ bool flag_wait(const uint32_t* flag, uint32_t want, C
 // ---- the kernel -----------------------------------------------------------------------------------------------------
 // PEERS: the launch has other ranks' outputs as destinations (kept out of the single-GPU instantiation, whose main loop
 // would otherwise pay for the forwarding code in registers).
-template <int TYPE, bool PAIR, bool PEERS = false>
+template <int TYPE, bool PAIR, bool PEERS = false, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ CUtensorMap raw_map,
                const __grid_constant__ CUtensorMap scale_map, const __grid_constant__ OutMaps out_maps,
@@ -311,7 +315,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
     // PAIR: blockIdx.x and blockIdx.x ^ 1 form a cluster (one unit); they share the token tile (each stages half of its
     // rows) and own the two 128-row halves of the tile. The even CTA (rank 0) issues the MMAs and owns the full[] and
     // acc_empty barriers.
-    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+    // SPLIT: the cluster holds p.splits pairs; `leader` is the cluster rank of this pair's even CTA.
+    static_assert(!SPLIT || (PAIR && !PEERS), "K ranges of a cluster are multiplied by CTA pairs");
+    const uint32_t crank = PAIR ? cluster_ctarank() : 0u, rank = crank & 1u, leader = SPLIT ? crank & ~1u : 0u;
     const uint32_t unit = PAIR ? blockIdx.x >> 1 : blockIdx.x;
     const uint32_t S = p.b_stages, T = p.tok_tile, Th = PAIR ? T / 2u : T, b_bytes = Th * kRowBytes;
     uint8_t* sB = base;                                               // S x Th*128 B activation stages
@@ -341,7 +347,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
             return;
         }
     }
-    const uint32_t it_begin = unit * p.iters, it_end = min(it_begin + p.iters, p.tiles * KB);
+    const uint32_t split = SPLIT ? crank >> 1 : 0u, tile0 = SPLIT ? unit / p.splits : 0u;
+    const uint32_t it_begin = SPLIT ? tile0 * KB + split * p.iters : unit * p.iters;
+    const uint32_t it_end = SPLIT ? min(it_begin + p.iters, (tile0 + 1u) * KB) : min(it_begin + p.iters, p.tiles * KB);
     uint32_t* status = p.status;
     AMV_TRACE_BEGIN(blockIdx.x)
     AMV_TRACE_STAMP(0)
@@ -412,7 +420,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
                     const uint32_t kbr = kb + rot < KB ? kb + rot : kb + rot - KB;
                     if (PAIR) {   // the even CTA expects both halves' bytes on its barrier; each CTA loads its own half
                         if (rank == 0u) mbar_arrive_expect_tx(full + 8u * st.idx, 2u * b_bytes);
-                        tma_load_2d_pair(smem_u32(sB + st.idx * b_bytes), &act_map, map_to_cta(full + 8u * st.idx, 0u),
+                        tma_load_2d_pair(smem_u32(sB + st.idx * b_bytes), &act_map, map_to_cta(full + 8u * st.idx, leader),
                                          (int)(kbr * C::kBlockK), (int)(m0 + rank * Th));
                     } else {
                         mbar_arrive_expect_tx(full + 8u * st.idx, b_bytes);
@@ -494,11 +502,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
                         for (uint32_t k = 0; k < 4; ++k)   // 32 bytes of K per instruction: 8 TMEM columns / +2 desc units
                             umma_ts<INT8, PAIR>(tmem, ta + 8u * k, db + 2u * k, idesc, (uint32_t)(kb != sg.kb0 || k != 0u));
                     }
-                    umma_commit<PAIR>(empty + 8u * st.idx);
+                    umma_commit<PAIR>(empty + 8u * st.idx, leader);
                     if (dg) w_issue += clock64() - ti;
                 }
                 if (!ok) ctl->abort = 1u;   // visible to whoever passes the accumulator barrier below
-                umma_commit<PAIR>(accum);
+                umma_commit<PAIR>(accum, leader);
                 if (nseg < 2u) { AMV_TRACE_STAMP_AT(ctl->trace_slot, 3u + 5u * nseg) }
                 ++nseg;
             }
@@ -516,7 +524,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
         //      (rows) 32 (w % 4) .. +31, one row and one whole K block per thread ----
         const uint32_t g = warp >> 2, q4 = warp & 3u, r = q4 * 32u + lane;
         const uint32_t eq = q4, cq = g;   // epilogue: TMEM lane quarter, column-chunk phase
-        const uint32_t full_remote = (PAIR && rank != 0u) ? map_to_cta(full, 0u) : 0u;
+        const uint32_t full_remote = (PAIR && rank != 0u) ? map_to_cta(full, leader) : 0u;
         float* stage_out = reinterpret_cast<float*>(sOut) + warp * 512u;
         float* my_unscale = reinterpret_cast<float*>(sUn) + warp * 64u;
         bool ok = true;
@@ -613,7 +621,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
                     __syncwarp();
                     if (lane == 0) {   // the accumulator may be overwritten by the next segment
                         if (PAIR && rank != 0u)
-                            mbar_arrive_cluster(map_to_cta(acc_empty, 0u));
+                            mbar_arrive_cluster(map_to_cta(acc_empty, leader));
                         else
                             mbar_arrive(acc_empty);
                     }
@@ -751,6 +759,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
             }
         };
 
+        if constexpr (SPLIT) {   // one segment, its sums left in shared memory
+            Seg cur;
+            uint32_t it = it_begin;
+            if (next_seg(it, it_end, KB, cur)) {
+                uint32_t kb = cur.kb0;
+                for (const uint32_t pre = min(cur.kb1, kb + S); kb < pre && ok; ++kb) dequant_step(cur, kb);
+                pdl_wait();
+                for (; kb < cur.kb1 && ok; ++kb) dequant_step(cur, kb);
+                // the MMAs have finished: nothing reads the activation stages any more, which become [T][128] sums
+                ok = ok && mbar_wait(accum, 0u, ctl, status, 0x500u) && !ctl->abort;
+                ok = __all_sync(0xffffffffu, ok);
+                tc_fence_after();
+                for (uint32_t c = cq; c * 16u < T && ok; c += kDequantGroups) {
+                    uint32_t v[16];
+                    tmem_ld16(tmem + ((eq * 32u) << 16) + c * 16u, v);
+#pragma unroll
+                    for (uint32_t j = 0; j < 16u; ++j) reinterpret_cast<uint32_t*>(sB)[(c * 16u + j) * kRows + r] = v[j];
+                }
+            }
+        } else {
         // Segments in order. Before the epilogue of a segment the warps run ahead into the next one by up to S K blocks:
         // those land in operand stages that the MMAs of the current segment free, so the waits cannot depend on the
         // epilogue they precede, and the MMA issuer finds work as soon as the accumulator has been read out.
@@ -781,11 +809,68 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
             have = have_next;
         }
         if (p.tma_store && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        }
         if (lane == 0 && q4 == 0u) {
             trace_val(p, 1610u + 4u * g, w_sc);
             trace_val(p, 1611u + 4u * g, w_raw);
             trace_val(p, 1612u + 4u * g, w_empty);
             trace_val(p, 1613u + 4u * g, w_accum);
+        }
+    }
+    if constexpr (SPLIT) {
+        // Tokens split, split + splits, ... of the tile are this pair's: a warp adds one token's 128 rows (16 bytes per lane and
+        // K range) in order of K, multiplies the token's factor and writes one 512-byte line.
+        const uint32_t m0 = (tile0 / p.row_units) * T, n0 = ((tile0 % p.row_units) * 2u + rank) * kRows;
+        constexpr uint32_t kMine = kTokMax / 2u / kDequantWarps;   // tokens per warp at most (two K ranges)
+        float factor[kMine];
+        if (warp < (uint32_t)kDequantWarps) {
+#pragma unroll
+            for (uint32_t i = 0; i < kMine; ++i) {
+                const uint32_t m = min(m0 + (i * kDequantWarps + warp) * p.splits + split, p.M - 1u);
+                factor[i] = INT8 ? __fmul_rn(__uint_as_float(__ldg(p.act + 2u * m)), p.w_scale) : __ldg(p.row_unscale + m);
+            }
+        }
+        __syncwarp();
+        cluster_sync();   // every pair's sums are in its shared memory (a pair that gave up leaves garbage; the host is told)
+        if (warp < (uint32_t)kDequantWarps && !ctl->abort) {
+            const uint32_t part = smem_u32(sB) + 16u * lane, row = n0 + 4u * lane;
+#pragma unroll
+            for (uint32_t i = 0; i < kMine; ++i) {
+                const uint32_t t = (i * kDequantWarps + warp) * p.splits + split, m = m0 + t;
+                if (t >= T || m >= p.M) continue;
+                uint4 x[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k)
+                    if (k < p.splits) x[k] = ld_cluster_u4(map_to_cta(part + t * (kRows * 4u), 2u * k + rank));
+                float y[4];
+                if (INT8) {
+                    uint4 sum = x[0];
+#pragma unroll
+                    for (uint32_t k = 1; k < 4u; ++k)
+                        if (k < p.splits) sum.x += x[k].x, sum.y += x[k].y, sum.z += x[k].z, sum.w += x[k].w;
+                    y[0] = (float)(int)sum.x, y[1] = (float)(int)sum.y, y[2] = (float)(int)sum.z, y[3] = (float)(int)sum.w;
+                } else {
+                    y[0] = __uint_as_float(x[0].x), y[1] = __uint_as_float(x[0].y), y[2] = __uint_as_float(x[0].z), y[3] = __uint_as_float(x[0].w);
+#pragma unroll
+                    for (uint32_t k = 1; k < 4u; ++k)
+                        if (k < p.splits) {
+                            y[0] += __uint_as_float(x[k].x);
+                            y[1] += __uint_as_float(x[k].y);
+                            y[2] += __uint_as_float(x[k].z);
+                            y[3] += __uint_as_float(x[k].w);
+                        }
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k) y[k] = __fmul_rn(y[k], factor[i]);
+                float* out = p.dst + (size_t)m * p.dst_stride + row;
+                if (p.tma_store && row + 3u < p.N) {   // (rows of the output 16-byte aligned)
+                    *reinterpret_cast<float4*>(out) = make_float4(y[0], y[1], y[2], y[3]);
+                } else {
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        if (row + k < p.N) out[k] = y[k];
+                }
+            }
         }
     }
     tc_fence_before();
@@ -1287,6 +1372,33 @@ static int resident_units(uint32_t smem_bytes, int sm_count) {
     return n;
 }
 
+// Clusters of `splits` CTA pairs of the SPLIT kernel that are resident at once.
+template <int TYPE>
+static int resident_split_clusters(uint32_t smem_bytes, uint32_t splits, int sm_count) {
+    static PerDeviceMemo memo[3];
+    const int dev = current_device();
+    int n = 0;
+    if (memo[splits - 2u].get(dev, smem_bytes, &n)) return n;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(2u * splits * (unsigned)sm_count);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2u * splits;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<TYPE, true, false, true>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    if (n > 0) memo[splits - 2u].put(dev, smem_bytes, n);
+    return n;
+}
+
 // Shared memory of the wide kernel: everything but the activation ring, then the ring for T tokens per accumulator.
 template <int TYPE>
 static uint32_t wide_smem_bytes(uint32_t T, uint32_t b_stages) {
@@ -1445,6 +1557,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
     }
     if (!ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, false>>((int)kSmemLimit) ||
         !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false>>((int)kSmemLimit) ||
+        !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false, true>>((int)kSmemLimit) ||
         !ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, true>>((int)kSmemLimit) ||
         !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, true>>((int)kSmemLimit))
         return AC_ERR_INVALID_WORK_GROUP_SIZE;
@@ -1538,6 +1651,36 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
         }
         break;
     }
+    // Few tiles: K ranges in clusters (SPLIT) where that finishes earlier. Costs in thirds of a microsecond, from measured
+    // launches: a K block about 0.55 us at 256 tokens and 0.4 us at few (the conversion's share), a flag chain 3 us per extra
+    // K range of a tile, the exchange through a cluster 2 us; every unit resident in one wave.
+    if (pair && !n_peers && !forced && !(diag & 64u) && (KB & 3u) == 0u) {
+        auto block_cost = [](uint32_t T) { return 12u + T / 50u; };   // per K block, in units of 1/30 us
+        const uint32_t chain = p.iters < KB ? (KB + p.iters - 1u) / p.iters : 1u;
+        uint64_t best = (uint64_t)((p.units + (uint32_t)sm_count / 2u - 1u) / ((uint32_t)sm_count / 2u)) * p.iters * block_cost(p.tok_tile) +
+                        90ull * (chain - 1u) + 90u + p.tok_tile / 4u;
+        uint32_t best_T = 0, best_n = 0, best_iters = 0;
+        for (uint32_t j = (M + tok_max - 1u) / tok_max, tries = 0; tries < 4u && j <= M; ++j, ++tries) {
+            const uint32_t T = (((M + j - 1u) / j) + 31u) & ~31u, tiles = p.row_units * ((M + T - 1u) / T);
+            if (fixed + (uint32_t)kMaxStages * (T / 2u) * kRowBytes > kSmemLimit) continue;   // (the sums take the eight stages' memory)
+            for (uint32_t n = 2u; n <= 4u; ++n) {
+                const uint32_t iters = ((KB + n - 1u) / n + 3u) & ~3u;
+                if ((KB + iters - 1u) / iters != n) continue;   // (every K range has blocks)
+                const int clusters = resident_split_clusters<TYPE>(fixed + (uint32_t)kMaxStages * (T / 2u) * kRowBytes, n, sm_count);
+                if (clusters < 1 || tiles > (uint32_t)clusters) continue;
+                const uint64_t cost = (uint64_t)iters * block_cost(T) + 60u + 90u + T / 4u / n;
+                if (cost < best) best = cost, best_T = T, best_n = n, best_iters = iters;
+            }
+        }
+        if (best_n) {
+            p.splits = best_n;
+            p.tok_tile = best_T;
+            p.b_stages = kMaxStages;
+            p.tiles = p.row_units * ((M + best_T - 1u) / best_T);
+            p.iters = best_iters;
+            p.units = p.tiles * best_n;
+        }
+    }
     const uint32_t tok_rows = pair ? p.tok_tile / 2u : p.tok_tile;   // token rows staged by one CTA
     const uint32_t smem_bytes = fixed + p.b_stages * tok_rows * kRowBytes;
 
@@ -1578,7 +1721,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
     cfg.stream = a.stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = pair ? 2 : 1;
+    attr[0].val.clusterDim.x = p.splits ? 2u * p.splits : pair ? 2 : 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see pdl_wait in the kernel
@@ -1586,7 +1729,9 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     cudaError_t e;
-    if (n_peers)
+    if (p.splits)
+        e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<TYPE, true, false, true>, act_map, raw_map, scale_map, out_maps, p);
+    else if (n_peers)
         e = pair ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<TYPE, true, true>, act_map, raw_map, scale_map, out_maps, p)
                  : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<TYPE, false, true>, act_map, raw_map, scale_map, out_maps, p);
     else

@@ -29,6 +29,15 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// 16 bytes of the shared memory of another CTA of the cluster (map_to_cta address)
+__device__ __forceinline__ uint4 ld_cluster_u4(uint32_t cluster_addr) {
+    uint4 v;
+    asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(cluster_addr)
+                 : "memory");
+    return v;
+}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -53,11 +62,12 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     else
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// One arrival on `bar` when the MMAs issued so far have finished; with PAIR on the barrier at that offset in both CTAs.
+// One arrival on `bar` when the MMAs issued so far have finished; with PAIR on the barrier at that offset in both CTAs (cluster
+// ranks leader and leader + 1).
 template <bool PAIR>
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t leader = 0u) {
     if (PAIR) {
-        const uint16_t both = 3;
+        const uint16_t both = (uint16_t)(3u << leader);
         asm volatile(
             "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
                 bar),
