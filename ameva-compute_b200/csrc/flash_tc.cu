@@ -8,15 +8,19 @@
 //   warp 4      issues the MMAs: S = Q K^T (both in shared memory) into one of two TMEM buffers, then O += P V with P read
 //               from tensor memory and V as an MN-major shared-memory operand; S of tile j + 1 is issued before P V of tile
 //               j, so the softmax of the next tile starts while the tensor core multiplies this one;
-//   warps 0-3   one row per thread: read the 64 scores, online softmax in fp32, write P (fp16) over the scores. The
-//               accumulator is rescaled only when a row's maximum has grown by more than kGrowth since its last rescale
-//               (probabilities then stay below e^kGrowth, well inside fp16, and the sum carries the same factor).
+//   warps 0-3   one row per thread: read the 64 scores, online softmax in fp32, write P over the scores as two fp16 halves
+//               (rounded value and remainder: the 64 columns of the scores hold both). The accumulator is rescaled only
+//               when a row's maximum has grown by more than kGrowth since its last rescale (probabilities then stay below
+//               e^kGrowth, well inside fp16, and the sum carries the same factor).
 // Before the tiles of a window are processed the mask is scanned once: tiles that are masked for all 128 rows are left out
 // of the list every role walks, tiles whose mask is all zero skip the mask arithmetic (a causal prompt has one or two mixed
 // tiles per CTA). Two CTAs per SM: the exponentials of one overlap the MMAs of the other.
 // Bound by: the exponentials (64 per thread and tile) and the MMAs, both about 500 cycles per tile and CTA. The form it
 // replaces (mma.sync, 64 rows per CTA) ran at 77 TFLOP/s.
-// Rounding as in the other attention kernels: Q and P to fp16 once, scores, sums and accumulation in fp32.
+// Rounding: Q to fp16 once as in the other attention kernels, scores, sums and accumulation in fp32. P with its remainder:
+// with the lazy reference the largest probability of a row is no longer exactly 1, and P rounded once left an error 1-5 %
+// above the mma.sync form's (2.9e-4 against 2.8e-4 of the result); with the remainder it is 2.1e-4. Rescaling at every
+// new maximum instead cost the same time and left 2.8e-4.
 // Every wait is bounded (sync_ptx.cuh); a CTA that gives up drains its copies and MMAs, frees its TMEM and returns.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -256,8 +260,11 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
                     tc_fence_after();
                     const uint64_t dv = make_v_desc(smem_u32(sV + vm.idx * L::kTile));
 #pragma unroll
-                    for (uint32_t k = 0; k < kKeys / 16u; ++k)   // 16 keys: 8 columns of P, two groups of eight V rows
-                        umma_ts<false, false>(tmem_o, tmem + (j & 1u) * kKeys + 8u * k, dv + 128u * k, idesc_o, (uint32_t)((j | k) != 0u));
+                    for (uint32_t k = 0; k < kKeys / 16u; ++k) {   // 16 keys: 8 columns of P (high, then low), two groups of eight V rows
+                        const uint32_t ta = tmem + (j & 1u) * kKeys + 8u * k;
+                        umma_ts<false, false>(tmem_o, ta, dv + 128u * k, idesc_o, (uint32_t)((j | k) != 0u));
+                        umma_ts<false, false>(tmem_o, ta + 32u, dv + 128u * k, idesc_o, 1u);
+                    }
                     umma_commit<false>(v_empty + 8u * vm.idx);
                     umma_commit<false>(pv_done + 8u * (j & 1u));
                     vm.advance();
@@ -337,7 +344,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
                 }
                 const float ref = (m_run == ninf ? 0.0f : m_run) * kLog2e, mul = plain ? scale * kLog2e : kLog2e;
                 const float m_nat = m_run == ninf ? 0.0f : m_run;
-                uint32_t ph[kKeys / 2u];
+                uint32_t ph[kKeys / 2u], pl[kKeys / 2u];   // P as fp16 and what that rounding left, again as fp16
+                auto split = [&](uint32_t k, float p0, float p1) {
+                    const __half2 h = __floats2half2_rn(p0, p1);
+                    const float2 f = __half22float2(h);
+                    ph[k] = *reinterpret_cast<const uint32_t*>(&h);
+                    pl[k] = pack_halves(p0 - f.x, p1 - f.y);
+                };
                 float s0 = 0.0f, s1 = 0.0f;
                 if (plain) {
 #pragma unroll
@@ -345,7 +358,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
                         const float p0 = ex2(fmaf(x[2u * k], mul, -ref)), p1 = ex2(fmaf(x[2u * k + 1u], mul, -ref));
                         s0 += p0;
                         s1 += p1;
-                        ph[k] = pack_halves(p0, p1);
+                        split(k, p0, p1);
                     }
                 } else {   // the difference first: scores next to a large mask value keep their spacing
 #pragma unroll
@@ -353,11 +366,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
                         const float p0 = ex2((x[2u * k] - m_nat) * kLog2e), p1 = ex2((x[2u * k + 1u] - m_nat) * kLog2e);
                         s0 += p0;
                         s1 += p1;
-                        ph[k] = pack_halves(p0, p1);
+                        split(k, p0, p1);
                     }
                 }
                 l_run += s0 + s1;
-                tmem_st32(tmem + lanes + b * kKeys, ph);   // over this tile's scores (waits for the store)
+                tmem_st32(tmem + lanes + b * kKeys, ph);   // over this tile's scores (waits for the stores)
+                tmem_st32(tmem + lanes + b * kKeys + 32u, pl);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(p_full + 8u * b);
