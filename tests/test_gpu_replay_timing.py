@@ -1,0 +1,71 @@
+"""GPU times of replayed batches: every event keeps its own, however many replays follow and whatever becomes of the batch."""
+import numpy as np
+import pytest
+
+from conftest import load_pkg
+
+pytestmark = pytest.mark.gpu
+pkg = load_pkg()
+rt = pkg.runtime
+
+
+@pytest.mark.parametrize("replays", [1, 62, 63, 64, 200])
+def test_every_replay_keeps_its_gpu_time(replays):
+    ctx = rt.init()
+    n = 1 << 20
+    a, b, d = (ctx.buffer(data=np.full(n, v, np.float32)) for v in (1.0, 2.0, 0.0))
+    batches = []
+    for k in (1, 16):       # a short one and one that takes several times as long
+        batch = ctx.batch(32)
+        for _ in range(k):
+            batch.dispatch(ctx.kernel("ameva_add_f32"), [a, b, d], [1, n, 1])
+        batch.instantiate()
+        batches.append(batch)
+    events = [[batches[i].replay() for _ in range(replays)] for i in (0, 1)]
+    for evs in events:
+        evs[-1].wait()
+    short = [0.0] * replays
+    for i, ev in enumerate(events[0]):
+        ev.wait()
+        short[i] = ev.gpu_duration_us()
+    for batch in batches:
+        batch.destroy()     # the times of the second batch are read after it is gone
+    for i, ev in enumerate(events[1]):
+        ev.wait()
+        us = ev.gpu_duration_us()
+        assert 0 < short[i] < us < 1e6
+        assert us == ev.gpu_duration_us()
+    for evs in events:
+        for ev in evs:
+            ev.destroy()
+    for x in (a, b, d):
+        x.destroy()
+    ctx.destroy()
+
+
+def test_more_replayable_batches_than_rings():
+    ctx = rt.init()
+    x = ctx.buffer(data=np.ones(1024, np.float32))
+    batches = []
+    for _ in range(70):
+        batch = ctx.batch(1)
+        batch.dispatch(ctx.kernel("ameva_add_f32"), [x, x, x], [1, 1024, 1])
+        batch.instantiate()
+        batches.append(batch)
+    for batch in batches:
+        ev = batch.replay()
+        ev.wait()
+        assert 0 < ev.gpu_duration_us() < 1e6
+        ev.destroy()
+    for batch in batches:
+        batch.destroy()
+    again = ctx.batch(1)
+    again.dispatch(ctx.kernel("ameva_add_f32"), [x, x, x], [1, 1024, 1])
+    again.instantiate()
+    ev = again.replay()
+    ev.wait()
+    assert ev.gpu_duration_us() > 0
+    ev.destroy()
+    again.destroy()
+    x.destroy()
+    ctx.destroy()
