@@ -1342,6 +1342,9 @@ static int resident_units(uint32_t smem_bytes, int sm_count) {
     const int dev = current_device();
     int n = 0;
     if (memo.get(dev, smem_bytes, &n)) return n;
+    if (PAIR ? !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true>>((int)kSmemLimit)   // (the queries need the limit raised)
+             : !ensure_dynamic_smem<gemm_tc_kernel<TYPE, false>>((int)kSmemLimit))
+        return 0;
     if (PAIR) {
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
@@ -1379,6 +1382,7 @@ static int resident_split_clusters(uint32_t smem_bytes, uint32_t splits, int sm_
     const int dev = current_device();
     int n = 0;
     if (memo[splits - 2u].get(dev, smem_bytes, &n)) return n;
+    if (!ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false, true>>((int)kSmemLimit)) return 0;   // (the query needs the limit raised)
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(2u * splits * (unsigned)sm_count);
@@ -1555,13 +1559,6 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
             (dst_stride & 3u) == 0u && ((uintptr_t)dstp & 15u) == 0u && (N & 3u) == 0u)
             return launch_wide<TYPE>(a, enc, Qp, Sp, act, dstp, M, N, K, dst_stride, row_unscale, diag);
     }
-    if (!ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, false>>((int)kSmemLimit) ||
-        !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false>>((int)kSmemLimit) ||
-        !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false, true>>((int)kSmemLimit) ||
-        !ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, true>>((int)kSmemLimit) ||
-        !ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, true>>((int)kSmemLimit))
-        return AC_ERR_INVALID_WORK_GROUP_SIZE;
-
     Params p;
     memset(&p, 0, sizeof(p));
     p.dst = (float*)dstp;
@@ -1666,6 +1663,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
             for (uint32_t n = 2u; n <= 4u; ++n) {
                 const uint32_t iters = ((KB + n - 1u) / n + 3u) & ~3u;
                 if ((KB + iters - 1u) / iters != n) continue;   // (every K range has blocks)
+                if (2u * n * tiles > (uint32_t)sm_count) continue;
                 const int clusters = resident_split_clusters<TYPE>(fixed + (uint32_t)kMaxStages * (T / 2u) * kRowBytes, n, sm_count);
                 if (clusters < 1 || tiles > (uint32_t)clusters) continue;
                 const uint64_t cost = (uint64_t)iters * block_cost(T) + 60u + 90u + T / 4u / n;
@@ -1728,6 +1726,13 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
+    // (only the kernel that is launched: asking for an attribute loads a kernel's code, milliseconds the first time)
+    const bool fits = p.splits ? ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false, true>>((int)kSmemLimit)
+                      : n_peers ? (pair ? ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, true>>((int)kSmemLimit)
+                                        : ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, true>>((int)kSmemLimit))
+                                : (pair ? ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false>>((int)kSmemLimit)
+                                        : ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, false>>((int)kSmemLimit));
+    if (!fits) return AC_ERR_INVALID_WORK_GROUP_SIZE;
     cudaError_t e;
     if (p.splits)
         e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<TYPE, true, false, true>, act_map, raw_map, scale_map, out_maps, p);

@@ -85,6 +85,19 @@ def test_gemm_i2s_bit_exact(ctx, M, N, K):
 
 
 @pytest.mark.parametrize("t", [Q8_0, Q4_0, Q4_K])
+@pytest.mark.parametrize("M,N,K", [(9, 129, 2048), (31, 257, 4096), (33, 511, 1280), (77, 1027, 3328), (160, 512, 6400), (255, 1024, 4096),
+                                   (256, 256, 8192), (300, 1000, 4096), (512, 258, 2304)])
+def test_k_ranges_in_clusters(ctx, t, M, N, K):
+    """Few tiles: two to four CTA pairs per tile, the last K range shorter, rows of the output on and off 16 bytes (N odd)."""
+    run_gemm(ctx, t, M, N, K, seed=M + K)
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 129, 2560), (77, 515, 6912), (128, 1024, 2560), (256, 300, 4096)])
+def test_i2s_k_ranges_in_clusters_bit_exact(ctx, M, N, K):
+    run_gemm(ctx, I2_S, M, N, K, seed=M + 1)
+
+
+@pytest.mark.parametrize("t", [Q8_0, Q4_0, Q4_K])
 def test_exact_path_block_sums_at_prefill_m(ctx, t):
     run_gemm(ctx, t, 24, 96, 512, seed=5, exact=True)
 
