@@ -40,7 +40,7 @@ uint64_t now_ns() {
 // GPU start and end times of the replays of a batch, written by a one-thread kernel at either end of its graph: a ring in
 // device memory that get_timing reads on demand. A pair of timed events around the graph took 6 us of every replay (a
 // one-kernel graph alone 2.0 us, with the events 8.2, with the stamps 4.1).
-constexpr uint32_t kStampSlots = 63;
+constexpr uint32_t kStampSlots = 1023;   // (about as many launches as a stream queues before it holds the host up)
 struct StampRing {
     unsigned long long seq;   // replays so far (device side)
     unsigned long long pad;
@@ -137,7 +137,7 @@ struct AcCommandBatch {
     bool started, completed;
     StampRing* ring;             // REPLAYABLE: device ring of this batch, or null
     uint64_t replays;
-    AcEvent* stamped[kStampSlots];   // the event that owns each slot
+    std::vector<AcEvent*> stamped;   // with a ring: the event that owns each slot
 };
 
 namespace {
@@ -1101,7 +1101,6 @@ AcResult ac_runtime_batch_begin_ex(AcContext* context, const AcBatchDesc* desc, 
     b->exec = nullptr;
     b->ring = nullptr;
     b->replays = 0;
-    memset(b->stamped, 0, sizeof(b->stamped));
     b->records.reserve(desc->max_dispatches < 256 ? desc->max_dispatches : 256);
     context->live_batches++;
     *out_batch = b;
@@ -1258,6 +1257,7 @@ AcResult ac_b200_batch_instantiate(AcCommandBatch* batch) {
         give_ring(ctx, batch->ring);
         batch->ring = nullptr;
     }
+    if (batch->ring) batch->stamped.assign(kStampSlots, nullptr);
     auto drop_ring = [&]() {
         give_ring(ctx, batch->ring);
         batch->ring = nullptr;
