@@ -14,7 +14,8 @@
 //               e^kGrowth, well inside fp16, and the sum carries the same factor).
 // Before the tiles of a window are processed the mask is scanned once: tiles that are masked for all 128 rows are left out
 // of the list every role walks, tiles whose mask is all zero skip the mask arithmetic (a causal prompt has one or two mixed
-// tiles per CTA). Two CTAs per SM: the exponentials of one overlap the MMAs of the other.
+// tiles per CTA), and of a mixed tile only the k-steps of 16 keys that some row sees are multiplied with V: what lies in the
+// cache behind the last visible key (never written, perhaps NaN) takes no part. Two CTAs per SM: the exponentials of one overlap the MMAs of the other.
 // Bound by: the exponentials (64 per thread and tile) and the MMAs, both about 500 cycles per tile and CTA. The form it
 // replaces (mma.sync, 64 rows per CTA) ran at 77 TFLOP/s.
 // Rounding: Q to fp16 once as in the other attention kernels, scores, sums and accumulation in fp32. P with its remainder:
@@ -42,6 +43,8 @@ using namespace tc;
 constexpr uint32_t kRows = 128, kKeys = 64, kStages = 2;
 constexpr uint32_t kSoftmaxWarps = 4, kWarpMma = 4, kWarpLoad = 5, kThreads = 192;
 constexpr uint32_t kWindow = 512;      // key tiles scanned and listed at a time
+// An entry of the list: tile of the window, a bit per 16 keys that some row sees, mixed.
+constexpr uint32_t kTileMask = kWindow - 1u, kStepShift = 9, kAllSteps = 15u << kStepShift, kMixed = 0x8000u, kNoTile = 0x7FFFu;
 constexpr uint32_t kTmemCols = 256;    // two S buffers of 64 columns, then D columns of O
 constexpr float kGrowth = 5.0f;        // e^5 = 148
 constexpr float kLog2e = 1.44269504088896340736f;
@@ -82,7 +85,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
     uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kStages * L::kTile);
     Ctl* ctl = reinterpret_cast<Ctl*>(bars + 24);
     uint32_t* s_count = reinterpret_cast<uint32_t*>(ctl + 1);
-    uint16_t* s_list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + 256);   // tile of the window | mixed << 15
+    uint16_t* s_list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + 256);   // see kTileMask
     const uint32_t k_full = smem_u32(bars), k_empty = k_full + 8u * kStages, v_full = k_empty + 8u * kStages,
                    v_empty = v_full + 8u * kStages, s_full = v_empty + 8u * kStages, p_full = s_full + 16u, pv_done = p_full + 16u,
                    drain = pv_done + 16u;
@@ -206,22 +209,25 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
                         }
                     }
                 }
-                open = __any_sync(0xffffffffu, open);
+                const uint32_t seen = __ballot_sync(0xffffffffu, open);   // lanes 8 r + p: keys 8 p .. 8 p + 7
                 nonzero = __any_sync(0xffffffffu, nonzero);
-                if (lane == 0) s_list[t] = (uint16_t)(open ? (t | (nonzero ? 0x8000u : 0u)) : 0x7FFFu);
+                uint32_t steps = 0;
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k) steps |= (seen & (0x03030303u << (2u * k))) ? 1u << k : 0u;
+                if (lane == 0) s_list[t] = (uint16_t)(seen ? (t | steps << kStepShift | (nonzero ? kMixed : 0u)) : kNoTile);
             }
         } else {
             for (uint32_t t = threadIdx.x; t < nw; t += kThreads)
-                s_list[t] = (uint16_t)(t | (key_begin + (w0 + t + 1u) * kKeys <= key_end ? 0u : 0x8000u));
+                s_list[t] = (uint16_t)(t | kAllSteps | (key_begin + (w0 + t + 1u) * kKeys <= key_end ? 0u : kMixed));
         }
         __syncthreads();
         if (warp == 0) {   // compaction in place: entries move to lower positions, 32 at a time
             uint32_t n = 0;
             for (uint32_t t = 0; t < nw; t += 32u) {
-                const uint16_t e = t + lane < nw ? s_list[t + lane] : (uint16_t)0x7FFFu;
-                const uint32_t keep = __ballot_sync(0xffffffffu, e != 0x7FFFu);
+                const uint16_t e = t + lane < nw ? s_list[t + lane] : (uint16_t)kNoTile;
+                const uint32_t keep = __ballot_sync(0xffffffffu, e != kNoTile);
                 __syncwarp();
-                if (e != 0x7FFFu) s_list[n + __popc(keep & ((1u << lane) - 1u))] = e;
+                if (e != kNoTile) s_list[n + __popc(keep & ((1u << lane) - 1u))] = e;
                 __syncwarp();
                 n += __popc(keep);
             }
@@ -233,7 +239,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
         if (warp == kWarpLoad) {
             if (lane == 0) {
                 for (uint32_t i = 0; i < n && ok; ++i) {
-                    const int key0 = (int)(key_begin + (w0 + (s_list[i] & 0x7FFFu)) * kKeys);
+                    const int key0 = (int)(key_begin + (w0 + (s_list[i] & kTileMask)) * kKeys);
                     ok = mbar_wait(k_empty + 8u * kl.idx, kl.phase ^ 1u, ctl, status, 0xB00u);
                     if (!ok) break;
                     mbar_arrive_expect_tx(k_full + 8u * kl.idx, L::kTile);
@@ -281,11 +287,15 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t dv = make_v_desc(smem_u32(sV + vm.idx * L::kTile));
+                    const uint32_t steps = (uint32_t)s_list[i] >> kStepShift;   // (at least one of a listed tile)
+                    uint32_t acc = j != 0u;
 #pragma unroll
                     for (uint32_t k = 0; k < kKeys / 16u; ++k) {   // 16 keys: 8 columns of P (high, then low), two groups of eight V rows
+                        if (!(steps >> k & 1u)) continue;
                         const uint32_t ta = tmem + (j & 1u) * kKeys + 8u * k;
-                        umma_ts<false, false>(tmem_o, ta, dv + 128u * k, idesc_o, (uint32_t)((j | k) != 0u));
+                        umma_ts<false, false>(tmem_o, ta, dv + 128u * k, idesc_o, acc);
                         umma_ts<false, false>(tmem_o, ta + 32u, dv + 128u * k, idesc_o, 1u);
+                        acc = 1u;
                     }
                     umma_commit<false>(v_empty + 8u * vm.idx);
                     umma_commit<false>(pv_done + 8u * (j & 1u));
@@ -296,8 +306,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
             const uint32_t lanes = (warp * 32u) << 16;
             for (uint32_t i = 0; i < n; ++i) {
                 const uint32_t j = done + i, b = j & 1u, e = s_list[i];
-                const uint32_t key0 = key_begin + (w0 + (e & 0x7FFFu)) * kKeys;
-                const bool mixed = (e & 0x8000u) != 0u;
+                const uint32_t key0 = key_begin + (w0 + (e & kTileMask)) * kKeys;
+                const bool mixed = (e & kMixed) != 0u;
                 ok = ok && mbar_wait(s_full + 8u * b, (j >> 1) & 1u, ctl, status, 0xB50u);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;

@@ -144,6 +144,21 @@ def test_masked_rows_and_lowest_values(ctx):
     assert np.max(np.abs(got[9] - want[9])) < 2e-2
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("last,m_off", [(288, 0), (272, 0), (304, 3), (16, 0)])
+def test_unused_cache_behind_the_last_key_of_a_tile(ctx, D, last, m_off):
+    """The keys in use end inside a tile of 64; behind them the cache holds NaN and infinities that no row sees (the mask read
+    in pieces of eight and one by one)."""
+    n_q, n_kv = 64, 512
+    q, k, v = inputs(n_q, n_kv, 2, 2, D, 5)
+    k[last:], v[last:] = np.inf, np.nan
+    mask = np.zeros((n_q, n_kv), np.float16)
+    mask[:, last:] = -np.inf
+    got = run(ctx, q, k, v, mask, D ** -0.5, m_off=m_off)
+    want = attention(q, k[:last], v[:last], None, D ** -0.5)
+    assert np.max(np.abs(got - want)) < TOL
+
+
 def test_more_keys_than_one_window(ctx):
     """More key tiles than one scan of the mask covers (512), in one split."""
     n_q, n_kv, D = 17, 512 * 64 + 200, 64
