@@ -22,7 +22,8 @@
 // with the lazy reference the largest probability of a row is no longer exactly 1, and P rounded once left an error 1-5 %
 // above the mma.sync form's (2.9e-4 against 2.8e-4 of the result); with the remainder it is 2.1e-4. Rescaling at every
 // new maximum instead cost the same time and left 2.8e-4.
-// Every wait is bounded (sync_ptx.cuh); a CTA that gives up drains its copies and MMAs, frees its TMEM and returns.
+// Every wait on a barrier is bounded (sync_ptx.cuh); a CTA that gives up drains its copies and MMAs, frees its TMEM and
+// returns. The allocation of TMEM has no bound of its own: it waits for CTAs that are resident already, and those end.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -107,7 +108,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
         fence_barrier_init();
     }
     if (warp == kWarpMma) tmem_alloc<false>(smem_u32(&ctl->tmem_base), kTmemCols);
-    pdl_trigger();
     pdl_wait();
     const uint32_t z = blockIdx.x, hkv = blockIdx.y;
     const uint32_t G = pc.n_head / pc.n_head_kv, h0 = hkv * G, QT = kRows / G;
@@ -148,6 +148,9 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // Not earlier than the barrier that publishes the allocation: a CTA of the kernel behind this one could otherwise take the
+    // tensor memory this CTA is still waiting for, and hold it while it waits for this grid.
+    pdl_trigger();
     const uint32_t tmem = ctl->tmem_base, tmem_o = tmem + 2u * kKeys;
 
     // softmax state of this thread's row (warps 0-3)

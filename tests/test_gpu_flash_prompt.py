@@ -181,3 +181,43 @@ def test_one_position_over_few_and_many_blocks(ctx, D, H, Hkv, n_kv):
     for _ in range(2):      # (the second launch finds the arrival counters as the first left them)
         assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5) - want)) < TOL
     assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5, scratch=64) - want)) < TOL
+
+
+def test_prompt_attention_among_kernels_with_tensor_memory(ctx):
+    """Attention and tensor-core products in turn in one batch: each holds tensor memory, and each may be scheduled while the
+    one before it still runs. Same bytes as one by one."""
+    qmm = pkg.qmm
+    from helpers import Q8_0, make_acts, make_weights
+    n_q, H, D = 160, 4, 64
+    q, k, v = inputs(n_q, n_q, H, H, D, 21)
+    mask = causal(n_q, n_q, 192)
+    N, K = 384, 256
+    blocks, scale = make_weights(Q8_0, N, K, 3)
+    w = qmm.QuantWeight.from_ggml(ctx, Q8_0, blocks, N, K, scale)
+    mm = qmm.MulMat(ctx, w, n_q)
+    push = [D, D, n_q, n_q, H, H, 0x11, 1, 0, H * D, D, 0, H * D, D, 0, H * D, D, 0, 192, 192 * n_q, 1, 0, fbits(D ** -0.5), 0, 0, 0, 0, 0,
+            0, 0, 0]
+    bufs = [ctx.buffer(data=np.ascontiguousarray(a)) for a in (q, k, v, mask)] + [ctx.buffer(n_q * H * D * 4), ctx.buffer(1 << 22)]
+    x, y = ctx.buffer(data=make_acts(n_q, K, 4)), ctx.buffer(n_q * N * 4)
+
+    def go(rounds):
+        batch = ctx.batch(64)
+        for _ in range(rounds):
+            batch.dispatch(ctx.kernel("ameva_flash_attn"), bufs, push, (1, 1, 1))
+            mm.record(batch, x, y, n_q)
+            batch.dispatch(ctx.kernel("ameva_flash_attn"), bufs, push, (1, 1, 1))
+            mm.record(batch, x, y, n_q, quantize=False)
+        ev = batch.submit()
+        ev.wait()
+        ev.destroy()
+        batch.destroy()
+        return bufs[4].read(np.uint8), y.read(np.uint8)
+
+    one, many = go(1), go(8)
+    assert np.array_equal(one[0], many[0]) and np.array_equal(one[1], many[1])
+    want = attention(q, k, v, mask[:, :n_q], D ** -0.5)
+    assert np.max(np.abs(one[0].view(np.float32).reshape(n_q, H, D) - want)) < TOL
+    mm.destroy()
+    w.destroy()
+    for b in bufs + [x, y]:
+        b.destroy()
