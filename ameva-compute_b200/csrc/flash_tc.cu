@@ -73,10 +73,54 @@ __device__ __forceinline__ uint64_t make_v_desc(uint32_t smem_addr) {
            (2ull << 61);
 }
 
+// One row by a whole warp, masked keys left out instead of multiplied by zero: a lane's D / 32 columns (from column lane * D / 32)
+// of sum p V over the keys of the split, p = exp(score - ref). For rows whose accumulator is not finite: the products above
+// multiply every key of a step with every row, so a NaN or an infinity in V would reach rows that do not see its key, and an
+// infinity would meet the remainder of its probability, which may be zero or negative. Rare, so simple: a lane per key for the
+// scores, all lanes on a key's columns for the sum.
+template <int D>
+__device__ __noinline__ float4 seen_keys_row(const float* qrow, const __half* k, const __half* v, const __half* mrow, uint32_t k_s1,
+                                             uint32_t v_s1, uint32_t key_begin, uint32_t key_end, float scale, float softcap, float ref) {
+    constexpr int C = D / 32;
+    const uint32_t lane = threadIdx.x & 31u;
+    const float ninf = __uint_as_float(0xFF800000u);
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (uint32_t key0 = key_begin; key0 < key_end; key0 += 32u) {
+        const uint32_t key = key0 + lane;
+        const float mv = key >= key_end ? ninf : mrow ? __half2float(mrow[key]) : 0.0f;
+        float p = 0.0f;
+        if (mv != ninf) {
+            const uint4* row = reinterpret_cast<const uint4*>(k + (uint64_t)key * k_s1);
+            float s = 0.0f;
+            for (uint32_t c = 0; c < (uint32_t)D / 8u; ++c) {
+                const uint4 x = row[c];
+                const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 kf = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+                    s = fmaf(h2f(f2h(qrow[8u * c + 2u * j])), kf.x, s);
+                    s = fmaf(h2f(f2h(qrow[8u * c + 2u * j + 1u])), kf.y, s);
+                }
+            }
+            s *= scale;
+            if (softcap != 0.0f) s = softcap * tanhf(s / softcap);
+            p = ex2((s + mv - ref) * kLog2e);
+        }
+        for (uint32_t seen = __ballot_sync(0xffffffffu, mv != ninf); seen; seen &= seen - 1u) {
+            const int b = __ffs(seen) - 1;
+            const float pb = __shfl_sync(0xffffffffu, p, b);
+            const __half* row = v + (uint64_t)(key0 + b) * v_s1 + C * lane;
+#pragma unroll
+            for (int c = 0; c < C; ++c) acc[c] = fmaf(pb, __half2float(row[c]), acc[c]);
+        }
+    }
+    return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads, 2)
 flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const float* __restrict__ q,
-                const __half* __restrict__ mask, float* __restrict__ o, float* __restrict__ part, const FlashArgs pc,
+                const __half* __restrict__ k, const __half* __restrict__ v, const __half* __restrict__ mask, float* __restrict__ o, float* __restrict__ part, const FlashArgs pc,
                 uint32_t n_splits, uint32_t vec, uint32_t* status) {
     using L = Smem<D>;
     constexpr uint32_t A = L::kAtoms;
@@ -427,21 +471,41 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant
             float* stage = reinterpret_cast<float*>(base) + warp * 32u * D;
             const float inv = n_splits == 1u ? 1.0f / l_run : 1.0f;
             const uint32_t lanes = (warp * 32u) << 16;
+            float check = 0.0f;   // NaN once a column is not finite
 #pragma unroll 1
             for (uint32_t c = 0; c < (uint32_t)D; c += 32u) {
-                uint32_t v[32];
+                uint32_t x[32];
                 if (done) {
-                    tmem_ld32_async(tmem_o + lanes + c, v);
+                    tmem_ld32_async(tmem_o + lanes + c, x);
                     tmem_wait_ld();
                 } else {   // every key was masked: nothing was accumulated
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) v[k] = 0u;
+                    for (int j = 0; j < 32; ++j) x[j] = 0u;
                 }
 #pragma unroll
-                for (uint32_t k = 0; k < 8u; ++k)
-                    reinterpret_cast<float4*>(stage)[lane * kChunks + (((c >> 2) + k) ^ (lane & 7u))] =
-                        make_float4(__uint_as_float(v[4u * k]) * inv, __uint_as_float(v[4u * k + 1u]) * inv,
-                                    __uint_as_float(v[4u * k + 2u]) * inv, __uint_as_float(v[4u * k + 3u]) * inv);
+                for (int j = 0; j < 32; ++j) check = fmaf(__uint_as_float(x[j]), 0.0f, check);
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j)
+                    reinterpret_cast<float4*>(stage)[lane * kChunks + (((c >> 2) + j) ^ (lane & 7u))] =
+                        make_float4(__uint_as_float(x[4u * j]) * inv, __uint_as_float(x[4u * j + 1u]) * inv,
+                                    __uint_as_float(x[4u * j + 2u]) * inv, __uint_as_float(x[4u * j + 3u]) * inv);
+            }
+            __syncwarp();
+            // (a sum of probabilities that is not finite says that the scores are not: the row is NaN either way)
+            for (uint32_t bad = __ballot_sync(0xffffffffu, my_valid && check != 0.0f && l_run - l_run == 0.0f); bad; bad &= bad - 1u) {
+                const int i = __ffs(bad) - 1;
+                const uint32_t r = warp * 32u + i, iq = q0 + r / G, head = h0 + r % G;
+                const float m = __shfl_sync(0xffffffffu, m_run, i), f = __shfl_sync(0xffffffffu, inv, i);
+                const __half* mrow = pc.has_mask ? mask + pc.m_off + (uint64_t)iq * pc.m_s1 + (uint64_t)(head % pc.m_ne2) * pc.m_s2 : nullptr;
+                const float4 x = seen_keys_row<D>(q + pc.q_off + (uint64_t)iq * pc.q_s1 + (uint64_t)head * pc.q_s2,
+                                                  k + pc.k_off + (uint64_t)hkv * pc.k_s2, v + pc.v_off + (uint64_t)hkv * pc.v_s2, mrow, pc.k_s1,
+                                                  pc.v_s1, key_begin, key_end, scale, softcap, m == ninf ? 0.0f : m);
+                const float y[4] = {x.x * f, x.y * f, x.z * f, x.w * f};
+#pragma unroll
+                for (uint32_t c = 0; c < D / 32u; ++c) {
+                    const uint32_t e = lane * (D / 32u) + c;
+                    stage[4u * (i * kChunks + ((e >> 2) ^ (i & 7u))) + (e & 3u)] = y[c];
+                }
             }
             __syncwarp();
             for (uint32_t i = 0; i < 32u; ++i) {
@@ -498,7 +562,8 @@ static bool launch_d(const LaunchArgs& a, const CUtensorMap& km, const CUtensorM
                      uint32_t q_tiles, uint32_t vec) {
     if (!ensure_dynamic_smem<flash_tc_kernel<D>>((int)Smem<D>::kBytes)) return false;
     launch_pdl(flash_tc_kernel<D>, dim3(n_splits, pc.n_head_kv, q_tiles), dim3(kThreads), Smem<D>::kBytes, a.stream, km, vm,
-               (const float*)a.ptr[0], (const __half*)a.ptr[3], (float*)a.ptr[4], (float*)a.ptr[5], pc, n_splits, vec, a.status);
+               (const float*)a.ptr[0], (const __half*)a.ptr[1], (const __half*)a.ptr[2], (const __half*)a.ptr[3], (float*)a.ptr[4],
+               (float*)a.ptr[5], pc, n_splits, vec, a.status);
     return true;
 }
 

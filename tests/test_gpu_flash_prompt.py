@@ -159,6 +159,42 @@ def test_unused_cache_behind_the_last_key_of_a_tile(ctx, D, last, m_off):
     assert np.max(np.abs(got - want)) < TOL
 
 
+def seen(q, k, v, mask, scale):
+    """As attention(), each row over the keys it sees only: what is masked is no term of the sum."""
+    out = np.zeros(q.shape)
+    rep = q.shape[1] // k.shape[1]
+    with np.errstate(invalid="ignore"):
+        for h in range(q.shape[1]):
+            for i in range(q.shape[0]):
+                at = mask[i] != -np.inf
+                s = k[at, h // rep].astype(np.float64) @ q[i, h].astype(np.float16).astype(np.float64) * scale
+                p = np.exp(s - s.max())
+                out[i, h] = (p[:, None] * v[at, h // rep].astype(np.float64)).sum(0) / p.sum()
+    return out
+
+
+@pytest.mark.parametrize("D,H,Hkv", [(64, 4, 4), (128, 4, 2), (128, 8, 1)])
+@pytest.mark.parametrize("scratch", [64, 1 << 24])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them(ctx, D, H, Hkv, scratch):
+    """V rows of infinities, of either sign, and of NaN: a position in front of them (causal mask) gives what it would give
+    without them, one behind them +inf, -inf or NaN in the same columns as the sum over its keys."""
+    n_q, n_kv = 150, 700
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 31)
+    mask = causal(n_q, n_kv, 704)
+    v[600, :, 1::3] = np.inf
+    v[655, :, 2::5] = -np.inf
+    v[690, 0, ::7] = np.nan
+    v[697:, :, :] = np.nan
+    mask[:, 697:] = -np.inf
+    want = seen(q, k, v, mask[:, :n_kv], D ** -0.5)
+    got = run(ctx, q, k, v, mask, D ** -0.5, scratch=scratch)
+    finite = np.isfinite(want)
+    assert finite.any() and np.isposinf(want).any() and np.isneginf(want).any() and np.isnan(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    assert np.max(np.abs(got[finite] - want[finite])) < TOL
+
+
 def test_more_keys_than_one_window(ctx):
     """More key tiles than one scan of the mask covers (512), in one split."""
     n_q, n_kv, D = 17, 512 * 64 + 200, 64
