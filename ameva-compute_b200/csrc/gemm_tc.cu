@@ -440,6 +440,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constan
         // ---- packed-weight TMA: rows n0 .. n0+127 (rows past N read as zero), one 128-byte-per-row box per kGroup K
         //      blocks; the scales of a 256-weight group once per 4 K blocks. Segments start on multiples of 4 blocks. ----
         if (lane == 0) {
+            // T_B8: the scale table may be the work of the kernel before this one (ameva_mmtc_scales); the scales of the other
+            // types are the weight's own (3203 x 3328, 77 rows: 18.4 us with and without the wait)
+            if (TYPE == T_B8) pdl_wait();
             Ring rr(C::kRawSlots), sr(kScaleSlots);
             Seg sg;
             uint32_t it = it_begin, groups = 0;

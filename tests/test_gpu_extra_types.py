@@ -292,3 +292,38 @@ def test_gemm_scale_table_holds_the_decoded_scales(ctx):
         finally:
             mm.destroy()
             w.destroy()
+
+
+@pytest.mark.parametrize("N,K,M", [(768, 4096, 33), (3203, 3328, 77), (4096, 512, 300)])
+def test_scale_table_written_right_before_the_product_that_reads_it(ctx, N, K, M):
+    """What a host without a table per weight records: quantize, table of the first weight, its product, the same table
+    filled from the second weight, its product, all in one batch. Same bytes as with tables of their own."""
+    x = make_acts(M, K, 5)
+    xb, shared = ctx.buffer(data=x), ctx.buffer(N * (K // 16) * 4)
+    ws = [qmm.QuantWeight.from_ggml(ctx, Q6_K, make_weights(Q6_K, N, K, s)[0], N, K) for s in (1, 2)]
+    mms = [qmm.MulMat(ctx, w, M) for w in ws]
+    outs, want = [ctx.buffer(M * N * 4) for _ in ws], []
+    grid = (1, 1, 1)
+    try:
+        for mm, o in zip(mms, outs):
+            mm.run(xb, o, M)
+            want.append(o.read(np.uint8))
+            o.write(np.zeros(M * N, np.float32))
+        batch = ctx.batch(64)
+        for _ in range(4):
+            mm = mms[0]
+            batch.dispatch(ctx.kernel("ameva_quant_a8b_f16"), [xb, mm.aq, mm.ad, mm.ah, mm.ae], [M, K, K, mm.q8k_mode], grid)
+            for m, o in zip(mms, outs):
+                batch.dispatch(ctx.kernel("ameva_mmtc_scales"), [m.sbind, shared], [Q6_K, N, K], grid)
+                batch.dispatch(ctx.kernel("ameva_mmtc_b8"), [m.qbind, shared, mm.ah, o, mm.ae], [M, N, K, N, 0, 1], grid)
+        batch.instantiate()
+        for _ in range(8):
+            ev = batch.replay()
+            ev.wait()
+            ev.destroy()
+            for o, y in zip(outs, want):
+                assert np.array_equal(o.read(np.uint8), y)
+        batch.destroy()
+    finally:
+        for o in mms + outs + [xb, shared] + ws:
+            o.destroy()
