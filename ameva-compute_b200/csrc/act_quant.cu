@@ -646,7 +646,7 @@ static QuantDst quant_dst(const LaunchArgs& a, QuantForm form) {
 
 // pieces per thread: a row of K floats over 512 threads, 4 (per-32) or 8 (per-256) floats to a piece
 template <int SCHEME, int PRE>
-static AcResult launch_rows(cudaStream_t stream, const float* src, const QuantDsts& dst, uint32_t M, uint32_t K, uint32_t stride,
+static AcResult launch_rows(LaunchStream stream, const float* src, const QuantDsts& dst, uint32_t M, uint32_t K, uint32_t stride,
                             uint32_t mode, const NormArgs& na) {
     const uint32_t per_thread = (K + (SCHEME ? 4095u : 2047u)) / (SCHEME ? 4096u : 2048u);
     auto go = [&](auto kernel) { launch_pdl(kernel, dim3(M), dim3(kRowThreads), 0, stream, src, dst, K, stride, mode, na); };
@@ -662,26 +662,27 @@ static AcResult launch_rows(cudaStream_t stream, const float* src, const QuantDs
 template <int SCHEME>
 static AcResult launch_quant_scheme(QuantForm form, const LaunchArgs& first, const QuantDsts& dst, const LaunchArgs* swiglu) {
     const uint32_t M = first.push[0], K = first.push[1], stride = first.push[2], mode = first.push[3];
+    const LaunchStream stream = swiglu ? swiglu->stream : first.stream;   // (of the dispatch that comes first)
     if (form == QUANT_NORM) {
         float eps;
         memcpy(&eps, &first.push[4], 4);
         const NormArgs na = {first.push[5] ? (const float*)first.ptr[1] : nullptr, (float*)first.ptr[2], eps};
-        return launch_rows<SCHEME, ROWS_NORM>(first.stream, (const float*)first.ptr[0], dst, M, K, stride, mode, na);
+        return launch_rows<SCHEME, ROWS_NORM>(stream, (const float*)first.ptr[0], dst, M, K, stride, mode, na);
     }
     const float* src = (const float*)(swiglu ? swiglu->ptr[0] : first.ptr[0]);
     if (form == QUANT_F16) {
         if (swiglu) {
             const NormArgs na = {(const float*)swiglu->ptr[1], (float*)swiglu->ptr[2], 0.0f};
-            return launch_rows<SCHEME, ROWS_SWIGLU>(first.stream, src, dst, M, K, K, mode, na);
+            return launch_rows<SCHEME, ROWS_SWIGLU>(stream, src, dst, M, K, K, mode, na);
         }
         const NormArgs na = {nullptr, nullptr, 0.0f};
-        return launch_rows<SCHEME, ROWS_PLAIN>(first.stream, src, dst, M, K, stride, mode, na);
+        return launch_rows<SCHEME, ROWS_PLAIN>(stream, src, dst, M, K, stride, mode, na);
     }
     const uint64_t blocks = ((uint64_t)M * (SCHEME ? (K >> 8) * 32ull : (K >> 5) * 8ull) + 255u) / 256u;
     if (blocks > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
     const GateArgs ga = {swiglu ? (const float*)swiglu->ptr[1] : nullptr, swiglu ? (float*)swiglu->ptr[2] : nullptr};
     auto go = [&](auto kernel) {
-        launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, first.stream, src, dst, M, K, swiglu ? K : stride, mode, ga);
+        launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, stream, src, dst, M, K, swiglu ? K : stride, mode, ga);
     };
     if (SCHEME == 0) {
         if (swiglu) go(quant_q8_0_kernel<true>);
@@ -733,7 +734,7 @@ bool bitnet_rows_fits(const LaunchArgs& a) {
 }
 
 template <int SOURCE>
-static void launch_bitnet_rows_j(cudaStream_t stream, const BitnetRows& g, uint32_t dim, uint32_t rows) {
+static void launch_bitnet_rows_j(LaunchStream stream, const BitnetRows& g, uint32_t dim, uint32_t rows) {
     const uint32_t J = ((dim >> 2) + 255u) / 256u;
     const dim3 grid(rows), block(256);
     if (J <= 1) launch_pdl(bitnet_rows_kernel<SOURCE, 1>, grid, block, 0, stream, g, dim);
@@ -745,6 +746,7 @@ static void launch_bitnet_rows_j(cudaStream_t stream, const BitnetRows& g, uint3
 AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const LaunchArgs* const* norm_q8, uint32_t n) {
     const LaunchArgs& first = *norm_q8[0];
     const uint32_t dim = first.push[0], rows = first.grid.x;
+    const LaunchStream stream = head ? head->stream : first.stream;   // (of the dispatch that comes first)
     BitnetRows g;
     memset(&g, 0, sizeof(g));
     g.n = n;
@@ -755,18 +757,18 @@ AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const L
     }
     if (source == BITNET_PLAIN) {
         g.a = (const float*)first.ptr[0];
-        launch_bitnet_rows_j<BITNET_PLAIN>(first.stream, g, dim, rows);
+        launch_bitnet_rows_j<BITNET_PLAIN>(stream, g, dim, rows);
     } else if (source == BITNET_NORM) {
         g.a = (const float*)head->ptr[0];
         g.b = head->push[3] ? (const float*)head->ptr[1] : nullptr;
         g.h = (float*)head->ptr[2];
         memcpy(&g.eps, &head->push[2], 4);
-        launch_bitnet_rows_j<BITNET_NORM>(first.stream, g, dim, rows);
+        launch_bitnet_rows_j<BITNET_NORM>(stream, g, dim, rows);
     } else {
         g.a = (const float*)head->ptr[0];
         g.b = (const float*)head->ptr[1];
         g.h = (float*)head->ptr[2];
-        launch_bitnet_rows_j<BITNET_SWIGLU>(first.stream, g, dim, rows);
+        launch_bitnet_rows_j<BITNET_SWIGLU>(stream, g, dim, rows);
     }
     return check_launch();
 }

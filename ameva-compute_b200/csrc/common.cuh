@@ -28,8 +28,18 @@ struct SideQueues {
     bool pending[8];   // work was queued on stream i since the last join
 };
 
+// The stream of a launch. in_order: not before everything in front of it has completed, i.e. without the programmatic launch
+// attribute (see launch_pdl); for a kernel whose early reads (BindingUse) something still running may write.
+struct LaunchStream {
+    cudaStream_t s;
+    bool in_order;
+    LaunchStream() = default;
+    LaunchStream(cudaStream_t stream) : s(stream), in_order(false) {}
+    operator cudaStream_t() const { return s; }
+};
+
 struct LaunchArgs {
-    cudaStream_t stream;
+    LaunchStream stream;
     uint32_t binding_count;
     void* ptr[16];
     uint64_t range[16];
@@ -58,6 +68,12 @@ struct KernelEntry {
 const KernelEntry* find_kernel(const char* name);
 uint32_t kernel_count();
 const KernelEntry* kernel_at(uint32_t i);
+// Bindings of a kernel (bit i: binding i) that it reads before it waits for the kernels in front of it (a product's weights),
+// and bindings that it does not write (those, and the tables and records of weights that other kernels read).
+struct BindingUse {
+    uint32_t early, read_only;
+};
+BindingUse binding_use(const KernelEntry* e, const uint32_t* push);
 AcResult register_kernel(const char* name, uint32_t binding_count, uint32_t push_bytes, AcB200LaunchFn fn);
 // repack.cu: the ggml -> device-regions permutation of blocks [first, first + nblk) of a tensor, from staged ggml bytes
 AcResult launch_repack(cudaStream_t stream, uint32_t type, const void* src, void* q_region, void* s_region, uint64_t first,
@@ -140,17 +156,19 @@ __device__ __forceinline__ void trace_stamp(uint32_t slot, uint32_t i) {
 #define AMV_TRACE_READER(file)
 #endif
 
-// Programmatic dependent launch. The quantize and mul_mat kernels are launched with the attribute (launch_pdl) and begin
-// with pdl_wait, which returns when the preceding grid of the stream has completed and its writes are visible, followed
-// by pdl_trigger, which lets the next kernel of the stream be scheduled once all CTAs of this grid have started. Nothing
-// touches memory before its wait, so only launch latency and set-up overlap. After a kernel that never triggers (the
-// peer barrier), or a copy, the dependent simply starts when that work is done.
+// Programmatic dependent launch. Kernels are launched with the attribute (launch_pdl); pdl_trigger lets the next kernel of the
+// stream be scheduled once all CTAs of this grid have issued it, pdl_wait returns when the preceding grid has completed (and
+// with it, by its own wait, every grid before) and its writes are visible. Before its wait a kernel touches nothing but the
+// weights of a product, which binding_use (registry.cu) names: they are requested while the kernels in front still run. So
+// nothing that is still running may write them, and the runtime sees to that (flush_batch): a product whose weights an
+// earlier dispatch of the batch may write, and the first launch of a batch, are launched in order. After a kernel that never
+// triggers (the peer barrier), or a copy, the dependent starts when that work is done.
 // ---------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, LaunchStream stream,
                               Args&&... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -162,7 +180,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = stream.in_order ? 0 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

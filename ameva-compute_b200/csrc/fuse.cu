@@ -153,7 +153,7 @@ AcResult fuse_bitnet_gemv(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
     for (uint32_t j = i + 1; j < n && j <= i + kLookahead && count < kFuseMax; ++j) {
         if (ops[j].done) continue;
         const LaunchArgs& p = ops[j].args;
-        if (is(ops[j], launch_bitnet_gemv_i2_s) && p.push[0] == K && (p.push[4] ? p.push[4] : 1u) == M &&
+        if (is(ops[j], launch_bitnet_gemv_i2_s) && !p.stream.in_order && p.push[0] == K && (p.push[4] ? p.push[4] : 1u) == M &&
             check_bitnet_gemv_i2_s(p) == AC_SUCCESS && can_hoist(ops, i, j, mask)) {
             bool ok = true;   // no product writes what another one reads or writes
             for (uint32_t m = 0; m < count && ok; ++m)
@@ -266,7 +266,7 @@ AcResult fuse_row_ops(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
     if (count < 2u) return AC_SUCCESS;
     *taken = true;
     for (uint32_t k = 0; k < count; ++k) ops[at[k]].done = true;
-    return launch_row_ops(rope, store, n_rope, set, n_set);
+    return launch_row_ops(ops[i].args.stream, rope, store, n_rope, set, n_set);
 }
 
 // ---- per-32 / per-256 quantizes of the same rows ----

@@ -42,7 +42,7 @@ AcResult launch_quant_group(QuantForm form, uint32_t scheme, const LaunchArgs& f
 // its result (store[i], nullptr: none)
 bool row_op_serves(const LaunchArgs& a, bool rope);
 bool rope_feeds_set_rows(const LaunchArgs& rope, const LaunchArgs& set);
-AcResult launch_row_ops(const LaunchArgs* const* rope, const LaunchArgs* const* store, uint32_t n_rope, const LaunchArgs* const* set,
-                        uint32_t n_set);
+AcResult launch_row_ops(LaunchStream stream, const LaunchArgs* const* rope, const LaunchArgs* const* store, uint32_t n_rope,
+                        const LaunchArgs* const* set, uint32_t n_set);
 
 }  // namespace amv

@@ -1522,7 +1522,7 @@ static AcResult launch_wide(const LaunchArgs& a, EncodeTiledFn enc, const void* 
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = a.stream.in_order ? 1 : 2;
     if (cudaLaunchKernelEx(&cfg, gemm_tc_wide_kernel<TYPE>, act_map, raw_map, scale_map, out_maps, p) != cudaSuccess) {
         cudaGetLastError();
         return AC_ERR_INVALID_WORK_GROUP_SIZE;
@@ -1728,7 +1728,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see pdl_wait in the kernel
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = a.stream.in_order ? 1 : 2;
     // (only the kernel that is launched: asking for an attribute loads a kernel's code, milliseconds the first time)
     const bool fits = p.splits ? ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false, true>>((int)kSmemLimit)
                       : n_peers ? (pair ? ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, true>>((int)kSmemLimit)

@@ -467,8 +467,8 @@ bool rope_feeds_set_rows(const LaunchArgs& rope, const LaunchArgs& set) {
            st.ne03 == 1u && (st.nr == 1u || st.a_s1 == r.d_s2);
 }
 
-AcResult launch_row_ops(const LaunchArgs* const* rope, const LaunchArgs* const* store, uint32_t n_rope, const LaunchArgs* const* set,
-                        uint32_t n_set) {
+AcResult launch_row_ops(LaunchStream stream, const LaunchArgs* const* rope, const LaunchArgs* const* store, uint32_t n_rope,
+                        const LaunchArgs* const* set, uint32_t n_set) {
     RowOps g;
     memset(&g, 0, sizeof(g));
     uint64_t ctas = 0;
@@ -504,7 +504,7 @@ AcResult launch_row_ops(const LaunchArgs* const* rope, const LaunchArgs* const* 
         g.end[2 + i] = (uint32_t)ctas;
     }
     if (ctas > 0x7FFFFFFFull) return AC_ERR_INVALID_WORK_ITEM_DIMS;
-    launch_pdl(row_ops_kernel, dim3((unsigned)ctas), dim3(256), 0, n_rope ? rope[0]->stream : set[0]->stream, g);
+    launch_pdl(row_ops_kernel, dim3((unsigned)ctas), dim3(256), 0, stream, g);
     return check_launch();
 }
 

@@ -202,6 +202,22 @@ const KernelEntry* kernel_at(uint32_t i) {
     if (i < kBuiltin) return &kTable[i];
     return i - kBuiltin < registered_count() ? &g_registered[i - kBuiltin] : nullptr;
 }
+BindingUse binding_use(const KernelEntry* e, const uint32_t* push) {
+    if (!e->launch) return {0u, 0u};
+    auto starts = [&](const char* prefix) { return strncmp(e->name, prefix, strlen(prefix)) == 0; };
+    if (starts("ameva_mm")) {
+        if (starts("ameva_mmtc_scales")) return {0u, 1u};
+        if (starts("ameva_mmvs_")) return {0u, 3u};      // Q, S, after its wait
+        if (starts("ameva_mmtc_b8")) return {1u, 3u};    // Q; the scale table after its wait
+        if (!starts("ameva_mmvqg")) return {3u, 3u};     // Q, S
+        const uint32_t qs = 0x6DBu & ((1u << 3u * (push[2] < 4u ? push[2] : 4u)) - 1u);   // (Q, S, dst) x count
+        return {qs, qs};
+    }
+    if (starts("bitnet_gemv_i2_s") || starts("bitnet_gemm_i2_s")) return {1u, 1u};        // W
+    if (starts("bitnet_gemv_f16") || starts("ameva_get_rows")) return {0u, 1u};           // the table may be a product's weight
+    return {0u, 0u};
+}
+
 const KernelEntry* find_kernel(const char* name) {
     if (!name) return nullptr;
     for (uint32_t i = 0, n = kernel_count(); i < n; ++i)

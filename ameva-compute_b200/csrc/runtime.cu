@@ -6,6 +6,7 @@
 // bounded event waits, and the generation-based first-error-wins error state (src/runtime/ac_error.cpp:30-93).
 // The execution model is the one the reference's OpenCL backend documents (include/ac_runtime.h:614-630): one in-order
 // queue per context (here a CUDA stream), batches that run at flush/submit, host access through write/read/fill only.
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -122,6 +123,34 @@ struct BatchRecord {
     AcDim3 grid;
 };
 
+// Address ranges, merged and in order: a few tens for a batch of any length, as its dispatches work on the same buffers.
+struct RangeSet {
+    std::vector<std::pair<uintptr_t, uintptr_t>> r;
+    std::vector<std::pair<uintptr_t, uintptr_t>>::iterator first_past(uintptr_t at) {   // the first range that ends behind `at`
+        return std::upper_bound(r.begin(), r.end(), at, [](uintptr_t x, const std::pair<uintptr_t, uintptr_t>& y) { return x < y.second; });
+    }
+    bool meets(const void* p, uint64_t n) {
+        const auto it = first_past((uintptr_t)p);
+        return it != r.end() && it->first < (uintptr_t)p + n;
+    }
+    void add(const void* p, uint64_t n) {
+        uintptr_t a = (uintptr_t)p, b = a + n;
+        auto it = first_past(a);
+        if (it != r.end() && it->first <= a && b <= it->second) return;
+        auto end = it;
+        for (; end != r.end() && end->first < b; ++end) {
+            a = std::min(a, end->first);
+            b = std::max(b, end->second);
+        }
+        if (it == end) {
+            r.insert(it, {a, b});
+        } else {
+            *it = {a, b};
+            r.erase(it + 1, end);
+        }
+    }
+};
+
 struct AcCommandBatch {
     uint32_t magic;
     AcContext* ctx;
@@ -130,6 +159,8 @@ struct AcCommandBatch {
     uint32_t max_dispatches, flags;
     std::vector<BatchRecord> records;
     size_t flushed;  // records already launched
+    uint32_t launches, launches_in_order;   // dispatches that left the host, alone or as a fused form; of those, in order
+    RangeSet written;   // device memory that the dispatches launched so far may have written
     AcBatchStats stats;
     cudaEvent_t t_begin;
     std::vector<cudaEvent_t> t_after;  // one per dispatch with AC_BATCH_FLAG_DISPATCH_TIMESTAMPS
@@ -230,7 +261,7 @@ LaunchArgs launch_args(AcContext* ctx, uint32_t nbind, void* const* ptrs, const 
 }
 
 AcResult launch_record(AcContext* ctx, const KernelEntry* e, uint32_t nbind, void* const* ptrs, const uint64_t* ranges,
-                       const uint32_t* push, AcDim3 grid) {
+                       const uint32_t* push, AcDim3 grid, bool in_order) {
     if (!e->launch) {   // a registered kernel: the public form of the same arguments
         AcB200Launch l;
         l.stream = ctx->stream;
@@ -243,7 +274,9 @@ AcResult launch_record(AcContext* ctx, const KernelEntry* e, uint32_t nbind, voi
         l.grid = grid;
         return e->ext(&l);
     }
-    return e->launch(launch_args(ctx, nbind, ptrs, ranges, push, grid));
+    LaunchArgs a = launch_args(ctx, nbind, ptrs, ranges, push, grid);
+    a.stream.in_order = in_order;
+    return e->launch(a);
 }
 
 bool abi_ok(uint32_t abi_version, uint32_t struct_size, size_t expect) {
@@ -396,7 +429,8 @@ void release_records(AcCommandBatch* b) {
     }
 }
 
-AcResult flush_batch(AcCommandBatch* b) {
+// capture: into a graph, whose first node starts when everything in front of the graph has completed
+AcResult flush_batch(AcCommandBatch* b, bool capture = false) {
     AcContext* ctx = b->ctx;
     DeviceGuard g(ctx->device);
     const bool ts = (b->flags & (AC_BATCH_FLAG_TIMESTAMPS | AC_BATCH_FLAG_DISPATCH_TIMESTAMPS)) != 0;
@@ -414,6 +448,15 @@ AcResult flush_batch(AcCommandBatch* b) {
         void* ptrs[16];
         for (uint32_t i = 0; i < r.nbind; ++i) ptrs[i] = (char*)r.buf[i]->dptr + r.offset[i];
         ops[k] = {r.kernel->entry, launch_args(ctx, r.nbind, ptrs, r.range, r.push, r.grid), false};
+        // Weights are read before the kernels in front have completed (see launch_pdl): not where one of them may write them.
+        // The first launch waits for all that other batches have in flight.
+        const BindingUse use = binding_use(r.kernel->entry, r.push);
+        bool in_order = k == 0 && !capture;
+        for (uint32_t i = 0; i < r.nbind; ++i)
+            if (use.early >> i & 1u) in_order = in_order || b->written.meets(ptrs[i], r.range[i]);
+        for (uint32_t i = 0; i < r.nbind; ++i)
+            if (!(use.read_only >> i & 1u)) b->written.add(ptrs[i], r.range[i]);
+        ops[k].args.stream.in_order = in_order;
     }
     // dispatch timestamps ask for the time of every dispatch: each is launched by itself
     const bool fuse = !(b->flags & AC_BATCH_FLAG_DISPATCH_TIMESTAMPS);
@@ -423,8 +466,10 @@ AcResult flush_batch(AcCommandBatch* b) {
         const KernelEntry* e = ops[k].entry;
         const LaunchArgs& a = ops[k].args;
         const AcResult rc = fuse && e->launch ? launch_fused(ops.data(), (uint32_t)n, (uint32_t)k)
-                                              : launch_record(ctx, e, a.binding_count, a.ptr, a.range, a.push, a.grid);
+                                              : launch_record(ctx, e, a.binding_count, a.ptr, a.range, a.push, a.grid, a.stream.in_order);
         if (rc != AC_SUCCESS) return fail(ctx, rc, AMEVA_BACKEND_OP_DISPATCH);
+        b->launches++;
+        b->launches_in_order += a.stream.in_order;
         if (b->flags & AC_BATCH_FLAG_DISPATCH_TIMESTAMPS) {
             cudaEvent_t ev;
             if (cudaEventCreate(&ev) != cudaSuccess) return AC_ERR_OUT_OF_HOST_MEMORY;
@@ -1014,7 +1059,7 @@ AcResult ac_runtime_dispatch(AcContext* ctx, const AcLaunchDesc* desc, AcEvent**
     r = make_event(ctx, true, &ev);
     if (r != AC_SUCCESS) return r;
     cudaEventRecord(ev->start, ctx->stream);
-    r = launch_record(ctx, e, desc->buffer_count, ptrs, ranges, push, desc->grid_dim);
+    r = launch_record(ctx, e, desc->buffer_count, ptrs, ranges, push, desc->grid_dim, true);
     if (r != AC_SUCCESS) {
         free_event(ev);
         return fail(ctx, r, AMEVA_BACKEND_OP_DISPATCH);
@@ -1095,6 +1140,7 @@ AcResult ac_runtime_batch_begin_ex(AcContext* context, const AcBatchDesc* desc, 
     b->max_dispatches = desc->max_dispatches;
     b->flags = desc->flags;
     b->flushed = 0;
+    b->launches = b->launches_in_order = 0;
     memset(&b->stats, 0, sizeof(b->stats));
     b->t_begin = b->t_end = nullptr;
     b->started = b->completed = false;
@@ -1268,7 +1314,7 @@ AcResult ac_b200_batch_instantiate(AcCommandBatch* batch) {
         return fail(ctx, AC_ERR_FEATURE_NOT_SUPPORTED, AMEVA_BACKEND_OP_DISPATCH);
     }
     if (batch->ring) amv::launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, ctx->stream, batch->ring, 0u);
-    const AcResult r = flush_batch(batch);
+    const AcResult r = flush_batch(batch, true);
     if (batch->ring) amv::launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, ctx->stream, batch->ring, 1u);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -1348,6 +1394,14 @@ void ac_runtime_batch_destroy(AcCommandBatch* batch) {
     ctx->live_batches--;
     batch->magic = kMagicDead;
     delete batch;
+}
+
+AcResult ac_b200_batch_get_launches(const AcCommandBatch* batch, uint32_t* out_launches, uint32_t* out_in_order) {
+    if (!bat_ok(batch)) return AC_ERR_INVALID_ARGUMENT;
+    if (!out_launches || !out_in_order) return AC_ERR_NULL_POINTER;
+    *out_launches = batch->launches;
+    *out_in_order = batch->launches_in_order;
+    return AC_SUCCESS;
 }
 
 AcResult ac_runtime_batch_get_dispatch_times(const AcCommandBatch* batch, uint64_t* out_ns, uint32_t capacity,

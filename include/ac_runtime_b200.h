@@ -377,6 +377,11 @@ AcResult ac_b200_context_synchronize(AcContext* ctx);
  * stay retained until ac_runtime_batch_destroy. */
 AcResult ac_b200_batch_instantiate(AcCommandBatch* batch);
 AcResult ac_b200_batch_replay(AcCommandBatch* batch, AcEvent** out_completion_event);
+/* What the flushes (or the instantiation) of a batch have launched so far: *out_launches counts dispatches that left the host,
+ * several that share a launch as one; *out_in_order those of them that were not allowed to start while the launch in front of
+ * them still ran (the first of a flush, and products whose weights an earlier dispatch of the batch may write: weights are
+ * otherwise requested ahead of time). No counterpart in the reference. */
+AcResult ac_b200_batch_get_launches(const AcCommandBatch* batch, uint32_t* out_launches, uint32_t* out_in_order);
 
 /* Weight codec: ggml block bytes <-> the device region layout the kernels read. Stands in for the reference's CPU
  * repack codec (adapters/llama/ggml-ameva/ggml-ameva-repack.cpp:82-247, ggml-ameva-buffer.cpp:300-330). type is the
