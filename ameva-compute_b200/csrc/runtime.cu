@@ -7,9 +7,11 @@
 // The execution model is the one the reference's OpenCL backend documents (include/ac_runtime.h:614-630): one in-order
 // queue per context (here a CUDA stream), batches that run at flush/submit, host access through write/read/fill only.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -38,9 +40,11 @@ uint64_t now_ns() {
 
 }  // namespace
 
-// GPU start and end times of the replays of a batch, written by a one-thread kernel at either end of its graph: a ring in
-// device memory that get_timing reads on demand. A pair of timed events around the graph took 6 us of every replay (a
-// one-kernel graph alone 2.0 us, with the events 8.2, with the stamps 4.1).
+// GPU start and end times of the replays of a batch, written by a one-thread kernel at either end of its graph into a ring in
+// device memory. A pair of timed events around the graph took 6 us of every replay (a one-kernel graph alone 2.0 us, with the
+// events 8.2, with the stamps 4.1; 6.1 with the ring in host memory). The host copies the ring as a whole: when the time of an
+// event is asked for (the copy answers for all events of replays that have ended by then), and, in stream order, in front of a
+// replay that would write over the times of an event that still exists.
 constexpr uint32_t kStampSlots = 1023;   // (about as many launches as a stream queues before it holds the host up)
 struct StampRing {
     unsigned long long seq;   // replays so far (device side)
@@ -59,6 +63,21 @@ __global__ void stamp_kernel(StampRing* ring, uint32_t end) {
     if (end) ring->seq = n + 1;
 }
 
+// A copy of a ring in pinned host memory, valid once `done` has completed; kept by the events whose times are in it.
+struct StampCopy {
+    AcContext* ctx = nullptr;
+    StampRing* host = nullptr;
+    cudaEvent_t done = nullptr;
+    ~StampCopy();
+};
+// The ring of a replayable batch and the events whose times it holds; lives as long as the batch or one of those events.
+struct Stamps {
+    AcContext* ctx = nullptr;
+    StampRing* ring = nullptr;
+    AcEvent* owner[kStampSlots] = {};
+    ~Stamps();
+};
+
 constexpr size_t kEventPool = 32;   // idle CUDA events a context keeps (creating and destroying one costs about a microsecond)
 
 struct AcContext {
@@ -69,13 +88,16 @@ struct AcContext {
     uint32_t* status_host;  // mapped pinned memory, 4 words
     uint32_t* status_dev;
     uint32_t* workspace;    // kWorkspaceBytes of zeroed device memory for the kernels' cross-CTA flags
-    uint32_t live_buffers, live_kernels, live_events, live_batches;
+    std::atomic<uint32_t> live_buffers, live_kernels, live_events, live_batches;   // (events may be destroyed on any thread)
     uint64_t id;
-    std::mutex event_mutex;                // guards the pools and the rings
+    std::mutex event_mutex;                // guards the pools and rings_used
+    std::mutex stamp_mutex;                // guards the owners of all rings, the stamp fields of events and read_copy
     std::vector<cudaEvent_t> idle_timed, idle_plain;
     StampRing* rings;                      // kStampRings of them
     uint64_t rings_used;                   // bit per ring
     cudaStream_t read_stream;              // reads the stamps beside the context's stream
+    StampRing* read_copy;                  // pinned: where it reads them to
+    cudaEvent_t read_done;
     SideQueues side;        // copy queues beside the stream, created by the first launcher that needs them
     // weight upload (ac_b200_weight_upload): two pinned host chunks and two device chunks, created by the first upload
     void* up_pinned[2];
@@ -106,9 +128,10 @@ struct AcEvent {
     uint32_t magic;
     AcContext* ctx;
     cudaEvent_t start, end;
-    AcCommandBatch* stamped;   // a replay whose times are in slot `slot` of this batch's ring (start is null then)
-    uint32_t slot;
-    uint64_t gpu_ns;           // those times, once read
+    std::shared_ptr<Stamps> stamps;      // a replay whose times are in a ring (start is null then) ...
+    std::shared_ptr<StampCopy> stamped;  // ... or were, and are in this copy; neither: in gpu_ns
+    uint64_t replay;                     // its number in the batch
+    uint64_t gpu_ns;
     uint64_t wall_submit_ns, wall_done_ns;
     bool signaled;
     AcResult result;
@@ -166,9 +189,8 @@ struct AcCommandBatch {
     std::vector<cudaEvent_t> t_after;  // one per dispatch with AC_BATCH_FLAG_DISPATCH_TIMESTAMPS
     cudaEvent_t t_end;
     bool started, completed;
-    StampRing* ring;             // REPLAYABLE: device ring of this batch, or null
+    std::shared_ptr<Stamps> stamps;   // REPLAYABLE: the times of its replays, or null (timed events)
     uint64_t replays;
-    std::vector<AcEvent*> stamped;   // with a ring: the event that owns each slot
 };
 
 namespace {
@@ -321,8 +343,7 @@ AcResult make_event(AcContext* ctx, bool timing, AcEvent** out) {
     e->ctx = ctx;
     e->start = nullptr;
     e->end = nullptr;
-    e->stamped = nullptr;
-    e->slot = 0;
+    e->replay = 0;
     e->gpu_ns = 0;
     e->signaled = false;
     e->result = AC_SUCCESS;
@@ -342,7 +363,14 @@ AcResult make_event(AcContext* ctx, bool timing, AcEvent** out) {
 }
 
 void free_event(AcEvent* e) {
-    if (e->stamped) e->stamped->stamped[e->slot] = nullptr;
+    std::shared_ptr<Stamps> s;   // (let go after the lock)
+    std::shared_ptr<StampCopy> c;
+    {
+        std::lock_guard<std::mutex> lock(e->ctx->stamp_mutex);
+        if (e->stamps) e->stamps->owner[e->replay % kStampSlots] = nullptr;
+        s.swap(e->stamps);
+        c.swap(e->stamped);
+    }
     give_event(e->ctx, e->end, e->start != nullptr);
     give_event(e->ctx, e->start, true);
     e->ctx->live_events--;
@@ -350,31 +378,77 @@ void free_event(AcEvent* e) {
     delete e;
 }
 
-// The stamps of a replay that has completed, copied out of the ring; the event no longer refers to the batch.
-void read_stamps(AcEvent* e) {
-    AcCommandBatch* b = e->stamped;
-    if (!b) return;
-    unsigned long long t[2] = {0, 0};
-    if (cudaMemcpyAsync(t, b->ring->t[e->slot], sizeof(t), cudaMemcpyDeviceToHost, e->ctx->read_stream) == cudaSuccess &&
-        cudaStreamSynchronize(e->ctx->read_stream) == cudaSuccess)
-        e->gpu_ns = t[1] > t[0] ? t[1] - t[0] : 0;
-    else
-        cudaGetLastError();
-    b->stamped[e->slot] = nullptr;
-    e->stamped = nullptr;
-}
-
-StampRing* take_ring(AcContext* ctx) {
+std::shared_ptr<Stamps> take_ring(AcContext* ctx) {
+    std::shared_ptr<Stamps> s = std::make_shared<Stamps>();
+    s->ctx = ctx;
     std::lock_guard<std::mutex> lock(ctx->event_mutex);
     if (!ctx->rings || ctx->rings_used == ~0ull) return nullptr;
     const int i = __builtin_ctzll(~ctx->rings_used);
     ctx->rings_used |= 1ull << i;
-    return ctx->rings + i;
+    s->ring = ctx->rings + i;
+    return s;
 }
-void give_ring(AcContext* ctx, StampRing* r) {
-    if (!r) return;
-    std::lock_guard<std::mutex> lock(ctx->event_mutex);
-    ctx->rings_used &= ~(1ull << (r - ctx->rings));
+
+uint64_t stamp_ns(const StampRing& r, uint64_t replay) {
+    const unsigned long long* t = r.t[replay % kStampSlots];
+    return t[1] > t[0] ? t[1] - t[0] : 0;
+}
+
+// gpu_ns of an event that has completed, from its copy of the ring or the ring itself.
+AcResult read_stamps(AcEvent* e) {
+    AcContext* ctx = e->ctx;
+    std::shared_ptr<Stamps> s;   // (let go after the lock)
+    std::shared_ptr<StampCopy> c;
+    std::lock_guard<std::mutex> lock(ctx->stamp_mutex);
+    if (e->stamped) {
+        const AcResult r = wait_cuda_event(ctx, e->stamped->done, kBlockingWaitNs);
+        if (r != AC_SUCCESS) return r;
+        e->gpu_ns = stamp_ns(*e->stamped->host, e->replay);
+        c.swap(e->stamped);
+    } else if (e->stamps) {
+        if (cudaMemcpyAsync(ctx->read_copy, e->stamps->ring, sizeof(StampRing), cudaMemcpyDeviceToHost, ctx->read_stream) != cudaSuccess ||
+            cudaEventRecord(ctx->read_done, ctx->read_stream) != cudaSuccess) {
+            cudaGetLastError();
+            return AC_ERR_DRIVER_CRASH_OR_LOST;
+        }
+        const AcResult r = wait_cuda_event(ctx, ctx->read_done, kBlockingWaitNs);
+        if (r != AC_SUCCESS) return r;
+        s = e->stamps;
+        // replays whose times the copy holds for sure: all before the one that counted last (it may still be writing), and e's
+        const uint64_t ended = ctx->read_copy->seq ? ctx->read_copy->seq - 1 : 0;
+        for (AcEvent*& o : s->owner) {
+            if (!o || (o != e && o->replay >= ended)) continue;
+            o->gpu_ns = stamp_ns(*ctx->read_copy, o->replay);
+            o->stamps.reset();
+            o = nullptr;
+        }
+    }
+    return AC_SUCCESS;
+}
+
+// The ring's next slot still belongs to an event: a copy of the ring is queued in front of the replay that will write over it,
+// and every event of the ring keeps that copy. (The copy is in stream order: all replays launched so far are complete in it.)
+AcResult save_stamps(AcContext* ctx, Stamps* s) {
+    auto c = std::make_shared<StampCopy>();
+    c->ctx = ctx;
+    c->done = take_event(ctx, false);
+    if (!c->done || cudaHostAlloc((void**)&c->host, sizeof(StampRing), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->host = nullptr;
+        return AC_ERR_OUT_OF_HOST_MEMORY;
+    }
+    if (cudaMemcpyAsync(c->host, s->ring, sizeof(StampRing), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
+        cudaEventRecord(c->done, ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return AC_ERR_DRIVER_CRASH_OR_LOST;
+    }
+    for (AcEvent*& o : s->owner) {
+        if (!o) continue;
+        o->stamped = c;
+        o->stamps.reset();   // (the batch holds the ring: this is not its last reference)
+        o = nullptr;
+    }
+    return AC_SUCCESS;
 }
 
 AcResult validate_metadata(const AcKernelRuntimeMetadata* md) {
@@ -490,6 +564,19 @@ void destroy_batch_events(AcCommandBatch* b) {
 
 }  // namespace
 
+StampCopy::~StampCopy() {
+    if (host) {
+        if (done) wait_cuda_event(ctx, done, kBlockingWaitNs);   // (the copy may still be on its way)
+        cudaFreeHost(host);
+    }
+    give_event(ctx, done, false);
+}
+Stamps::~Stamps() {
+    if (!ring) return;
+    std::lock_guard<std::mutex> lock(ctx->event_mutex);
+    ctx->rings_used &= ~(1ull << (ring - ctx->rings));
+}
+
 extern "C" {
 
 uint32_t ac_runtime_abi_version(void) { return AC_ABI_VERSION; }
@@ -535,7 +622,11 @@ AcResult ac_runtime_context_create(const AcContextDesc* desc, AcContext** out_ct
     memset(c->status_host, 0, 16);
     // without the rings (no memory, no stream) replays are timed with events
     if (cudaStreamCreateWithFlags(&c->read_stream, cudaStreamNonBlocking) != cudaSuccess) c->read_stream = nullptr;
-    if (!c->read_stream || cudaMalloc((void**)&c->rings, kStampRings * sizeof(StampRing)) != cudaSuccess) c->rings = nullptr;
+    if (cudaHostAlloc((void**)&c->read_copy, sizeof(StampRing), cudaHostAllocDefault) != cudaSuccess) c->read_copy = nullptr;
+    if (cudaEventCreateWithFlags(&c->read_done, cudaEventDisableTiming) != cudaSuccess) c->read_done = nullptr;
+    if (!c->read_stream || !c->read_copy || !c->read_done ||
+        cudaMalloc((void**)&c->rings, kStampRings * sizeof(StampRing)) != cudaSuccess)
+        c->rings = nullptr;
     cudaGetLastError();
     {
         std::lock_guard<std::mutex> lock(g_id_mutex);
@@ -569,6 +660,8 @@ AcResult ac_runtime_context_destroy(AcContext* ctx) {
     for (cudaEvent_t e : ctx->idle_timed) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->idle_plain) cudaEventDestroy(e);
     if (ctx->rings) cudaFree(ctx->rings);
+    if (ctx->read_done) cudaEventDestroy(ctx->read_done);
+    if (ctx->read_copy) cudaFreeHost(ctx->read_copy);
     if (ctx->read_stream) cudaStreamDestroy(ctx->read_stream);
     cudaStreamDestroy(ctx->stream);
     cudaFreeHost(ctx->status_host);
@@ -1096,7 +1189,8 @@ AcResult ac_runtime_event_get_timing(AcEvent* event, uint64_t* out_wall_latency_
     if (out_wall_latency_ns) *out_wall_latency_ns = event->wall_done_ns - event->wall_submit_ns;
     if (out_gpu_duration_ns && !event->start) {   // a replay: its stamps
         DeviceGuard g(event->ctx->device);
-        read_stamps(event);
+        const AcResult r = read_stamps(event);
+        if (r != AC_SUCCESS) return fail(event->ctx, r, AMEVA_BACKEND_OP_SYNC);
         *out_gpu_duration_ns = event->gpu_ns;
     }
     if (out_gpu_duration_ns && event->start) {
@@ -1145,7 +1239,6 @@ AcResult ac_runtime_batch_begin_ex(AcContext* context, const AcBatchDesc* desc, 
     b->t_begin = b->t_end = nullptr;
     b->started = b->completed = false;
     b->exec = nullptr;
-    b->ring = nullptr;
     b->replays = 0;
     b->records.reserve(desc->max_dispatches < 256 ? desc->max_dispatches : 256);
     context->live_batches++;
@@ -1297,25 +1390,21 @@ AcResult ac_b200_batch_instantiate(AcCommandBatch* batch) {
     if (batch->flags & (AC_BATCH_FLAG_TIMESTAMPS | AC_BATCH_FLAG_DISPATCH_TIMESTAMPS)) return AC_ERR_FEATURE_NOT_SUPPORTED;
     AcContext* ctx = batch->ctx;
     DeviceGuard g(ctx->device);
-    batch->ring = take_ring(ctx);
-    if (batch->ring && cudaMemsetAsync(batch->ring, 0, sizeof(StampRing), ctx->stream) != cudaSuccess) {
+    batch->stamps = take_ring(ctx);
+    if (batch->stamps && cudaMemsetAsync(batch->stamps->ring, 0, sizeof(StampRing), ctx->stream) != cudaSuccess) {
         cudaGetLastError();
-        give_ring(ctx, batch->ring);
-        batch->ring = nullptr;
+        batch->stamps.reset();
     }
-    if (batch->ring) batch->stamped.assign(kStampSlots, nullptr);
-    auto drop_ring = [&]() {
-        give_ring(ctx, batch->ring);
-        batch->ring = nullptr;
-    };
+    auto drop_ring = [&]() { batch->stamps.reset(); };
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         drop_ring();
         return fail(ctx, AC_ERR_FEATURE_NOT_SUPPORTED, AMEVA_BACKEND_OP_DISPATCH);
     }
-    if (batch->ring) amv::launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, ctx->stream, batch->ring, 0u);
+    StampRing* ring = batch->stamps ? batch->stamps->ring : nullptr;
+    if (ring) amv::launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, ctx->stream, ring, 0u);
     const AcResult r = flush_batch(batch, true);
-    if (batch->ring) amv::launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, ctx->stream, batch->ring, 1u);
+    if (ring) amv::launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, ctx->stream, ring, 1u);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     if (r != AC_SUCCESS || e != cudaSuccess || !graph) {
@@ -1348,13 +1437,13 @@ AcResult ac_b200_batch_replay(AcCommandBatch* batch, AcEvent** out_completion_ev
     AcContext* ctx = batch->ctx;
     DeviceGuard g(ctx->device);
     AcEvent* ev = nullptr;
-    const uint32_t slot = (uint32_t)(batch->replays % kStampSlots);
-    if (batch->ring && batch->stamped[slot]) {   // the slot's last owner is still around: its times before they are overwritten
-        AcEvent* owner = batch->stamped[slot];
-        cudaEventSynchronize(owner->end);
-        read_stamps(owner);
+    AcResult r = AC_SUCCESS;
+    if (Stamps* s = batch->stamps.get()) {
+        std::lock_guard<std::mutex> lock(ctx->stamp_mutex);
+        if (s->owner[batch->replays % kStampSlots]) r = save_stamps(ctx, s);
     }
-    AcResult r = make_event(ctx, batch->ring == nullptr, &ev);
+    if (r != AC_SUCCESS) return fail(ctx, r, AMEVA_BACKEND_OP_DISPATCH);
+    r = make_event(ctx, batch->stamps == nullptr, &ev);
     if (r != AC_SUCCESS) return r;
     if (ev->start) cudaEventRecord(ev->start, ctx->stream);
     if (cudaGraphLaunch(batch->exec, ctx->stream) != cudaSuccess) {
@@ -1363,11 +1452,11 @@ AcResult ac_b200_batch_replay(AcCommandBatch* batch, AcEvent** out_completion_ev
         return fail(ctx, AC_ERR_DRIVER_CRASH_OR_LOST, AMEVA_BACKEND_OP_DISPATCH);
     }
     cudaEventRecord(ev->end, ctx->stream);
-    if (batch->ring) {
-        ev->stamped = batch;
-        ev->slot = slot;
-        batch->stamped[slot] = ev;
-        batch->replays++;
+    if (batch->stamps) {
+        std::lock_guard<std::mutex> lock(ctx->stamp_mutex);
+        ev->stamps = batch->stamps;
+        ev->replay = batch->replays++;
+        batch->stamps->owner[ev->replay % kStampSlots] = ev;
     }
     batch->started = true;   // work of this batch may be in flight: destroy synchronizes
     batch->stats.flushes++;
@@ -1385,10 +1474,7 @@ void ac_runtime_batch_destroy(AcCommandBatch* batch) {
     AcContext* ctx = batch->ctx;
     DeviceGuard g(ctx->device);
     if (batch->started && !batch->completed) cudaStreamSynchronize(ctx->stream);  // launched work may still run
-    for (AcEvent* e : batch->stamped)
-        if (e) read_stamps(e);
     if (batch->exec) cudaGraphExecDestroy(batch->exec);
-    give_ring(ctx, batch->ring);
     release_records(batch);
     destroy_batch_events(batch);
     ctx->live_batches--;

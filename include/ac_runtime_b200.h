@@ -374,7 +374,13 @@ AcResult ac_b200_context_synchronize(AcContext* ctx);
  * capture, so argument checks and errors are those of a normal flush, and nothing executes yet. ac_b200_batch_replay
  * enqueues the graph on the context's stream (any number of times, in stream order with everything else) and returns a
  * completion event with GPU timing, or blocks when out_completion_event is NULL. The buffers and kernels of the batch
- * stay retained until ac_runtime_batch_destroy. */
+ * stay retained until ac_runtime_batch_destroy.
+ * The GPU duration of a replay is the time from the start of its first dispatch to the end of its last one on the device,
+ * taken inside the graph (launch gaps in front of it do not count); ac_runtime_event_get_timing fetches it from the device
+ * the first time it is asked for, together with those of all other replays of the batch that have ended by then. Events may
+ * be waited for, timed and destroyed on any thread, while the batch is replayed, and after it is destroyed. With more than 64
+ * replayable batches at a time (a batch counts until its events are timed or destroyed) the others are timed from the
+ * stream, launch gaps included. */
 AcResult ac_b200_batch_instantiate(AcCommandBatch* batch);
 AcResult ac_b200_batch_replay(AcCommandBatch* batch, AcEvent** out_completion_event);
 /* What the flushes (or the instantiation) of a batch have launched so far: *out_launches counts dispatches that left the host,

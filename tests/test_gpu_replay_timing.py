@@ -71,3 +71,44 @@ def test_more_replayable_batches_than_rings():
     again.destroy()
     x.destroy()
     ctx.destroy()
+
+
+def test_events_timed_and_destroyed_on_another_thread():
+    """One thread replays and destroys the batch, another waits for the events, asks for their times and destroys them."""
+    import queue
+    import threading
+    ctx = rt.init()
+    n = 1 << 14
+    x = ctx.buffer(data=np.ones(n, np.float32))
+    todo, times, errors = queue.SimpleQueue(), [], []
+
+    def drain():
+        try:
+            while (ev := todo.get()) is not None:
+                ev.wait()
+                if len(times) % 3:          # (some are destroyed without a look at their time)
+                    times.append(ev.gpu_duration_us())
+                else:
+                    times.append(1.0)
+                ev.destroy()
+        except Exception as e:              # noqa: BLE001 (reported by the main thread)
+            errors.append(e)
+
+    worker = threading.Thread(target=drain)
+    worker.start()
+    replays = 0
+    for _ in range(3):
+        batch = ctx.batch(4)
+        for _ in range(2):
+            batch.dispatch(ctx.kernel("ameva_add_f32"), [x, x, x], [1, n, 1])
+        batch.instantiate()
+        for _ in range(1500):
+            todo.put(batch.replay())
+            replays += 1
+        batch.destroy()                     # the worker still holds events of it
+    todo.put(None)
+    worker.join(60)
+    assert not worker.is_alive() and not errors
+    assert len(times) == replays and all(0 < t < 1e6 for t in times)
+    x.destroy()
+    ctx.destroy()
