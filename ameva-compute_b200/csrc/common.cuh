@@ -29,12 +29,13 @@ struct SideQueues {
 };
 
 // The stream of a launch. in_order: not before everything in front of it has completed, i.e. without the programmatic launch
-// attribute (see launch_pdl); for a kernel whose early reads (BindingUse) something still running may write.
+// attribute (see launch_pdl); for a kernel whose early reads (BindingUse) something still running may write. dry: all checks
+// of the launcher, nothing launched (the products, quantizes and the I2_S kernels, which fuse.cu looks past).
 struct LaunchStream {
     cudaStream_t s;
-    bool in_order;
+    bool in_order, dry;
     LaunchStream() = default;
-    LaunchStream(cudaStream_t stream) : s(stream), in_order(false) {}
+    LaunchStream(cudaStream_t stream) : s(stream), in_order(false), dry(false) {}
     operator cudaStream_t() const { return s; }
 };
 
@@ -170,6 +171,7 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, LaunchStream stream,
                               Args&&... args) {
+    if (stream.dry) return cudaSuccess;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;

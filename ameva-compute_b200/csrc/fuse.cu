@@ -2,7 +2,8 @@
 // recorded in between touches any range it binds (reads of the same range count as touching: the check knows no directions),
 // so running it early changes neither what it reads nor what the others read. Only kernels whose effects are confined to
 // their bindings are looked past (the output exchange between ranks and kernels a host has registered are not). A form is
-// taken only when every member passes the checks of its own launcher; anything else is launched by itself, errors included.
+// taken only when every member, and every dispatch it is moved past, passes the checks of its own launcher; anything else is
+// launched by itself, errors included: when a dispatch is refused, nothing recorded behind it has run.
 #include "fuse.h"
 
 namespace amv {
@@ -59,10 +60,16 @@ bool confined(const FuseOp& op) {
 }
 
 // May ops[j] run together with ops[i], i < j? Members of the group being formed (marked in `member`) are checked by the caller.
-bool can_hoist(const FuseOp* ops, uint32_t i, uint32_t j, uint64_t member) {
+bool can_hoist(FuseOp* ops, uint32_t i, uint32_t j, uint64_t member) {
     for (uint32_t k = i + 1; k < j; ++k) {
         if (ops[k].done || (member >> (k - i) & 1u)) continue;
         if (!confined(ops[k]) || !disjoint(ops[k].args, ops[j].args)) return false;
+        if (ops[k].checks == FuseOp::UNKNOWN) {
+            LaunchArgs a = ops[k].args;
+            a.stream.dry = true;
+            ops[k].checks = ops[k].entry->launch(a) == AC_SUCCESS ? FuseOp::PASSES : FuseOp::REFUSED;
+        }
+        if (ops[k].checks == FuseOp::REFUSED) return false;
     }
     return true;
 }

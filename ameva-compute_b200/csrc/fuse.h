@@ -11,6 +11,7 @@ struct FuseOp {
     const KernelEntry* entry;
     LaunchArgs args;
     bool done;   // launched, alone or as part of a fused form
+    enum { UNKNOWN, PASSES, REFUSED } checks;   // of its launcher, where a later operation is to run before it
 };
 
 // Launches ops[i] together with the later operations that can join it, and marks all of them done.

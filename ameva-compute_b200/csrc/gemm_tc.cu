@@ -1523,6 +1523,7 @@ static AcResult launch_wide(const LaunchArgs& a, EncodeTiledFn enc, const void* 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = a.stream.in_order ? 1 : 2;
+    if (a.stream.dry) return AC_SUCCESS;
     if (cudaLaunchKernelEx(&cfg, gemm_tc_wide_kernel<TYPE>, act_map, raw_map, scale_map, out_maps, p) != cudaSuccess) {
         cudaGetLastError();
         return AC_ERR_INVALID_WORK_GROUP_SIZE;
@@ -1736,6 +1737,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
                                 : (pair ? ensure_dynamic_smem<gemm_tc_kernel<TYPE, true, false>>((int)kSmemLimit)
                                         : ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, false>>((int)kSmemLimit));
     if (!fits) return AC_ERR_INVALID_WORK_GROUP_SIZE;
+    if (a.stream.dry) return AC_SUCCESS;
     cudaError_t e;
     if (p.splits)
         e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<TYPE, true, false, true>, act_map, raw_map, scale_map, out_maps, p);

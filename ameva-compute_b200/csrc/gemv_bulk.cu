@@ -571,6 +571,7 @@ static AcResult launch_one(const LaunchArgs& a, Params& p, bool whole_rows = fal
     const uint32_t NB = p.group_warps ? (p.N + p.group_warps * R - 1) / (p.group_warps * R) : (p.N + RB - 1) / RB;
     const uint32_t sms = a.sm_count > 0 ? (uint32_t)a.sm_count : 148u;
     const uint32_t grid = NB < sms ? NB : sms;
+    if (a.stream.dry) return AC_SUCCESS;
     if (p.diag & 4u) gemv_bulk_kernel<TYPE, M, R><<<grid, kThreads, smem_bytes, a.stream>>>(p);
     else launch_pdl(gemv_bulk_kernel<TYPE, M, R>, dim3(grid), dim3(kThreads), smem_bytes, a.stream, p);
     return check_launch();

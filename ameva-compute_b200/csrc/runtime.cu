@@ -521,7 +521,7 @@ AcResult flush_batch(AcCommandBatch* b, bool capture = false) {
         const BatchRecord& r = b->records[first + k];
         void* ptrs[16];
         for (uint32_t i = 0; i < r.nbind; ++i) ptrs[i] = (char*)r.buf[i]->dptr + r.offset[i];
-        ops[k] = {r.kernel->entry, launch_args(ctx, r.nbind, ptrs, r.range, r.push, r.grid), false};
+        ops[k] = {r.kernel->entry, launch_args(ctx, r.nbind, ptrs, r.range, r.push, r.grid), false, FuseOp::UNKNOWN};
         // Weights are read before the kernels in front have completed (see launch_pdl): not where one of them may write them.
         // The first launch waits for all that other batches have in flight.
         const BindingUse use = binding_use(r.kernel->entry, r.push);

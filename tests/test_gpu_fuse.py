@@ -186,3 +186,31 @@ def test_byte_decoded_products_with_the_add_behind_them(ctx, name, unit, rec, ac
     for a, b, out in (("o", "e", "r"), ("e", "o", "r"), ("o", "e", "e"), ("o", "e", "o"), ("o", "o", "r")):
         check(ctx, bufs, [gemv, ("ameva_add_f32", [a, b, out], [M, N, M], ONE)])
     check(ctx, bufs, [gemv, ("ameva_add_f32", ["o", "e", "r"], [M, N, 1], ONE)])      # one row of e over all
+
+
+@pytest.mark.parametrize("bad", ["gemv", "gemm", "mmv", "mmtc", "quant"])
+def test_nothing_behind_a_refused_dispatch_has_run(ctx, bad):
+    """A dispatch with arguments its launcher refuses, between two quantizes of the same rows that would otherwise leave in one
+    launch: the batch fails there, what is in front has run and what is behind has not."""
+    M, K, N = 1, 512, 64
+    rng = np.random.default_rng(1)
+    bufs = {"x": rng.standard_normal(M * K).astype(np.float32)}
+    ops = [i2_s(f"p{j}", "x", M, N, K, rng, bufs, f"o{j}")[0] for j in (0, 1)]
+    for n, size in (("w", N * K), ("s", N * K), ("aq", M * K), ("ad", M * K), ("ah", 2 * M * K), ("ae", 4 * M), ("o", 4 * M * N)):
+        bufs[n] = np.zeros(size, np.uint8)
+    wrong = {"gemv": ("bitnet_gemv_i2_s_l32w1", ["w", "aq", "o", "ad"], [K - 64, N, fbits(0.02), 0, M, N]),       # K % 128
+             "gemm": ("bitnet_gemm_i2_s", ["w", "aq", "o", "ad"], [M, 16 * N, K, 16 * N, fbits(0.02)]),            # outputs too small
+             "mmv": ("ameva_mmvq_q8_0", ["w", "s", "aq", "ad", "o"], [M, N, K - 1, N]),
+             "mmtc": ("ameva_mmtc_q8_0", ["w", "s", "ah", "o", "ae"], [M, N, K, N - 1, 0]),                        # rows closer than N
+             "quant": ("ameva_quant_a8", ["o", "aq", "ad"], [M, K, K, 7])}[bad] + (ONE,)
+    held = {n: ctx.buffer(data=a) for n, a in bufs.items()}
+    batch = ctx.batch(4)
+    for name, binds, push, grid in [ops[0], wrong, ops[1]]:
+        batch.dispatch(ctx.kernel(name), [held[b] for b in binds], push, grid)
+    with pytest.raises(rt.AmevaComputeError):
+        batch.submit()
+    batch.destroy()
+    ctx.synchronize()
+    assert any(held["p0q"].read(np.uint8)) and not any(held["p1q"].read(np.uint8)) and not any(held["p1y"].read(np.uint8))
+    for b in held.values():
+        b.destroy()
