@@ -824,9 +824,9 @@ AcResult launch_gemv_f16(const LaunchArgs& a) {
 // The keys are split over the grid (flash decoding): CTA (z, kv head, query position) walks keys [z * split, (z + 1) *
 // split) for all G = n_head / n_head_kv heads of its group, so every K and V byte is read once per query position. Each
 // warp takes 16 keys at a time through tiles of its own in shared memory, an online softmax per head; the warps of a CTA are
-// merged in shared memory with the usual maximum / sum rescaling, the CTAs of a row by the one that finishes last
-// (ameva_fa_combine's job in the reference). The work is bound by reading the KV cache from HBM: n_kv * n_head_kv * (D + DV)
-// * 2 bytes per query position.
+// merged in shared memory with the usual maximum / sum rescaling, the splits by a second kernel (ameva_fa_combine's job in the
+// reference, flash_combine_kernel here). The work is bound by reading the KV cache from HBM: n_kv * n_head_kv * (D + DV) * 2
+// bytes per query position.
 // n_q > 1, D <= 128: up to sixteen rows of positions x heads 16 / G positions per CTA (flash_tile_kernel below), more the
 // tensor-core kernel of flash_tc.cu; D = 256: one position per CTA.
 // Not taken: ALiBi (max_bias != 0), f32 or quantized K / V, G > 8, D != DV: refused with AC_ERR_FEATURE_NOT_SUPPORTED
@@ -851,15 +851,11 @@ constexpr size_t flash_tile_smem_bytes() {   // the kernel for prompts merges si
     constexpr size_t tiles = 2 * sizeof(__half) * kFaWarps * 32 * D, merge = sizeof(float) * kFaWarps * 16 * (D + 2);
     return tiles > merge ? tiles : merge;
 }
-// The one-position kernel: a CTA per SM (D = 128: 12 warps with four tiles of 16 keys each, two of K and two of V: 192 KB on
-// their way to an SM that consumes 45 KB per microsecond at the full HBM rate).
+// The one-position kernel, W warps with four tiles of 16 keys each (two of K, two of V).
 constexpr uint32_t kFdKeys = 16, kFdStages = 2;
-template <int D>
-constexpr int fd_warps() { return D == 64 ? 16 : D == 128 ? 12 : 6; }
-template <int D>
+template <int D, int W>
 constexpr size_t flash_smem_bytes() {
-    constexpr size_t tiles = 2 * kFdStages * sizeof(__half) * fd_warps<D>() * kFdKeys * D,
-                     merge = sizeof(float) * fd_warps<D>() * kFaHeads * (D + 2);
+    constexpr size_t tiles = 2 * kFdStages * sizeof(__half) * W * kFdKeys * D, merge = sizeof(float) * W * kFaHeads * (D + 4);
     return tiles > merge ? tiles : merge;
 }
 
@@ -908,23 +904,20 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 // the second product, P V, whose B fragments are the staged V rows through ldmatrix.trans. Q and the probabilities
 // are rounded to f16 (ggml's CPU kernel rounds Q to f16 as well and accumulates V in f16; here accumulation is fp32).
 //
-// Blocks of 16 keys: a short context then still gives every warp of the chip a block (32 heads x 2048 keys: 4096 blocks on 1776
-// warps; blocks of 32 left a third of the warps with half the work of the others). K(b) .. V(b + 1) are on their way when block
-// b starts; a tile is requested again as soon as it has been read.
-// counters: one zero word per (KV head, position), left zero; nullptr: the partial results are merged by the kernel below.
-template <int D>
-__global__ void __launch_bounds__(fd_warps<D>() * 32, 1) flash_decode_kernel(const float* __restrict__ q, const __half* __restrict__ k,
+// K(b) .. V(b + 1) are on their way when block b starts; a tile is requested again as soon as it has been read.
+template <int D, int W>
+__global__ void __launch_bounds__(W * 32, D == 64 && W == 8 ? 2 : 1) flash_decode_kernel(const float* __restrict__ q, const __half* __restrict__ k,
                                                                           const __half* __restrict__ v,
                                                                           const __half* __restrict__ mask, float* __restrict__ o,
-                                                                          float* part, const FlashArgs pc,
-                                                                          uint32_t n_splits, uint32_t* counters) {
+                                                                          float* __restrict__ part, const FlashArgs pc,
+                                                                          uint32_t n_splits) {
     constexpr int KS = D / 16;                // k-steps of the score product
     constexpr int NT = D / 8;                 // n-tiles of the output
     constexpr uint32_t P = D / 8;             // 16-byte pieces per K or V row
-    constexpr uint32_t W = fd_warps<D>(), TILE = kFdKeys * D;   // (halves)
+    constexpr uint32_t TILE = kFdKeys * D;    // (halves)
     extern __shared__ __align__(16) uint8_t fa_smem[];
-    float (*s_acc)[kFaHeads][D + 2] = reinterpret_cast<float (*)[kFaHeads][D + 2]>(fa_smem);   // per warp: D sums, max, sum
-    __shared__ uint32_t s_last;
+    float (*s_acc)[kFaHeads][D + 4] = reinterpret_cast<float (*)[kFaHeads][D + 4]>(fa_smem);   // per warp: D sums, sum, max of all
+    __shared__ float s_max[W][kFaHeads];
     pdl_trigger();
     pdl_wait();
     const uint32_t z = blockIdx.x, hkv = blockIdx.y, iq1 = blockIdx.z;
@@ -1063,107 +1056,51 @@ __global__ void __launch_bounds__(fd_warps<D>() * 32, 1) flash_decode_kernel(con
         request_v(st, ahead);
     }
     cp_async_wait_group<0>();
-    __syncthreads();   // every warp is done with its tiles: the memory is reused for the merge
-    // merge the warps of the CTA: thread (g, t4) holds columns 8 nt + 2 t4 + {0, 1} of head g
+    // the warps' maxima first, so that every thread brings its own columns (8 nt + 2 t4 + {0, 1} of head g) to the common one
+    if (t4 == 0) s_max[warp][g] = m_run;
+    __syncthreads();   // (every warp is done with its tiles, too: the memory is reused)
     if (head) {
+        float mx = ninf;
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            s_acc[warp][g][8 * nt + 2 * t4] = oc[nt][0];
-            s_acc[warp][g][8 * nt + 2 * t4 + 1] = oc[nt][1];
-        }
+        for (uint32_t w = 0; w < W; ++w) mx = fmaxf(mx, s_max[w][g]);
+        const float f = m_run == ninf ? 0.0f : expf(m_run - mx);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+            *reinterpret_cast<float2*>(&s_acc[warp][g][8 * nt + 2 * t4]) = make_float2(oc[nt][0] * f, oc[nt][1] * f);
         if (t4 == 0) {
-            s_acc[warp][g][D] = m_run;
-            s_acc[warp][g][D + 1] = l_run;
+            s_acc[warp][g][D] = l_run * f;
+            s_acc[warp][g][D + 1] = mx;
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < G * D; i += W * 32u) {
-        const uint32_t gg = i / D, d = i - gg * D;
-        float mx = ninf;
-#pragma unroll
-        for (uint32_t w = 0; w < W; ++w) mx = fmaxf(mx, s_acc[w][gg][D]);
-        float num = 0.0f, den = 0.0f;
+    for (uint32_t i = threadIdx.x; i < G * (D / 4u); i += W * 32u) {
+        const uint32_t gg = i / (D / 4u), d = 4u * (i - gg * (D / 4u));
+        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+        float den = 0.0f;
 #pragma unroll
         for (uint32_t w = 0; w < W; ++w) {
-            const float mw = s_acc[w][gg][D];
-            const float f = mw == ninf ? 0.0f : expf(mw - mx);
-            num = fmaf(s_acc[w][gg][d], f, num);
-            den = fmaf(s_acc[w][gg][D + 1], f, den);
+            const float4 x = *reinterpret_cast<const float4*>(&s_acc[w][gg][d]);
+            num.x += x.x;
+            num.y += x.y;
+            num.z += x.z;
+            num.w += x.w;
+            den += s_acc[w][gg][D];
         }
         const uint64_t r = (uint64_t)iq1 * pc.n_head + h0 + gg;   // output row
         if (n_splits == 1u) {
-            o[pc.o_off + r * D + d] = num / den;
+            float* dst = o + pc.o_off + r * D + d;
+            dst[0] = num.x / den;
+            dst[1] = num.y / den;
+            dst[2] = num.z / den;
+            dst[3] = num.w / den;
         } else {
             float* pr = part + pc.part_off + ((uint64_t)z * pc.n_q * pc.n_head + r) * (D + 4);   // max, sum, 2 unused, D sums
-            pr[4 + d] = num;
+            *reinterpret_cast<float4*>(pr + 4 + d) = num;
             if (d == 0) {
-                pr[0] = mx;
+                pr[0] = s_acc[0][gg][D + 1];
                 pr[1] = den;
             }
         }
-    }
-    if (n_splits == 1u || counters == nullptr) return;
-    // the CTA that finishes last merges the splits of its rows
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t* c = counters + iq1 * pc.n_head_kv + hkv;
-        const bool last = atomicAdd(c, 1u) == n_splits - 1u;
-        if (last) *c = 0u;   // as the next launch expects it
-        s_last = last;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    float* s_f = reinterpret_cast<float*>(fa_smem);              // [G][n_splits]: exp(m_z - max)
-    float* s_den = s_f + kFaHeads * kFaMaxSplits;                // [G]
-    float4* s_part = reinterpret_cast<float4*>(s_den + kFaHeads);   // [groups of splits][G * D / 4]
-    const float* first = part + pc.part_off + ((uint64_t)iq1 * pc.n_head + h0) * (D + 4);
-    const uint64_t zs = (uint64_t)pc.n_q * pc.n_head * (D + 4);   // floats between two splits of a row
-    for (uint32_t gg = warp; gg < G; gg += W) {
-        float mx = ninf, den = 0.0f;
-        for (uint32_t zz = lane; zz < n_splits; zz += 32u) mx = fmaxf(mx, __ldcg(first + zz * zs + gg * (D + 4)));
-        mx = warp_max(mx);
-        for (uint32_t zz = lane; zz < n_splits; zz += 32u) {
-            const float2 ml = __ldcg(reinterpret_cast<const float2*>(first + zz * zs + gg * (D + 4)));
-            const float f = ml.x == ninf ? 0.0f : expf(ml.x - mx);
-            s_f[gg * n_splits + zz] = f;
-            den = fmaf(ml.y, f, den);
-        }
-        den = warp_sum(den);
-        if (lane == 0) s_den[gg] = den;
-    }
-    __syncthreads();
-    const uint32_t cols = G * (D / 4), groups = W * 32u / cols ? W * 32u / cols : 1u;
-    for (uint32_t i = threadIdx.x; i < groups * cols; i += W * 32u) {
-        const uint32_t grp = i / cols, col = i - grp * cols, gg = col / (D / 4), c4 = col - gg * (D / 4);
-        const float* src = first + gg * (D + 4) + 4 + 4u * c4;
-        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (uint32_t zz = grp; zz < n_splits; zz += groups) {
-            const float4 xx = __ldcg(reinterpret_cast<const float4*>(src + zz * zs));
-            const float f = s_f[gg * n_splits + zz];
-            num.x = fmaf(xx.x, f, num.x);
-            num.y = fmaf(xx.y, f, num.y);
-            num.z = fmaf(xx.z, f, num.z);
-            num.w = fmaf(xx.w, f, num.w);
-        }
-        s_part[i] = num;
-    }
-    __syncthreads();
-    for (uint32_t col = threadIdx.x; col < cols; col += W * 32u) {
-        const uint32_t gg = col / (D / 4), c4 = col - gg * (D / 4);
-        float4 num = s_part[col];
-        for (uint32_t grp = 1; grp < groups; ++grp) {
-            const float4 xx = s_part[grp * cols + col];
-            num.x += xx.x;
-            num.y += xx.y;
-            num.z += xx.z;
-            num.w += xx.w;
-        }
-        const float den = s_den[gg];
-        *reinterpret_cast<float4*>(o + pc.o_off + ((uint64_t)iq1 * pc.n_head + h0 + gg) * D + 4u * c4) =
-            make_float4(num.x / den, num.y / den, num.z / den, num.w / den);
     }
 }
 
@@ -1444,15 +1381,38 @@ static bool launch_flash_tile_d(const LaunchArgs& a, const FlashArgs& pc, uint32
     return true;
 }
 
-template <int D>
-static bool launch_flash_d(const LaunchArgs& a, const FlashArgs& pc, uint32_t n_splits, uint32_t* counters) {
-    constexpr size_t smem = flash_smem_bytes<D>();
-    static_assert(smem >= sizeof(float) * (kFaHeads * kFaMaxSplits + kFaHeads + 4 * fd_warps<D>() * 32 + kFaHeads * D), "the merge of the splits");
-    if (!ensure_dynamic_smem<flash_decode_kernel<D>>((int)smem)) return false;
-    const dim3 grid(n_splits, pc.n_head_kv, pc.n_q), block(fd_warps<D>() * 32);
-    launch_pdl(flash_decode_kernel<D>, grid, block, smem, a.stream, (const float*)a.ptr[0], (const __half*)a.ptr[1],
-               (const __half*)a.ptr[2], (const __half*)a.ptr[3], (float*)a.ptr[4], (float*)a.ptr[5], pc, n_splits, counters);
+template <int D, int W>
+static bool launch_flash_d(const LaunchArgs& a, const FlashArgs& pc, uint32_t n_splits) {
+    constexpr size_t smem = flash_smem_bytes<D, W>();
+    if (!ensure_dynamic_smem<flash_decode_kernel<D, W>>((int)smem)) return false;
+    const dim3 grid(n_splits, pc.n_head_kv, pc.n_q), block(W * 32);
+    launch_pdl(flash_decode_kernel<D, W>, grid, block, smem, a.stream, (const float*)a.ptr[0], (const __half*)a.ptr[1],
+               (const __half*)a.ptr[2], (const __half*)a.ptr[3], (float*)a.ptr[4], (float*)a.ptr[5], pc, n_splits);
     return true;
+}
+
+// The one-position kernel's form. Measured with caches in rotation and a quantize behind each launch, us per pair; in brackets
+// the kernel of 4 warps x 32 keys that it replaced:
+//   warps  D 64: 8 (two CTAs per SM), D 128: 8, D 256: 4; D <= 128 from 1537 keys on 16 / 12, whose larger CTAs keep more
+//          bytes on their way: 8 KV heads of 128, 32768 keys 32.0 against 34.5 with 8 warps (36.5), 2048 keys 10.0 / 10.4
+//          (10.9), 4096 keys 13.6 / 13.1 (14.6); 1000 keys of one head 9.6 / 9.0 (10.2)
+//   split  at least 64 keys each, or 128 from 1537 keys on, where there are many (1 KV head of 128, 8 warps: 1000 keys 9.0 /
+//          9.4 with 128 (10.2); 4096 keys 11.7 / 11.3 with 128 (12.5))
+//   none   up to one block of 16 keys per warp (D 64, 256: two): 2 KV heads of 64, 256 keys 5.8 against 6.9 in four parts (8.1);
+//          8 of 128, 128 keys 6.4, in two parts of four warps 7.9 (6.7), 256 keys 8.1, in four parts 7.9 (9.3)
+// Splits merged by the CTA that finishes last, instead of a second kernel, cost more at every size, since one CTA then reads
+// all of them: 1 KV head of 256, 4096 keys 51.8 against 15.5, 8 of 128, 4096 keys 15.8 against 13.0.
+struct FdForm {
+    uint32_t wide, per_sm, min_keys, one_keys;
+};
+static FdForm fd_form(uint32_t D, uint32_t n_kv) {
+    const bool many = n_kv > 1536u;
+    FdForm f;
+    f.wide = D <= 128u && many;
+    f.per_sm = D == 64u && !many ? 2u : 1u;
+    f.min_keys = many ? 128u : 64u;
+    f.one_keys = D == 64u ? 256u : 128u;
+    return f;
 }
 
 // ameva_flash_attn: bindings 0 q f32, 1 k f16, 2 v f16, 3 mask f16 (any range when has_mask = 0), 4 dst f32,
@@ -1479,8 +1439,7 @@ AcResult launch_flash_attn(const LaunchArgs& a) {
                                                 pc.m_s1, pc.m_s2, 0u) * 2u) ||
         a.range[4] < ((uint64_t)pc.o_off + rows * pc.D) * 4u)
         return AC_ERR_INVALID_BUFFER_SIZE;
-    // key splits: one wave of CTAs (as many as are resident at once), at least 128 keys (one block of 32 per warp) each,
-    // as many as the scratch holds
+    // key splits: one wave of CTAs (as many as are resident at once), as many as the scratch holds
     const uint32_t sms = a.sm_count > 0 ? (uint32_t)a.sm_count : 148u;
     // more than sixteen rows of positions x heads: the tensor-core kernel, 128 / G positions per CTA (flash_tc.cu); it reads
     // K and V through tensor maps, so strides that no map expresses stay on the kernels here
@@ -1493,17 +1452,15 @@ AcResult launch_flash_attn(const LaunchArgs& a) {
     const uint64_t ctas = (uint64_t)pc.n_head_kv * q_tiles;
     if (q_tiles > 65535u) return AC_ERR_INVALID_WORK_ITEM_DIMS;
     const size_t smem = pc.D == 64u ? flash_tile_smem_bytes<64>() : flash_tile_smem_bytes<128>();
-    uint32_t per_sm = prompt ? kFlashTcPerSm : tile ? (uint32_t)((227u * 1024u) / (smem + 1024u)) : 1u;
+    const FdForm fd = fd_form(pc.D, pc.n_kv);   // (neither prompt nor tile)
+    uint32_t per_sm = prompt ? kFlashTcPerSm : tile ? (uint32_t)((227u * 1024u) / (smem + 1024u)) : fd.per_sm;
     if (per_sm > 4u) per_sm = 4u;
-    // one position: a block of keys for every warp of a CTA before the keys are split further, and no split at all (no merge)
-    // up to two blocks (14 heads on 2 KV heads of 64, 333 keys: a layer takes 35.1 us in one part, 36.9 us in two; 20 heads on
-    // 5 of 128, 777 keys: 48.1 us in five parts, 51.3 us in three)
-    const uint32_t fd_keys = kFdKeys * (pc.D == 64u ? fd_warps<64>() : pc.D == 128u ? fd_warps<128>() : fd_warps<256>());
     uint32_t n_splits = (uint32_t)(((uint64_t)per_sm * sms) / ctas);
-    const uint32_t block = prompt ? kFlashTcKeys : tile ? 32u : kFdKeys, min_keys = prompt ? 4u * kFlashTcKeys : tile ? 128u : fd_keys;
+    const uint32_t block = prompt ? kFlashTcKeys : tile ? 32u : kFdKeys;
+    const uint32_t min_keys = prompt ? 4u * kFlashTcKeys : tile ? 128u : fd.min_keys;   // (tile: a block of 32 per warp)
     const uint32_t max_by_keys = (pc.n_kv + min_keys - 1u) / min_keys;
     if (n_splits > max_by_keys) n_splits = max_by_keys;
-    if (!prompt && !tile && pc.n_kv <= 2u * fd_keys) n_splits = 1u;
+    if (!prompt && !tile && pc.n_kv <= fd.one_keys) n_splits = 1u;
     const uint64_t per_split = rows * (pc.D + 4u) * 4u;
     const uint64_t room = a.range[5] > (uint64_t)pc.part_off * 4u ? a.range[5] - (uint64_t)pc.part_off * 4u : 0u;
     if ((uint64_t)n_splits * per_split > room) n_splits = (uint32_t)(room / per_split);
@@ -1513,15 +1470,15 @@ AcResult launch_flash_attn(const LaunchArgs& a) {
     if (n_splits > kFaMaxSplits) n_splits = kFaMaxSplits;
     pc.split_keys = ((pc.n_kv + n_splits - 1u) / n_splits + block - 1u) & ~(block - 1u);
     n_splits = (pc.n_kv + pc.split_keys - 1u) / pc.split_keys;
-    uint32_t* counters = !prompt && !tile && a.workspace && (uint64_t)pc.n_head_kv * pc.n_q * 4u <= a.workspace_bytes ? a.workspace : nullptr;
     const bool fits = prompt ? launch_flash_tc(a, maps, pc, n_splits, q_tiles)
                       : tile ? (pc.D == 64u ? launch_flash_tile_d<64>(a, pc, n_splits, q_tiles)
                                           : launch_flash_tile_d<128>(a, pc, n_splits, q_tiles))
-                      : pc.D == 64u ? launch_flash_d<64>(a, pc, n_splits, counters)
-                      : pc.D == 128u ? launch_flash_d<128>(a, pc, n_splits, counters) : launch_flash_d<256>(a, pc, n_splits, counters);
+                      : pc.D == 64u ? (fd.wide ? launch_flash_d<64, 16>(a, pc, n_splits) : launch_flash_d<64, 8>(a, pc, n_splits))
+                      : pc.D == 128u ? (fd.wide ? launch_flash_d<128, 12>(a, pc, n_splits) : launch_flash_d<128, 8>(a, pc, n_splits))
+                                     : launch_flash_d<256, 4>(a, pc, n_splits);
     if (!fits) return AC_ERR_INVALID_WORK_GROUP_SIZE;
     AcResult rc = check_launch();
-    if (rc != AC_SUCCESS || n_splits == 1u || counters) return rc;
+    if (rc != AC_SUCCESS || n_splits == 1u) return rc;
     launch_pdl(flash_combine_kernel, dim3((unsigned)rows), dim3(128), 0, a.stream, (const float*)a.ptr[5], (float*)a.ptr[4],
                pc.D, (uint32_t)rows, n_splits, pc.part_off, pc.o_off);
     return check_launch();

@@ -219,6 +219,18 @@ def test_one_position_over_few_and_many_blocks(ctx, D, H, Hkv, n_kv):
     assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5, scratch=64) - want)) < TOL
 
 
+@pytest.mark.parametrize("D,H,Hkv,n_q,n_kv", [(128, 8, 8, 1, 1536), (128, 8, 8, 1, 1537), (64, 8, 2, 1, 1536), (64, 8, 2, 1, 1537),
+                                              (128, 32, 32, 1, 3551), (128, 8, 1, 1, 20000), (64, 32, 8, 1, 14301), (256, 8, 1, 1, 2500),
+                                              (256, 4, 2, 3, 700)])
+def test_one_position_on_both_sides_of_the_rules(ctx, D, H, Hkv, n_q, n_kv):
+    """The longest context with fine splits and the first with the wider CTAs and coarse ones; long ones; D = 256."""
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 13)
+    mask = causal(n_q, n_kv, (n_kv + 63) // 64 * 64)
+    want = attention(q, k, v, mask[:, :n_kv], D ** -0.5)
+    for scratch in (1 << 24, n_q * H * (D + 4) * 4 * 3 + 64):
+        assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5, scratch=scratch) - want)) < TOL
+
+
 def test_prompt_attention_among_kernels_with_tensor_memory(ctx):
     """Attention and tensor-core products in turn in one batch: each holds tensor memory, and each may be scheduled while the
     one before it still runs. Same bytes as one by one."""
