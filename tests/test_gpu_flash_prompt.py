@@ -236,15 +236,15 @@ def test_prompt_attention_among_kernels_with_tensor_memory(ctx):
     one before it still runs. Same bytes as one by one."""
     qmm = pkg.qmm
     from helpers import Q8_0, make_acts, make_weights
-    n_q, H, D = 160, 4, 64
-    q, k, v = inputs(n_q, n_q, H, H, D, 21)
-    mask = causal(n_q, n_q, 192)
+    n_q, H, Hkv, D = 256, 32, 8, 128
+    q, k, v = inputs(n_q, n_q, H, Hkv, D, 21)
+    mask = causal(n_q, n_q, 256)
     N, K = 384, 256
     blocks, scale = make_weights(Q8_0, N, K, 3)
     w = qmm.QuantWeight.from_ggml(ctx, Q8_0, blocks, N, K, scale)
     mm = qmm.MulMat(ctx, w, n_q)
-    push = [D, D, n_q, n_q, H, H, 0x11, 1, 0, H * D, D, 0, H * D, D, 0, H * D, D, 0, 192, 192 * n_q, 1, 0, fbits(D ** -0.5), 0, 0, 0, 0, 0,
-            0, 0, 0]
+    push = [D, D, n_q, n_q, H, Hkv, 0x11, 1, 0, H * D, D, 0, Hkv * D, D, 0, Hkv * D, D, 0, 256, 256 * n_q, 1, 0, fbits(D ** -0.5), 0, 0, 0,
+            0, 0, 0, 0, 0]
     bufs = [ctx.buffer(data=np.ascontiguousarray(a)) for a in (q, k, v, mask)] + [ctx.buffer(n_q * H * D * 4), ctx.buffer(1 << 22)]
     x, y = ctx.buffer(data=make_acts(n_q, K, 4)), ctx.buffer(n_q * N * 4)
 
@@ -269,3 +269,91 @@ def test_prompt_attention_among_kernels_with_tensor_memory(ctx):
     w.destroy()
     for b in bufs + [x, y]:
         b.destroy()
+
+
+@pytest.mark.parametrize("n_q,n_kv,H,Hkv,D", [(60, 1041, 32, 8, 128), (60, 1043, 32, 8, 128), (129, 1000, 14, 2, 64), (300, 1000, 14, 2, 64),
+                                              (75, 1250, 32, 32, 128), (150, 1250, 32, 32, 128), (130, 4100, 8, 8, 64), (420, 1800, 8, 8, 64)])
+def test_prompts_on_both_sides_of_the_work_rule(ctx, n_q, n_kv, H, Hkv, D):
+    """Little work (64 rows per CTA) and more (128 rows, tensor memory), grouped heads and not; the same tolerance."""
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 41)
+    mask = causal(n_q, n_kv, (n_kv + 63) // 64 * 64)
+    want = attention(q, k, v, mask[:, :n_kv], D ** -0.5)
+    for scratch in (64, 1 << 24):
+        assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5, scratch=scratch) - want)) < TOL
+
+
+# ---- the 128-row kernel: the same edges with enough heads that the work rule picks it -------------------------------------
+@pytest.mark.parametrize("n_q,n_kv,H,Hkv,D", [(50, 1100, 48, 16, 128), (43, 3001, 28, 4, 128), (129, 700, 24, 3, 128), (65, 2000, 32, 16, 64),
+                                              (300, 2600, 8, 8, 128), (17, 8200, 64, 64, 64)])
+def test_ragged_tiles_of_the_large_kernel(ctx, n_q, n_kv, H, Hkv, D):
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 51)
+    mask = causal(n_q, n_kv, (n_kv + 63) // 64 * 64)
+    want = attention(q, k, v, mask[:, :n_kv], D ** -0.5)
+    for scratch in (64, 1 << 26):
+        assert np.max(np.abs(run(ctx, q, k, v, mask, D ** -0.5, scratch=scratch) - want)) < TOL
+
+
+def test_forms_of_the_large_kernel(ctx):
+    n_q, n_kv, H, Hkv, D = 64, 520, 64, 32, 128
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 53)
+    rng = np.random.default_rng(53)
+    bias = rng.standard_normal((n_q, n_kv)).astype(np.float16)
+    per_head = np.where(rng.random((H, n_q, n_kv)) < 0.5, -np.inf, 0).astype(np.float16)
+    per_head[:, :, 0] = 0
+    for name, mask, scale, cap, kw in [("none", None, 0.09, 0.0, {}), ("bias", bias, 0.09, 0.0, {}), ("heads", per_head, 0.09, 0.0, {}),
+                                       ("odd", bias, 0.09, 0.0, {"m_off": 3}), ("cap", bias, 0.5, 5.0, {}), ("negative", None, -0.05, 0.0, {}),
+                                       ("zero", None, 0.0, 0.0, {}), ("output offset", None, 0.09, 0.0, {"o_off": 3, "scratch": 64}),
+                                       ("pitch", bias, 0.09, 0.0, {"kv_pitch": Hkv * D + 8})]:
+        assert np.max(np.abs(run(ctx, q, k, v, mask, scale, cap, **kw) - attention(q, k, v, mask, scale, cap))) < TOL, name
+
+
+def test_growing_scores_in_the_large_kernel(ctx):
+    n_q, n_kv, D = 64, 1024, 128
+    q, k, v = inputs(n_q, n_kv, 32, 16, D, 9)
+    q = np.abs(q).astype(np.float16)
+    k = (np.abs(k.astype(np.float32)) * np.linspace(0, 1, n_kv)[:, None, None]).astype(np.float16)
+    for scale in (0.02, 0.2, 1.0):
+        assert np.max(np.abs(run(ctx, q.astype(np.float32), k, v, None, scale) - attention(q, k, v, None, scale))) < TOL
+
+
+@pytest.mark.parametrize("D,H,Hkv", [(64, 128, 64), (128, 64, 32)])
+@pytest.mark.parametrize("last,m_off", [(320, 0), (288, 0), (272, 0), (304, 3), (16, 0)])
+def test_unused_cache_in_the_large_kernel(ctx, D, H, Hkv, last, m_off):
+    n_q, n_kv = 64, 512
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 5)
+    k[last:], v[last:] = np.inf, np.nan
+    mask = np.zeros((n_q, n_kv), np.float16)
+    mask[:, last:] = -np.inf
+    mask[7, :] = -np.inf
+    got = run(ctx, q, k, v, mask, D ** -0.5, m_off=m_off)
+    want = attention(q, k[:last], v[:last], None, D ** -0.5)
+    keep = [i for i in range(n_q) if i != 7]
+    assert np.isnan(got[7]).all() and np.max(np.abs(got[keep] - want[keep])) < TOL
+
+
+@pytest.mark.parametrize("D,H,Hkv", [(64, 48, 6), (128, 24, 12)])
+@pytest.mark.parametrize("scratch", [64, 1 << 26])
+def test_values_that_are_not_finite_in_the_large_kernel(ctx, D, H, Hkv, scratch):
+    n_q, n_kv = 150, 700
+    q, k, v = inputs(n_q, n_kv, H, Hkv, D, 31)
+    mask = causal(n_q, n_kv, 704)
+    v[600, :, 1::3] = np.inf
+    v[655, :, 2::5] = -np.inf
+    v[690, 0, ::7] = np.nan
+    v[697:, :, :] = np.nan
+    mask[:, 697:] = -np.inf
+    want = seen(q, k, v, mask[:, :n_kv], D ** -0.5)
+    got = run(ctx, q, k, v, mask, D ** -0.5, scratch=scratch)
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    assert np.max(np.abs(got[finite] - want[finite])) < TOL
+
+
+def test_more_keys_than_one_window_of_the_large_kernel(ctx):
+    n_q, n_kv, D = 17, 512 * 64 + 200, 64
+    q, k, v = inputs(n_q, n_kv, 8, 1, D, 6)
+    mask = causal(n_q, n_kv, n_kv)
+    mask[:, 1000:20000] = -np.inf
+    got = run(ctx, q, k, v, mask, D ** -0.5, scratch=64)
+    assert np.max(np.abs(got - attention(q, k, v, mask, D ** -0.5))) < TOL
