@@ -15,9 +15,11 @@
 // Before the tiles of a window are processed the mask is scanned once: tiles that are masked for all 128 rows are left out
 // of the list every role walks, tiles whose mask is all zero skip the mask arithmetic (a causal prompt has one or two mixed
 // tiles per CTA), and of a mixed tile only the k-steps of 16 keys that some row sees are multiplied with V: what lies in the
-// cache behind the last visible key (never written, perhaps NaN) takes no part. Two CTAs per SM: the exponentials of one overlap the MMAs of the other.
-// Bound by: the exponentials (64 per thread and tile) and the MMAs, both about 500 cycles per tile and CTA. The form it
-// replaces (mma.sync, 64 rows per CTA) ran at 77 TFLOP/s.
+// cache behind the last visible key (never written, perhaps NaN) takes no part. Up to two CTAs per SM.
+// Bound by latency: 512 positions x 2048 keys of 32 heads on 8 of 128 are 128 CTAs, one per SM with one softmax warp per
+// scheduler, tensor pipe 15 % active, DRAM idle (64 exponentials per thread and tile, S and P V in turn). 64 us at 2748 keys,
+// 327 TFLOP/s of unmasked products; the mma.sync form (64 rows per CTA) takes 242 us. For prompts of little work that form is the
+// faster one (flash_small in layer_ops.cu).
 // Rounding: Q to fp16 once as in the other attention kernels, scores, sums and accumulation in fp32. P with its remainder:
 // with the lazy reference the largest probability of a row is no longer exactly 1, and P rounded once left an error 1-5 %
 // above the mma.sync form's (2.9e-4 against 2.8e-4 of the result); with the remainder it is 2.1e-4. Rescaling at every

@@ -868,7 +868,7 @@ def layer_op_lines(env, steps=3):
                       "frac": nbytes / s / 1e9 / pk["hbm_gbs"], "launches_per_step": 1, "parity_max_abs_error": worst}
         for b in ks + vs + [qb, mb, ob, pb]:
             b.destroy()
-    # ---- attention over a prompt: 512 positions against themselves under a causal mask (tensor-bound, mma.sync) ----
+    # ---- attention over a prompt: 512 positions against themselves under a causal mask (the kernel of flash_tc.cu, bound by latency) ----
     n_q = n_kv = 512
     kv = (rng.standard_normal((n_head_kv, n_kv, D), dtype=np.float32)).astype(np.float16)
     q = rng.standard_normal((n_head, n_q, D)).astype(np.float32)
