@@ -165,6 +165,9 @@ __global__ void __launch_bounds__(256) rms_norm_f32_vec_kernel(const float* x, c
 // From here on the vector forms: below it (rows of token generation) one element per thread spreads the few thousand elements
 // over more SMs (a decoder layer at one row, 4096 wide: 93.0 against 93.9 us).
 constexpr uint64_t kVecMin = 1u << 16;
+// SWIGLU: eight exponentials and divisions in a row per thread take longer than the loads they save until the chip is full
+// (us, vector form / scalar: 65536 elements 2.8 / 1.8, 524288 3.6 / 3.3, 2097152 6.2 / 9.5)
+constexpr uint64_t kVecMinGate = 1u << 20;
 
 // ameva_add_f32 / ameva_mul_f32: bindings 0 a f32 [rows][cols], 1 b f32 [b_rows][cols], 2 dst f32 [rows][cols];
 //   push {rows, cols, b_rows (rows % b_rows == 0; 1 = one row broadcast over all)}
@@ -197,7 +200,7 @@ AcResult launch_swiglu_f32(const LaunchArgs& a) {
     const uint64_t n = a.push[0];
     if (n == 0) return AC_ERR_KERNEL_ARG_INVALID;
     if (a.range[0] < n * 4u || a.range[1] < n * 4u || a.range[2] < n * 4u) return AC_ERR_INVALID_BUFFER_SIZE;
-    if (n >= kVecMin) {
+    if (n >= kVecMinGate) {
         const uint64_t span = 4u * kVecThreads * kVecPieces;
         launch_pdl(swiglu_f32_vec_kernel, dim3((unsigned)((n + span - 1u) / span)), dim3(kVecThreads), 0, a.stream,
                    (const float*)a.ptr[0], (const float*)a.ptr[1], (float*)a.ptr[2], n);

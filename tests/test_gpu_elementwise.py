@@ -123,3 +123,18 @@ def test_rms_norm_at_the_edges_of_the_register_form(ctx, cols):
     assert np.all(np.abs(xb.read(np.float32).reshape(3, cols) - want) <= 1.5e-6 * np.abs(want) + 1e-30)
     xb.destroy()
     wb.destroy()
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 3, (1 << 20) + 2047, (1 << 20) + 2050])
+def test_swiglu_on_both_sides_of_its_vector_form(ctx, n):
+    rng = np.random.default_rng(n)
+    g, u = (rng.standard_normal(n).astype(np.float32) * 3 for _ in range(2))
+    gb, ub, db = ctx.buffer(data=g), ctx.buffer(data=u), ctx.buffer(n * 4 + 64)
+    db.write(np.zeros(n + 16, np.float32))
+    _run(ctx, "ameva_swiglu_f32", [gb, ub, db], [n])
+    got = db.read(np.float32)
+    g64 = g.astype(np.float64)
+    assert np.allclose(got[:n], g64 / (1 + np.exp(-g64)) * u, rtol=2e-6, atol=1e-7)
+    assert not got[n:].any()
+    for b in (gb, ub, db):
+        b.destroy()
