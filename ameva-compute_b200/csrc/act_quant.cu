@@ -26,6 +26,13 @@ struct QuantDsts {
     uint32_t n;
     QuantDst d[kFuseMax];
 };
+// store(d) for every destination; the first, mostly the only one, from parameters at fixed offsets
+template <class Store>
+__device__ __forceinline__ void for_each_dst(const QuantDsts& dst, Store store) {
+    store(dst.d[0]);
+#pragma unroll 1
+    for (uint32_t i = 1; i < dst.n; ++i) store(dst.d[i]);
+}
 // What is quantized: the rows at src; or, SWIGLU, silu(src) * up, written to act as ameva_swiglu_f32 writes it (rows of K
 // floats, no gaps in any of the three).
 struct GateArgs {
@@ -65,10 +72,10 @@ __global__ void __launch_bounds__(256) quant_q8_0_kernel(const float* __restrict
     quant_unit_q8_0(x, round_mode, q, d, s);
     if (live) {
         const uint32_t word = scale_word_q8_0(d, s);
-        for (uint32_t i = 0; i < dst.n; ++i) {
-            reinterpret_cast<uint32_t*>(dst.d[i].aq + (size_t)m * K + 32u * u)[sub] = pack_q4(q);
-            if (sub == 0) reinterpret_cast<uint32_t*>(dst.d[i].ad)[(size_t)m * U + u] = word;
-        }
+        for_each_dst(dst, [&](const QuantDst& to) {
+            reinterpret_cast<uint32_t*>(to.aq + (size_t)m * K + 32u * u)[sub] = pack_q4(q);
+            if (sub == 0) reinterpret_cast<uint32_t*>(to.ad)[(size_t)m * U + u] = word;
+        });
     }
 }
 
@@ -116,16 +123,16 @@ __global__ void __launch_bounds__(256) quant_q8_K_kernel(const float* __restrict
         w1 |= (uint32_t)(q[i + 4] & 0xFF) << (8 * i);
     }
     s += __shfl_xor_sync(0xffffffffu, s, 1);  // lanes 2j, 2j+1 -> 16-element group j
-    for (uint32_t i = 0; i < dst.n; ++i) {
-        *reinterpret_cast<uint2*>(dst.d[i].aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
-        uint8_t* blk = dst.d[i].ad + ((size_t)m * B + b) * kABBytes;
+    for_each_dst(dst, [&](const QuantDst& to) {
+        *reinterpret_cast<uint2*>(to.aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
+        uint8_t* blk = to.ad + ((size_t)m * B + b) * kABBytes;
         if ((lane & 1u) == 0u) reinterpret_cast<int16_t*>(blk)[lane >> 1] = (int16_t)s;
         if (lane == 0) {
             *reinterpret_cast<float*>(blk + 32) = d;
             *reinterpret_cast<uint32_t*>(blk + 36) = 0u;
             *reinterpret_cast<uint2*>(blk + 40) = make_uint2(0u, 0u);
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -254,7 +261,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
         amax = block_max<kRowThreads / 32>(amax, red);
         float s, inv;
         row_factor(amax, s, inv);
-        if (t < dst.n && dst.d[t].ae) dst.d[t].ae[m] = inv;
+        if (t == 0) for_each_dst(dst, [&](const QuantDst& to) { if (to.ae) to.ae[m] = inv; });
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const uint32_t i = t + (uint32_t)kRowThreads * j, u = i >> 3;
@@ -264,16 +271,16 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
             quant_unit_q8_0(v[j], mode, q, d, sum);
             if (live) {
                 const uint32_t word = scale_word_q8_0(d, sum);
-                const float dh = __fmul_rn(h2f(f2h(d)), s);   // the fp16-rounded scale the dot product uses, times 2^-e
-                const __half2 h01 = __floats2half2_rn((float)q[0] * dh, (float)q[1] * dh);
-                const __half2 h23 = __floats2half2_rn((float)q[2] * dh, (float)q[3] * dh);
-                const uint2 o = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
-                for (uint32_t k = 0; k < dst.n; ++k) {
-                    const QuantDst& to = dst.d[k];
+                for_each_dst(dst, [&](const QuantDst& to) {
                     reinterpret_cast<uint32_t*>(to.aq + (size_t)m * K)[i] = pack_q4(q);
                     if (sub == 0) reinterpret_cast<uint32_t*>(to.ad)[(size_t)m * U + u] = word;
-                    if (to.ah) *reinterpret_cast<uint2*>(to.ah + (size_t)m * K + 4u * i) = o;
-                }
+                    if (!to.ah) return;
+                    const float dh = __fmul_rn(h2f(f2h(d)), s);   // the fp16-rounded scale the dot product uses, times 2^-e
+                    const __half2 h01 = __floats2half2_rn((float)q[0] * dh, (float)q[1] * dh);
+                    const __half2 h23 = __floats2half2_rn((float)q[2] * dh, (float)q[3] * dh);
+                    *reinterpret_cast<uint2*>(to.ah + (size_t)m * K + 4u * i) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+                });
             }
         }
     } else {
@@ -345,7 +352,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
         amax = block_max<kRowThreads / 32>(amax, red);
         float s, inv;
         row_factor(amax, s, inv);
-        if (t < dst.n && dst.d[t].ae) dst.d[t].ae[m] = inv;
+        if (t == 0) for_each_dst(dst, [&](const QuantDst& to) { if (to.ae) to.ae[m] = inv; });
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const uint32_t b = (t >> 5) + (uint32_t)(kRowThreads / 32) * j;
@@ -361,19 +368,19 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
                 w0 |= (uint32_t)(q[i] & 0xFF) << (8 * i);
                 w1 |= (uint32_t)(q[i + 4] & 0xFF) << (8 * i);
             }
-            const float ds = __fmul_rn(d, s);
-            uint32_t o[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const __half2 hh = __floats2half2_rn((float)q[2 * i] * ds, (float)q[2 * i + 1] * ds);
-                o[i] = *reinterpret_cast<const uint32_t*>(&hh);
-            }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);  // lanes 2j, 2j+1 -> 16-element group j
-            for (uint32_t k = 0; k < dst.n; ++k) {
-                const QuantDst& to = dst.d[k];
+            for_each_dst(dst, [&](const QuantDst& to) {
                 *reinterpret_cast<uint2*>(to.aq + (size_t)m * K + 256u * b + 8u * lane) = make_uint2(w0, w1);
-                if (to.ah)
+                if (to.ah) {
+                    const float ds = __fmul_rn(d, s);
+                    uint32_t o[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const __half2 hh = __floats2half2_rn((float)q[2 * i] * ds, (float)q[2 * i + 1] * ds);
+                        o[i] = *reinterpret_cast<const uint32_t*>(&hh);
+                    }
                     *reinterpret_cast<uint4*>(to.ah + (size_t)m * K + 256u * b + 8u * lane) = make_uint4(o[0], o[1], o[2], o[3]);
+                }
                 uint8_t* blk = to.ad + ((size_t)m * B + b) * kABBytes;
                 if ((lane & 1u) == 0u) reinterpret_cast<int16_t*>(blk)[lane >> 1] = (int16_t)sum;
                 if (lane == 0) {
@@ -381,7 +388,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_f16_kernel(const float
                     *reinterpret_cast<uint32_t*>(blk + 36) = 0u;
                     *reinterpret_cast<uint2*>(blk + 40) = make_uint2(0u, 0u);
                 }
-            }
+            });
         }
     }
 }
