@@ -160,7 +160,7 @@ AcResult fuse_bitnet_gemv(FuseOp* ops, uint32_t n, uint32_t i, bool* taken) {
     for (uint32_t j = i + 1; j < n && j <= i + kLookahead && count < kFuseMax; ++j) {
         if (ops[j].done) continue;
         const LaunchArgs& p = ops[j].args;
-        if (is(ops[j], launch_bitnet_gemv_i2_s) && !p.stream.in_order && p.push[0] == K && (p.push[4] ? p.push[4] : 1u) == M &&
+        if (M <= 2u && is(ops[j], launch_bitnet_gemv_i2_s) && !p.stream.in_order && p.push[0] == K && (p.push[4] ? p.push[4] : 1u) == M &&
             check_bitnet_gemv_i2_s(p) == AC_SUCCESS && can_hoist(ops, i, j, mask)) {
             bool ok = true;   // no product writes what another one reads or writes
             for (uint32_t m = 0; m < count && ok; ++m)

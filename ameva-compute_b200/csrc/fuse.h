@@ -27,7 +27,7 @@ AcResult check_bitnet_norm_q8(const LaunchArgs& a);
 bool bitnet_rows_fits(const LaunchArgs& norm_q8);   // a plain quantize (mode 0, no norm) the row kernel serves
 AcResult launch_bitnet_rows(BitnetSource source, const LaunchArgs* head, const LaunchArgs* const* norm_q8, uint32_t n);
 
-// up to four I2_S products (bitnet_gemv_i2_s_*) of the same K and row count in one launch; add: with n == 1, the
+// up to four I2_S products (bitnet_gemv_i2_s_*) of the same K and row count (1 or 2) in one launch; add: with n == 1, the
 // ameva_add_f32 whose first (swapped: second) operand is the product
 AcResult check_bitnet_gemv_i2_s(const LaunchArgs& a);
 AcResult launch_bitnet_gemv_i2_s_group(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped);

@@ -542,16 +542,22 @@ struct I2sGroup {
     float* out;                    // nullptr: no ADD
 };
 
-template <int M, int R, bool ACC>
-__global__ void __launch_bounds__(kGemvThreads)
+// MODE: one product (I2S_ONE, I2S_ACC: added to the output), or the group, whose pointers are no longer the same for all warps:
+// they take registers, 160 against 117 with three rows, one CTA per SM instead of two, so groups have at most two rows.
+enum { I2S_ONE, I2S_ACC, I2S_GROUP };
+template <int M, int R, int MODE>
+__global__ void __launch_bounds__(kGemvThreads, MODE == I2S_GROUP ? 0 : M <= 2 ? 4 : M == 3 ? 2 : 0)
 gemv_i2_s_kernel(const I2sGroup gr, uint32_t K) {
+    constexpr bool ACC = MODE == I2S_ACC;
     uint32_t warp = (blockIdx.x * kGemvThreads + threadIdx.x) >> 5, j = 0;
     const uint32_t lane = threadIdx.x & 31u;
     if (warp >= gr.warp_end[kFuseMax - 1]) return;
+    if constexpr (MODE == I2S_GROUP) {
 #pragma unroll
-    for (uint32_t i = 0; i + 1u < kFuseMax; ++i)
-        if (warp >= gr.warp_end[i]) j = i + 1u;
-    if (j) warp -= gr.warp_end[j - 1u];
+        for (uint32_t i = 0; i + 1u < kFuseMax; ++i)
+            if (warp >= gr.warp_end[i]) j = i + 1u;
+        if (j) warp -= gr.warp_end[j - 1u];
+    }
     const uint4* __restrict__ W = gr.W[j];
     const int8_t* __restrict__ AQ = gr.AQ[j];
     const uint32_t* __restrict__ ACT = gr.ACT[j];
@@ -616,14 +622,21 @@ gemv_i2_s_kernel(const I2sGroup gr, uint32_t K) {
         c0 += 32 * UN;
         if (c0 < C) load_weights(c0);
     }
+    // the rows' records before the first store, which they would have to wait for otherwise
+    uint32_t act_scale[M], act_sum[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        act_scale[m] = __ldg(ACT + 2 * m);
+        act_sum[m] = __ldg(ACT + 2 * m + 1);
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int m = 0; m < M; ++m) {
             const int tot = warp_sum_i(acc[r][m]);
             if (lane == 0 && row0 + r < N) {
-                const int sum = tot - (int)__ldg(ACT + 2 * m + 1);
-                const float total_scale = __fmul_rn(__uint_as_float(__ldg(ACT + 2 * m)), w_scale);
+                const int sum = tot - (int)act_sum[m];
+                const float total_scale = __fmul_rn(__uint_as_float(act_scale[m]), w_scale);
                 const float v = __fmul_rn((float)sum, total_scale);
                 float* o = dst + (size_t)m * dst_stride + row0 + r;
                 *o = ACC ? __fadd_rn(*o, v) : v;
@@ -890,7 +903,7 @@ AcResult check_bitnet_gemv_i2_s(const LaunchArgs& a) {
 }
 
 // checked products of the same K and row count
-template <bool ACC>
+template <int MODE>
 static AcResult launch_i2s(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped) {
     const LaunchArgs& a = *gemv[0];
     const uint32_t K = a.push[0], M = a.push[4] ? a.push[4] : 1u, R = M <= 2u ? 2u : 4u;   // (R as in AMV_GEMV_SWITCH)
@@ -917,19 +930,24 @@ static AcResult launch_i2s(const LaunchArgs* const* gemv, uint32_t n, const Laun
         g.out = (float*)add->ptr[2];
     }
     const uint32_t N = (uint32_t)warps * R;   // (the switch's row count: whole warps of every product)
-    AMV_GEMV_SWITCH(gemv_i2_s_kernel, ACC, g, K)
+    if constexpr (MODE == I2S_GROUP) {
+        if (M == 1u) launch_pdl(gemv_i2_s_kernel<1, 2, MODE>, dim3(gemv_blocks<2>(N)), dim3(kGemvThreads), 0, a.stream, g, K);
+        else launch_pdl(gemv_i2_s_kernel<2, 2, MODE>, dim3(gemv_blocks<2>(N)), dim3(kGemvThreads), 0, a.stream, g, K);
+    } else {
+        AMV_GEMV_SWITCH(gemv_i2_s_kernel, MODE, g, K)
+    }
     return check_launch();
 }
 AcResult launch_bitnet_gemv_i2_s_group(const LaunchArgs* const* gemv, uint32_t n, const LaunchArgs* add, bool swapped) {
-    return launch_i2s<false>(gemv, n, add, swapped);
+    return n > 1u ? launch_i2s<I2S_GROUP>(gemv, n, add, swapped) : launch_i2s<I2S_ONE>(gemv, n, add, swapped);
 }
-template <bool ACC>
+template <int MODE>
 static AcResult launch_i2s_one(const LaunchArgs& a) {
     const AcResult rc = check_bitnet_gemv_i2_s(a);
     const LaunchArgs* one = &a;
-    return rc != AC_SUCCESS ? rc : launch_i2s<ACC>(&one, 1u, nullptr, false);
+    return rc != AC_SUCCESS ? rc : launch_i2s<MODE>(&one, 1u, nullptr, false);
 }
-AcResult launch_bitnet_gemv_i2_s(const LaunchArgs& a) { return launch_i2s_one<false>(a); }
-AcResult launch_bitnet_gemv_i2_s_acc(const LaunchArgs& a) { return launch_i2s_one<true>(a); }
+AcResult launch_bitnet_gemv_i2_s(const LaunchArgs& a) { return launch_i2s_one<I2S_ONE>(a); }
+AcResult launch_bitnet_gemv_i2_s_acc(const LaunchArgs& a) { return launch_i2s_one<I2S_ACC>(a); }
 
 }  // namespace amv
