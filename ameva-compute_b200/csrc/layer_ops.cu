@@ -83,7 +83,8 @@ __device__ __forceinline__ void st_pair(T* d, uint64_t e0, uint64_t e1, bool vec
 }
 
 // How the pairs are dealt to a grid: a CTA takes one position and `heads_per_cta` heads (`chunks` CTAs per position); threads:
-// jt consecutive pairs x 256 / jt head lanes. vec: f32 pairs (e0, e0 + 1) start on 8 bytes in source and destination.
+// jt consecutive pairs x 256 / jt head lanes (jt: the pairs of a row, 8 to 256). vec: f32 pairs (e0, e0 + 1) start on 8 bytes in
+// source and destination.
 struct RopePlan {
     uint32_t jt, chunks, heads_per_cta, vec, ctas;
 };
@@ -109,7 +110,8 @@ template <typename T>
 __device__ __forceinline__ void rope_body(const T* a, const int32_t* __restrict__ pos, const float* __restrict__ ff, T* d,
                                           const RopeArgs& pc, const RopePlan& plan, const uint32_t block, const RopeStore* store) {
     const uint32_t jt = plan.jt, chunks = plan.chunks, heads_per_cta = plan.heads_per_cta, vec = plan.vec;
-    const uint32_t half_ne0 = pc.ne0 >> 1, hg = 256u / jt, j0 = threadIdx.x & (jt - 1u), hl = threadIdx.x / jt;
+    const uint32_t half_ne0 = pc.ne0 >> 1, hg = 256u / jt, hl = threadIdx.x / jt, j0 = threadIdx.x - hl * jt;
+    if (hl >= hg) return;   // (threads past the last whole head lane)
     const uint32_t row = block / chunks, chunk = block - row * chunks;
     const uint32_t i3 = row / pc.ne2, i2 = row - i3 * pc.ne2;
     const uint64_t a23 = pc.a_off + (uint64_t)i2 * pc.a_s2 + (uint64_t)i3 * pc.a_s3;
@@ -217,8 +219,7 @@ static AcResult check_rope_t(const LaunchArgs& a, RopeArgs* out, RopePlan* plan)
         (pc.has_ff && a.range[2] < ((uint64_t)pc.ff_off + pc.n_dims / 2u) * 4u))
         return AC_ERR_INVALID_BUFFER_SIZE;
     const uint64_t rows = (uint64_t)pc.ne2 * pc.ne3;
-    uint32_t jt = 8u;
-    while (jt < pc.ne0 / 2u && jt < 256u) jt *= 2u;
+    const uint32_t half = pc.ne0 / 2u, jt = half < 8u ? 8u : half < 256u ? half : 256u;
     const uint32_t hg = 256u / jt;
     // few positions (token generation): one head per thread, so that the heads spread over the SMs; many: all the heads a
     // thread can carry, so that sine and cosine are formed once

@@ -416,6 +416,21 @@ def test_rope_over_many_positions_and_odd_heads(ctx, shape, n_dims, a_off, neox)
         b.destroy()
 
 
+@pytest.mark.parametrize("neox", [False, True])
+@pytest.mark.parametrize("shape,n_dims", [((1, 100, 32, 80), 80), ((1, 200, 7, 96), 64), ((1, 3, 33, 160), 160), ((1, 160, 9, 14), 14), ((1, 2, 5, 510), 510)])
+def test_rope_in_place_on_rows_of_other_than_a_power_of_two(ctx, shape, n_dims, neox):
+    """Every pair is rotated once, also by the threads next to the idle ones of a CTA."""
+    rng = np.random.default_rng(shape[3])
+    x = rng.standard_normal(shape).astype(np.float32)
+    pos = rng.integers(0, 8192, shape[1]).astype(np.int32)
+    xb, pb = ctx.buffer(data=x), ctx.buffer(data=pos)
+    _run(ctx, "ameva_rope", [xb, pb, pb, xb], _rope_push(shape, n_dims, neox, 0, ops.rope_theta_scale(10000.0, n_dims), 1.0, 0.0, 1.0, (0.0, 0.0)))
+    got = xb.read(np.float32).reshape(shape)
+    assert np.max(np.abs(got - ops.rope(x, pos, n_dims, neox, 10000.0))) <= 4e-6 * np.max(np.abs(x))
+    xb.destroy()
+    pb.destroy()
+
+
 @pytest.mark.parametrize("dst_dtype", [np.float16, np.float32])
 @pytest.mark.parametrize("nc", [4, 1020, 1024, 1028, 1030])
 def test_set_rows_at_the_edges_of_the_vector_form(ctx, nc, dst_dtype):
