@@ -186,21 +186,22 @@ __device__ __forceinline__ void group_dot_q23(const uint4 w, uint32_t gi, const 
 // The kernel. A policy names the weights per scale record (1 << kUnit), the bytes of a record and the dot product of one
 // 16-weight group. add: the ADD behind the product, when the launch carries it (M rows of N floats without gaps).
 // ---------------------------------------------------------------------------------------------------------------------
-#define AMV_BYTE_POLICY(NAME, UNIT, REC, DOT)                                                                              \
+#define AMV_BYTE_POLICY(NAME, UNIT, REC, AHEAD, DOT)                                                                       \
     struct NAME {                                                                                                          \
         static constexpr uint32_t kUnit = UNIT, kRec = REC;                                                                \
+        static constexpr bool kAhead = AHEAD;                                                                              \
         template <int M>                                                                                                   \
         static __device__ __forceinline__ void dot(const uint4 w, uint32_t gi, const uint8_t* s, const int8_t* __restrict__ AQ, \
                                                    const uint8_t* __restrict__ AD, uint32_t K, uint32_t units, float (&acc)[M]) { \
             DOT(w, gi, s, AQ, AD, K, units, acc);                                                                          \
         }                                                                                                                  \
     };
-AMV_BYTE_POLICY(ByteQ6K, 8, kQ6ScaleBytes, group_dot<M>)
-AMV_BYTE_POLICY(ByteQ5K, 8, 16, group_dot_q5<M>)
-AMV_BYTE_POLICY(ByteIq4Xs, 8, 8, group_dot_iq4xs<M>)
-AMV_BYTE_POLICY(ByteQ41, 5, 4, group_dot_q41<M>)
-AMV_BYTE_POLICY(ByteQ3K, 8, 14, (group_dot_q23<M, 3>))
-AMV_BYTE_POLICY(ByteQ2K, 8, 20, (group_dot_q23<M, 2>))
+AMV_BYTE_POLICY(ByteQ6K, 8, kQ6ScaleBytes, true, group_dot<M>)
+AMV_BYTE_POLICY(ByteQ5K, 8, 16, false, group_dot_q5<M>)
+AMV_BYTE_POLICY(ByteIq4Xs, 8, 8, true, group_dot_iq4xs<M>)
+AMV_BYTE_POLICY(ByteQ41, 5, 4, true, group_dot_q41<M>)
+AMV_BYTE_POLICY(ByteQ3K, 8, 14, true, (group_dot_q23<M, 3>))
+AMV_BYTE_POLICY(ByteQ2K, 8, 20, true, (group_dot_q23<M, 2>))
 #undef AMV_BYTE_POLICY
 
 struct ByteAdd {
@@ -208,9 +209,12 @@ struct ByteAdd {
     float* out;
 };
 
-// (one row: 64 registers, so that four CTAs are resident and a 4096-row product is one wave)
-template <class T, int M>
-__global__ void __launch_bounds__(kQ6Warps * 32, M == 1 ? 4 : 1)
+// AHEAD (see the launcher): the first two steps of weights are requested before the wait, and a step is always in flight during
+// the arithmetic. Otherwise a step is requested when it is needed. 64 registers for both, four CTAs per SM: left to itself the
+// compiler takes 32-60 without AHEAD and keeps fewer loads in flight (Q5_K x 8 rows, 4096 x 14336: 60.8 us, with the bound 42.4;
+// the kernels of the single types took 45.1).
+template <class T, int M, bool AHEAD>
+__global__ void __launch_bounds__(kQ6Warps * 32, 4)
 byte_gemv_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S, const int8_t* __restrict__ AQ,
                  const uint8_t* __restrict__ AD, float* __restrict__ dst, uint32_t N, uint32_t K, uint32_t dst_stride,
                  const ByteAdd add) {
@@ -223,17 +227,13 @@ byte_gemv_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S, c
     extern __shared__ __align__(16) uint8_t byte_smem[];
     const uint32_t rec_bytes = units * T::kRec;
     uint8_t* s = byte_smem + (size_t)warp * ((rec_bytes + 15u) & ~15u);
-    uint4 w[UN], nx[UN];
-    auto load = [&](uint4 (&to)[UN], uint32_t base) {
-#pragma unroll
-        for (uint32_t u = 0; u < UN; ++u) {
-            const uint32_t gi = base + 32u * u + lane;
-            if (gi < groups) to[u] = ld_stream_u4(q + gi);
-        }
-    };
     // neither the weights nor their scale records depend on the kernel before this one
-    load(w, 0u);
-    load(nx, STEP);
+    uint4 ahead[AHEAD ? 2u * UN : 1u];
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (uint32_t u = 0; u < 2u * UN; ++u)
+            if (32u * u + lane < groups) ahead[u] = ld_stream_u4(q + 32u * u + lane);
+    }
     const uint8_t* src = S + (size_t)row * rec_bytes;
     if (((uintptr_t)src & 3u) == 0u && (rec_bytes & 3u) == 0u) {
         for (uint32_t i = lane; i < rec_bytes / 4u; i += 32u) reinterpret_cast<uint32_t*>(s)[i] = __ldg(reinterpret_cast<const uint32_t*>(src) + i);
@@ -246,15 +246,30 @@ byte_gemv_kernel(const uint8_t* __restrict__ Q, const uint8_t* __restrict__ S, c
     float acc[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) acc[m] = 0.0f;
-    for (uint32_t base = 0; base < groups; base += STEP) {
+    if constexpr (AHEAD) {
+        for (uint32_t base = 0; base < groups; base += STEP) {
 #pragma unroll
-        for (uint32_t u = 0; u < UN; ++u) {
-            const uint32_t gi = base + 32u * u + lane;
-            if (gi < groups) T::template dot<M>(w[u], gi, s, AQ, AD, K, units, acc);
+            for (uint32_t u = 0; u < UN; ++u) {
+                const uint32_t gi = base + 32u * u + lane;
+                if (gi < groups) T::template dot<M>(ahead[u], gi, s, AQ, AD, K, units, acc);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < UN; ++u) {
+                ahead[u] = ahead[UN + u];
+                const uint32_t gi = base + 2u * STEP + 32u * u + lane;
+                if (gi < groups) ahead[UN + u] = ld_stream_u4(q + gi);
+            }
         }
+    } else {
+        uint32_t gi = lane;
+        for (; gi + 32u * (UN - 1u) < groups; gi += STEP) {
+            uint4 w[UN];
 #pragma unroll
-        for (uint32_t u = 0; u < UN; ++u) w[u] = nx[u];
-        load(nx, base + 2u * STEP);
+            for (uint32_t u = 0; u < UN; ++u) w[u] = ld_stream_u4(q + gi + 32u * u);
+#pragma unroll
+            for (uint32_t u = 0; u < UN; ++u) T::template dot<M>(w[u], gi + 32u * u, s, AQ, AD, K, units, acc);
+        }
+        for (; gi < groups; gi += 32u) T::template dot<M>(ld_stream_u4(q + gi), gi, s, AQ, AD, K, units, acc);
     }
 #pragma unroll
     for (int m = 0; m < M; ++m) {
@@ -287,15 +302,28 @@ static AcResult launch_byte_gemv(const LaunchArgs& a, uint32_t max_k, uintptr_t 
         launch_pdl(kernel, dim3((N + kQ6Warps - 1) / kQ6Warps), dim3(kQ6Warps * 32), smem, a.stream, (const uint8_t*)a.ptr[0],
                    (const uint8_t*)a.ptr[1], (const int8_t*)a.ptr[2], (const uint8_t*)a.ptr[3], (float*)a.ptr[4], N, K, dst_stride, add);
     };
+    // AHEAD where its four CTAs per SM are a wave of their own or one of many (us, AHEAD / not, Q6_K x 1 row: 4096 x 14336 10.0 /
+    // 14.6, 4096 x 4096 3.4 / 4.6, 28672 x 4096 20.0 / 20.9; 5203 x 4096 5.5 / 4.9, 1024 x 4096 2.8 / 2.6); never for Q5_K, whose
+    // dot product does not fit 64 registers with it (5203 x 4096 10.2 / 5.6)
+    const uint64_t ctas = (N + kQ6Warps - 1) / kQ6Warps, sms = a.sm_count > 0 ? (uint64_t)a.sm_count : 148u;
+    const bool ahead = (ctas > sms && ctas <= 4u * sms) || ctas >= 16u * sms;
     switch (M) {
-        case 1: go(byte_gemv_kernel<T, 1>); break;
-        case 2: go(byte_gemv_kernel<T, 2>); break;
-        case 3: go(byte_gemv_kernel<T, 3>); break;
-        case 4: go(byte_gemv_kernel<T, 4>); break;
-        case 5: go(byte_gemv_kernel<T, 5>); break;
-        case 6: go(byte_gemv_kernel<T, 6>); break;
-        case 7: go(byte_gemv_kernel<T, 7>); break;
-        default: go(byte_gemv_kernel<T, 8>); break;
+        case 1:
+            if constexpr (T::kAhead) {
+                if (ahead) {
+                    go(byte_gemv_kernel<T, 1, true>);
+                    break;
+                }
+            }
+            go(byte_gemv_kernel<T, 1, false>);
+            break;
+        case 2: go(byte_gemv_kernel<T, 2, false>); break;
+        case 3: go(byte_gemv_kernel<T, 3, false>); break;
+        case 4: go(byte_gemv_kernel<T, 4, false>); break;
+        case 5: go(byte_gemv_kernel<T, 5, false>); break;
+        case 6: go(byte_gemv_kernel<T, 6, false>); break;
+        case 7: go(byte_gemv_kernel<T, 7, false>); break;
+        default: go(byte_gemv_kernel<T, 8, false>); break;
     }
     return check_launch();
 }
