@@ -29,8 +29,9 @@ static inline float u2f_host(uint32_t u) {
 __device__ __forceinline__ uint64_t linear_id() { return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// ROPE (ggml_rope_ext forward), modes NORMAL and NEOX, optional frequency factors, YaRN mixing. The angle is built as ggml's CPU backend builds it: theta = pos * theta_scale^j by repeated f32 multiplication
-// (bit-identical angle), divided by the frequency factor, mixed, then sinf / cosf. F16: source and destination are f16
+// ROPE (ggml_rope_ext forward), modes NORMAL and NEOX, optional frequency factors, YaRN mixing. The angle is built as ggml's
+// CPU backend builds it: theta = pos * theta_scale^j by repeated f32 multiplication (bit-identical angle), divided by the
+// frequency factor, mixed, then sinf / cosf. F16: source and destination are f16
 // and may be the same range (llama.cpp rotates stored keys in place): a thread reads its two elements before it writes
 // them and no other thread touches them; 16-bit stores need no atomics here.
 // ---------------------------------------------------------------------------------------------------------------------
