@@ -1652,7 +1652,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
         }
         break;
     }
-    // Few tiles: K ranges in clusters (SPLIT) where that finishes earlier. Costs in thirds of a microsecond, from measured
+    // Few tiles: K ranges in clusters (SPLIT) where that finishes earlier. Costs in thirtieths of a microsecond, from measured
     // launches: a K block about 0.55 us at 256 tokens and 0.4 us at few (the conversion's share), a flag chain 3 us per extra
     // K range of a tile, the exchange through a cluster 2 us; every unit resident in one wave.
     if (pair && !n_peers && !forced && !(diag & 64u) && (KB & 3u) == 0u) {
