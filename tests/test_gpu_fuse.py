@@ -214,3 +214,69 @@ def test_nothing_behind_a_refused_dispatch_has_run(ctx, bad):
     assert any(held["p0q"].read(np.uint8)) and not any(held["p1q"].read(np.uint8)) and not any(held["p1y"].read(np.uint8))
     for b in held.values():
         b.destroy()
+
+
+def launches(ctx, bufs, ops):
+    """How many launches the dispatches leave in when they are one batch."""
+    held = {n: ctx.buffer(data=a) for n, a in bufs.items()}
+    batch = ctx.batch(len(ops))
+    for name, binds, push, grid in ops:
+        batch.dispatch(ctx.kernel(name), [held[b] for b in binds], push, grid)
+    ev = batch.submit()
+    ev.wait()
+    n = batch.launches()[0]
+    ev.destroy()
+    batch.destroy()
+    for b in held.values():
+        b.destroy()
+    return n
+
+
+def test_number_of_launches(ctx):
+    """The forms above leave in fewer launches, aliased operands in as many as before."""
+    rng = np.random.default_rng(7)
+    K = 512
+
+    def base(M):
+        return {n: rng.standard_normal(M * K).astype(np.float32) for n in ("x", "w", "h", "gate", "up", "act")}
+
+    # I2_S: norm, three quantizes and three products (one or two rows: two launches; three rows: the products alone)
+    for M, want in ((1, 2), (2, 2), (3, 4)):
+        bufs = base(M)
+        ops = [("ameva_rms_norm_f32", ["x", "w", "h"], [M, K, fbits(1e-5), 1], ONE)]
+        for j, N in enumerate((64, 33, 128)):
+            ops += i2_s(f"p{j}", "h", M, N, K, rng, bufs, f"o{j}")
+        assert launches(ctx, bufs, ops) == want
+    # the quantize writes the rows that it reads: it stays apart from the norm, and so does what follows
+    bufs = base(1)
+    ops = [("ameva_rms_norm_f32", ["x", "w", "h"], [1, K, fbits(1e-5), 1], ONE)] + i2_s("p0", "h", 1, 64, K, rng, bufs, "o0", y="h")
+    assert launches(ctx, bufs, ops) == 3
+    # gate, quantize, product and residual: two; with the sum written over the quantized row: three
+    bufs = dict(base(1), res=np.zeros(64, np.float32), sum=np.zeros(K, np.float32))
+    ops = [("ameva_swiglu_f32", ["gate", "up", "act"], [K], ONE)] + i2_s("d", "act", 1, 64, K, rng, bufs, "tmp")
+    add = ("ameva_add_f32", ["tmp", "res", "sum"], [1, 64, 1], ONE)
+    assert launches(ctx, bufs, ops + [add]) == 2
+    assert launches(ctx, bufs, [(k, ["sum" if b == "dq" else b for b in binds], p, g) for k, binds, p, g in ops] + [add]) == 3
+    # ropes and cache writes: one; a rope of the rotated rows: not
+    D, kv, heads, M, rows = 64, 2, 14, 3, 40
+    bufs = {n: rng.standard_normal(M * c * D).astype(np.float32) for n, c in (("q", heads), ("k", kv), ("v", kv), ("qr", heads), ("kr", kv))}
+    bufs.update(pos=np.arange(M, dtype=np.int32), idx=np.arange(M, dtype=np.int64), status=np.array([0, 0xFFFFFFFF], np.uint32))
+    bufs.update({c: np.zeros(rows * kv * D, np.float16) for c in ("kc", "vc")})
+    q, k = rope("q", "qr", D, heads, M), rope("k", "kr", D, kv, M)
+    ks, vs = store("kr", "kc", kv * D, M, rows), store("v", "vc", kv * D, M, rows)
+    assert launches(ctx, bufs, [q, k, ks, vs]) == 1
+    assert launches(ctx, bufs, [q, rope("qr", "q", D, heads, M), k, ks]) == 2
+    # quantizes of the same rows: up to four together, with the gate in front; of other arguments: apart
+    for scheme, f16 in (("a8", 0), ("a8", 1), ("a8b", 0), ("a8b", 1)):
+        bufs = base(9)
+        qs = [quant(scheme, f16, "act", f"m{j}", 9, K, bufs) for j in range(4)]
+        gate = ("ameva_swiglu_f32", ["gate", "up", "act"], [9 * K], ONE)
+        assert launches(ctx, bufs, qs) == 1 and launches(ctx, bufs, [gate] + qs) == 1
+        assert launches(ctx, bufs, [qs[0], quant(scheme, f16, "act", "m1", 9, K, bufs, mode=1)]) == 2
+    # a product of a byte-decoded type and the ADD behind it: one; in place of the product: two
+    N = 96
+    bufs = {"q": np.zeros(N * K, np.uint8), "s": np.zeros(N * (K // 256) * 18, np.uint8), "aq": np.zeros(K, np.uint8),
+            "ad": np.zeros(K // 256 * 48, np.uint8), "o": np.zeros(N, np.float32), "e": np.zeros(N, np.float32), "r": np.zeros(N, np.float32)}
+    gemv = ("ameva_mmvqb_q6_K", ["q", "s", "aq", "ad", "o"], [1, N, K, N], ONE)
+    assert launches(ctx, bufs, [gemv, ("ameva_add_f32", ["o", "e", "r"], [1, N, 1], ONE)]) == 1
+    assert launches(ctx, bufs, [gemv, ("ameva_add_f32", ["o", "e", "o"], [1, N, 1], ONE)]) == 2
