@@ -1305,6 +1305,8 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_co
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------
+// (for tests of the choice below: K ranges per tile of the GEMM this thread launched last)
+static thread_local uint32_t g_last_k_ranges = 0;
 static bool encode_2d(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType dt, uint32_t esz, const void* ptr,
                       uint64_t inner, uint64_t rows, uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_rows,
                       CUtensorMapSwizzle sw) {
@@ -1524,6 +1526,7 @@ static AcResult launch_wide(const LaunchArgs& a, EncodeTiledFn enc, const void* 
     cfg.attrs = attr;
     cfg.numAttrs = a.stream.in_order ? 1 : 2;
     if (a.stream.dry) return AC_SUCCESS;
+    g_last_k_ranges = 1u;
     if (cudaLaunchKernelEx(&cfg, gemm_tc_wide_kernel<TYPE>, act_map, raw_map, scale_map, out_maps, p) != cudaSuccess) {
         cudaGetLastError();
         return AC_ERR_INVALID_WORK_GROUP_SIZE;
@@ -1738,6 +1741,7 @@ static AcResult launch(const LaunchArgs& a, const void* Qp, const void* Sp, cons
                                         : ensure_dynamic_smem<gemm_tc_kernel<TYPE, false, false>>((int)kSmemLimit));
     if (!fits) return AC_ERR_INVALID_WORK_GROUP_SIZE;
     if (a.stream.dry) return AC_SUCCESS;
+    g_last_k_ranges = p.splits ? p.splits : 1u;
     cudaError_t e;
     if (p.splits)
         e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<TYPE, true, false, true>, act_map, raw_map, scale_map, out_maps, p);
@@ -1818,3 +1822,5 @@ AcResult launch_bitnet_gemm_i2_s(const LaunchArgs& a) {
 }  // namespace amv
 
 AMV_TRACE_READER(gemm_tc)
+
+extern "C" uint32_t ac_b200_gemm_last_k_ranges(void) { return amv::tc::g_last_k_ranges; }

@@ -388,6 +388,9 @@ AcResult ac_b200_batch_replay(AcCommandBatch* batch, AcEvent** out_completion_ev
  * them still ran (the first of a flush, and products whose weights an earlier dispatch of the batch may write: weights are
  * otherwise requested ahead of time). No counterpart in the reference. */
 AcResult ac_b200_batch_get_launches(const AcCommandBatch* batch, uint32_t* out_launches, uint32_t* out_in_order);
+/* For measurements and tests: into how many K ranges, multiplied by CTA pairs of one cluster, the tensor-core GEMM that the
+ * calling thread launched last has cut every output tile (1: not cut that way; 0: none launched yet). */
+uint32_t ac_b200_gemm_last_k_ranges(void);
 
 /* Weight codec: ggml block bytes <-> the device region layout the kernels read. Stands in for the reference's CPU
  * repack codec (adapters/llama/ggml-ameva/ggml-ameva-repack.cpp:82-247, ggml-ameva-buffer.cpp:300-330). type is the

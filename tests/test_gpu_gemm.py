@@ -97,6 +97,16 @@ def test_i2s_k_ranges_in_clusters_bit_exact(ctx, M, N, K):
     run_gemm(ctx, I2_S, M, N, K, seed=M + 1)
 
 
+@pytest.mark.parametrize("t,M,N,K,cut", [(Q8_0, 77, 1027, 3328, True), (Q4_0, 33, 511, 1280, True), (Q4_K, 256, 256, 8192, True), (Q4_0, 512, 258, 2304, True),
+                                         (I2_S, 77, 515, 6656, True), (I2_S, 128, 1024, 2560, True), (I2_S, 77, 515, 6912, False),
+                                         (Q8_0, 512, 11008, 4096, False)])
+def test_products_that_are_cut_into_k_ranges(ctx, t, M, N, K, cut):
+    """The forms above do run in clusters (a multiple of four K blocks and few tiles), and the others do not."""
+    run_gemm(ctx, t, M, N, K, seed=M)
+    got = pkg.runtime.load_library().ac_b200_gemm_last_k_ranges()
+    assert got >= 2 if cut else got == 1
+
+
 @pytest.mark.parametrize("t", [Q8_0, Q4_0, Q4_K])
 def test_exact_path_block_sums_at_prefill_m(ctx, t):
     run_gemm(ctx, t, 24, 96, 512, seed=5, exact=True)
